@@ -226,7 +226,7 @@ def step_algorithmic_bytes(st, mesh, precision, cfg):
 
 def pcg_kernel_name(precision, prof):
     if precision != "mixed":
-        return "k_pcg"
+        return "k_pcg64"
     info = prof.get("launch_info") or {}
     return "k_mx_pcg_cluster" if info.get("pcgClusterCtas") else "k_mx_pcg"
 

@@ -15,6 +15,7 @@
 #include "contact.cuh"
 #include "contact_host.hpp"
 #include "graph_ctx.hpp"
+#include "ordered_sum.cuh"
 #include "solver.hpp"
 
 namespace cs {
@@ -67,12 +68,6 @@ __device__ __forceinline__ int v_ncand(const CView& v) { return v.acnt ? v.acnt[
 __device__ __forceinline__ int v_lag(const CView& v) { return v.acnt ? v.acnt[AC_LAG] : v.lagCount; }
 // A contact count passed by the host, or (negative) read from the device.
 __device__ __forceinline__ int v_na(const CView& v, int na) { return na >= 0 ? na : v.acnt[AC_NA]; }
-
-__device__ __forceinline__ double seq_sum(const double* t, int n) {
-  double s = 0.0;
-  for (int i = 0; i < n; i++) s = s + t[i];
-  return s;
-}
 
 // Order-preserving map of a non-NaN double onto an unsigned 64-bit integer
 // (negative values bit-flipped, non-negative ones with the sign bit set), so
@@ -440,16 +435,20 @@ __global__ void k_contact_prep(CView v, const double* x, int na) {
 }
 
 // Barrier energy and friction work of the step's diagnostics. The FP64 path
-// adds the terms left to right like the reference; the mixed path (tree = 1)
-// uses a fixed-order block tree: each of the 1024 threads adds a strided
-// subset, then warp and block trees (same bits on every run).
-__global__ void __launch_bounds__(1024) k_contact_chains(CView v, int na, int tree) {
+// (k_contact_sums, one block per sum) adds the terms left to right like the
+// reference; the mixed path (k_contact_chains) uses a fixed-order block tree:
+// each of the 1024 threads adds a strided subset, then warp and block trees
+// (same bits on every run).
+constexpr int kSumThreads = 1024;
+__global__ void __launch_bounds__(kSumThreads) k_contact_sums(CView v, int na) {
+  __shared__ OrdSmem<kSumThreads / 32> os;
+  const double s = block_ordered_sum(blockIdx.x == 0 ? v.tc : v.tf, na, os);
+  if (threadIdx.x != 0) return;
+  if (blockIdx.x == 0) v.diag->barrierEnergy = s;
+  else v.diag->frictionWork = v.diag->frictionWork + s;
+}
+__global__ void __launch_bounds__(1024) k_contact_chains(CView v, int na) {
   if (na < 0) na = v.acnt ? v.acnt[AC_NA] : 0;
-  if (!tree) {
-    if (threadIdx.x == 0) v.diag->barrierEnergy = seq_sum(v.tc, na);
-    if (threadIdx.x == 32) v.diag->frictionWork = v.diag->frictionWork + seq_sum(v.tf, na);
-    return;
-  }
   __shared__ double ws[2][32];
   double a = 0, b = 0;
   for (int i = threadIdx.x; i < na; i += blockDim.x) {
@@ -1321,12 +1320,11 @@ void ContactHost::gradient_terms(Solver& s) {
   CView v = view(*this, s);
   if (na > 0) {
     k_contact_prep<<<cnb(na), kCT, 0, st>>>(v, s.d.x, na);
-    k_contact_chains<<<1, s.mixed() ? 1024 : 64, 0, st>>>(v, na, s.mixed() ? 1 : 0);
-    lc += 2;
-  } else {
-    k_contact_chains<<<1, 64, 0, st>>>(v, 0, 0);
     lc++;
   }
+  if (s.mixed()) k_contact_chains<<<1, 1024, 0, st>>>(v, na);
+  else k_contact_sums<<<2, kSumThreads, 0, st>>>(v, na);
+  lc++;
   if (na > 0) {
     k_contact_grad_rec<<<cnb(4l * na), kCT, 0, st>>>(v, 4 * na);
     lc++;
@@ -1805,7 +1803,7 @@ void ContactHost::cap_gradient_terms(Solver& s, GraphCtx& g) {
   CView v = cview(*this, s);
   const long cap = (long)actCap;
   k_contact_prep<<<cnb(cap), kCT, 0, st>>>(v, s.d.x, -1);
-  k_contact_chains<<<1, s.mixed() ? 1024 : 64, 0, st>>>(v, -1, s.mixed() ? 1 : 0);
+  k_contact_chains<<<1, 1024, 0, st>>>(v, -1);
   k_contact_grad_rec<<<cnb(4 * cap), kCT, 0, st>>>(v, (int)(4 * cap));
   k_contact_grad_gather<<<cnb(n), kCT, 0, st>>>(v, s.d.cgrad);
   k_contact_curv<<<cnb(cap), kCT, 0, st>>>(v, s.d.x, -1);

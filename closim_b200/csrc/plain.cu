@@ -3,15 +3,14 @@
 // One thread per element over SoA mesh constants writes element-local results;
 // one thread per vertex gathers them through the element-ordered CSR
 // incidence, so each vertex sum adds the same terms in the same order as the
-// reference's scatter (src/mesh/incidence.ts:1-7). The PCG solve runs as one
-// cooperative persistent kernel: grid-wide barriers separate its phases and
-// every reduction is a fixed-order two-level sum that all blocks evaluate
-// identically, so control decisions agree across the grid and runs repeat
-// bit for bit.
+// reference's scatter (src/mesh/incidence.ts:1-7). Sums the reference
+// accumulates in a loop are ordered sums (ordered_sum.cuh). The PCG solve is
+// pcg64.cu's.
 #include <cstdio>
 
 #include "adjoint_math.cuh"
 #include "contact.cuh"
+#include "ordered_sum.cuh"
 #include "plain.cuh"
 
 namespace cs {
@@ -22,58 +21,8 @@ __device__ __forceinline__ void load3(const double* x, int v, double o[3]) {
   o[0] = x[v * 3]; o[1] = x[v * 3 + 1]; o[2] = x[v * 3 + 2];
 }
 
-// s0 + t[0] + t[1] + ... evaluated left to right by one thread: the
-// reference's `for (i...) s += t[i]` accumulation, rounding for rounding.
-__device__ __forceinline__ double seq_chain(const double* t, int n, double s = 0.0) {
-  int i = 0;
-  for (; i + 4 <= n; i += 4) {
-    const double a0 = t[i], a1 = t[i + 1], a2 = t[i + 2], a3 = t[i + 3];
-    s = s + a0;
-    s = s + a1;
-    s = s + a2;
-    s = s + a3;
-  }
-  for (; i < n; i++) s = s + t[i];
-  return s;
-}
-
-// The same left-to-right chain, run by a whole block: warps 1.. stream the
-// terms through a double-buffered shared-memory stage while thread 0 adds the
-// previous stage in order. Every thread of the block must call it; the sum is
-// valid in thread 0.
-constexpr int kChunk = 2048;
-__device__ __forceinline__ double block_chain(const double* t, int n, double* buf) {
-  double s = 0.0;
-  const int first = n < kChunk ? n : kChunk;
-  for (int j = threadIdx.x; j < first; j += blockDim.x) buf[j] = t[j];
-  __syncthreads();
-  const int nchunks = (n + kChunk - 1) / kChunk;
-  for (int c = 0; c < nchunks; c++) {
-    const int base = c * kChunk;
-    const int len = n - base < kChunk ? n - base : kChunk;
-    const double* cur = buf + (c & 1) * kChunk;
-    if (threadIdx.x >= 32) {
-      const int nbase = base + kChunk;
-      if (nbase < n) {
-        double* nxt = buf + ((c + 1) & 1) * kChunk;
-        const int nlen = n - nbase < kChunk ? n - nbase : kChunk;
-        for (int j = threadIdx.x - 32; j < nlen; j += blockDim.x - 32) nxt[j] = t[nbase + j];
-      }
-    } else if (threadIdx.x == 0) {
-      int j = 0;
-      for (; j + 16 <= len; j += 16) {
-        double a[16];
-#pragma unroll
-        for (int q = 0; q < 16; q++) a[q] = cur[j + q];
-#pragma unroll
-        for (int q = 0; q < 16; q++) s = s + a[q];
-      }
-      for (; j < len; j++) s = s + cur[j];
-    }
-    __syncthreads();
-  }
-  return s;
-}
+// Block size of the kernels that evaluate one ordered sum (ordered_sum.cuh).
+constexpr int kOrdThreads = 1024;
 
 // ---- predictor (newton.ts:41-50) -------------------------------------------
 // yHat = x0 + h v + h^2 g is the inertial target and, in the reference, the
@@ -185,9 +134,9 @@ __global__ void __launch_bounds__(kThreads) k_gather_grad(Dev d) {
 
 // Final reduction of the gradient pass: sqrt(sum g^2) in index order
 // (newton.ts:128), max strain (order-free).
-__global__ void __launch_bounds__(kThreads) k_grad_final(Dev d, int nbT) {
-  __shared__ double cbuf[2 * kChunk];
-  const double gs = block_chain(d.T0, d.n * 3, cbuf);
+__global__ void __launch_bounds__(kOrdThreads) k_grad_final(Dev d, int nbT) {
+  __shared__ OrdSmem<kOrdThreads / 32> os;
+  const double gs = block_ordered_sum(d.T0, d.n * 3, os);
   if (threadIdx.x >= 32) return;
   const double ms = warp_max_partials(d.part + 0 * d.partStride, nbT);
   if (threadIdx.x == 0) {
@@ -225,12 +174,11 @@ __global__ void __launch_bounds__(kThreads) k_energy(Dev d, const double* x) {
 
 // totalEnergy (newton.ts:76-88): ((sum inertia) + internal) + merit, each sum a
 // left-to-right chain; block 0 inertia, block 1 internal, block 2 merit.
-__global__ void __launch_bounds__(kThreads) k_energy_chains(Dev d, int nMerit) {
-  __shared__ double cbuf[2 * kChunk];
-  double v = 0.0;
-  if (blockIdx.x == 0) v = block_chain(d.T0, d.n * 3, cbuf);
-  if (blockIdx.x == 1) v = block_chain(d.T1, d.m + (d.kb > 0 ? d.hg : 0), cbuf);
-  if (blockIdx.x == 2) v = d.hasContact ? block_chain(d.Tc, nMerit, cbuf) : 0.0;
+__global__ void __launch_bounds__(kOrdThreads) k_energy_chains(Dev d, int nMerit) {
+  __shared__ OrdSmem<kOrdThreads / 32> os;
+  const double* t = blockIdx.x == 0 ? d.T0 : blockIdx.x == 1 ? d.T1 : d.Tc;
+  const int n = blockIdx.x == 0 ? d.n * 3 : blockIdx.x == 1 ? d.m + (d.kb > 0 ? d.hg : 0) : d.hasContact ? nMerit : 0;
+  const double v = block_ordered_sum(t, n, os);
   if (threadIdx.x == 0) d.scal[S_E_INERTIA + blockIdx.x] = v;
 }
 __global__ void k_energy_final(Dev d) {
@@ -320,7 +268,8 @@ __global__ void __launch_bounds__(kSchwarzWarps * 32) k_schwarz_factor(Dev d) {
   double* L = d.L + (size_t)dom * 576;
   if (ok) {
     for (int i = lane; i < dw; i += 32)
-      for (int j = 0; j < 24; j++) L[i * 24 + j] = j <= i && j < dw ? a[i * dw + j] : 0.0;
+      for (int j = 0; j < 24; j++)  // the upper triangle holds L^T: a column read gives both
+        L[i * 24 + j] = j >= dw ? 0.0 : j <= i ? a[i * dw + j] : a[j * dw + i];
   } else {
     for (int i = lane; i < dw; i += 32) {
       const int v = d.domVerts[start + i / 3];
@@ -390,334 +339,6 @@ __global__ void __launch_bounds__(kThreads) k_coarse_diag(Dev d) {
   for (int a = 0; a < 3; a++) d.dcoarse[dom * 3 + a] = dc[a];
 }
 
-// z = M^-1 r on one domain; returns sum r.z over its (pin-filtered) dofs.
-__device__ double schwarz_apply_domain(const Dev& d, int dom) {
-  const int start = d.domStart[dom], dv = d.domStart[dom + 1] - start, dw = dv * 3;
-  const double* L = d.L + (size_t)dom * 576;
-  double rhs[24], y[24], sol[24];
-  for (int l = 0; l < dv; l++) {
-    const int v = d.domVerts[start + l];
-    rhs[l * 3] = d.r[v * 3]; rhs[l * 3 + 1] = d.r[v * 3 + 1]; rhs[l * 3 + 2] = d.r[v * 3 + 2];
-  }
-  if (d.domFlag[dom]) {
-    for (int i = 0; i < dw; i++) {
-      double s = rhs[i];
-      for (int j = 0; j < i; j++) s -= L[i * 24 + j] * y[j];
-      y[i] = s / L[i * 24 + i];
-    }
-    for (int i = dw - 1; i >= 0; i--) {
-      double s = y[i];
-      for (int j = i + 1; j < dw; j++) s -= L[j * 24 + i] * sol[j];
-      sol[i] = s / L[i * 24 + i];
-    }
-  } else {
-    for (int i = 0; i < dw; i++) {
-      double s = 0;
-      for (int j = 0; j < dw; j++) s += L[i * 24 + j] * rhs[j];
-      sol[i] = s;
-    }
-  }
-  // two-level: + P (omega Dc^-1) R r on this domain (applyMasTwoLevel,
-  // mas.ts:110-145, omega = 0.5; the coarse vector of a domain is constant per
-  // component over its members, scaled by 1/sqrt(|d|) both ways)
-  double cz[3] = {0, 0, 0};
-  const double sc = 1 / sqrt((double)dv);
-  if (d.precond == 2) {
-    double rc[3] = {0, 0, 0};
-    for (int l = 0; l < dv; l++)
-      for (int k = 0; k < 3; k++) rc[k] += rhs[l * 3 + k] * sc;
-    for (int k = 0; k < 3; k++) {
-      const double dd = d.dcoarse[dom * 3 + k];
-      cz[k] = dd > 1e-12 ? (0.5 * rc[k]) / dd : 0.0;
-    }
-  }
-  for (int l = 0; l < dv; l++) {
-    const int v = d.domVerts[start + l];
-    const bool pin = d.pinned[v];
-    for (int k = 0; k < 3; k++) {
-      double zz = 0.0 + sol[l * 3 + k];
-      if (d.precond == 2) zz += cz[k] * sc;
-      if (pin) zz = 0.0;
-      d.z[v * 3 + k] = zz;
-      d.T2[v * 3 + k] = d.r[v * 3 + k] * zz;
-    }
-  }
-  return 0.0;
-}
-
-// ---- PCG as one cooperative kernel (pcg.ts:11-95 + newton.ts:148-179) ----------
-struct PcgArgs {
-  Dev d;
-  int maxIters;
-  double tol;
-};
-
-// Block partial -> row slot; after grid.sync every block reads the same total.
-__device__ __forceinline__ void put_partial(const Dev& d, int row, double v, double* sm) {
-  const double b = block_sum(v, sm);
-  if (threadIdx.x == 0) d.part[row * d.partStride + blockIdx.x] = b;
-}
-__device__ __forceinline__ double get_total(const Dev& d, int row, double* bc) {
-  if (threadIdx.x < 32) {
-    const double s = warp_sum_partials(d.part + row * d.partStride, gridDim.x);
-    if (threadIdx.x == 0) bc[0] = s;
-  }
-  __syncthreads();
-  const double r = bc[0];
-  __syncthreads();
-  return r;
-}
-__device__ __forceinline__ double get_max_nonan(const Dev& d, int row, double* bc) {
-  if (threadIdx.x < 32) {
-    const int lane = threadIdx.x;
-    double s = 0;
-    for (int i = lane; i < (int)gridDim.x; i += 32) {
-      const double v = d.part[row * d.partStride + i];
-      if (v > s) s = v;
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-      const double w = __shfl_xor_sync(0xffffffffu, s, o);
-      if (w > s) s = w;
-    }
-    if (lane == 0) bc[0] = s;
-  }
-  __syncthreads();
-  const double r = bc[0];
-  __syncthreads();
-  return r;
-}
-__device__ __forceinline__ double block_max_nonan(double v, double* sm) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int o = 16; o > 0; o >>= 1) {
-    const double w = __shfl_down_sync(0xffffffffu, v, o);
-    if (w > v) v = w;
-  }
-  __syncthreads();
-  if (lane == 0) sm[warp] = v;
-  __syncthreads();
-  double r = 0;
-  if (threadIdx.x == 0) {
-    for (int i = 0; i < (int)(blockDim.x >> 5); i++)
-      if (sm[i] > r) r = sm[i];
-    sm[0] = r;
-  }
-  __syncthreads();
-  r = sm[0];
-  __syncthreads();
-  return r;
-}
-
-// Chained sums after a grid barrier: chain w (w < nch) runs on block w as a
-// block_chain; results land in scal[S_CH0 + w]. With fewer blocks than chains,
-// block 0 runs them one after another.
-__device__ __forceinline__ void run_chains(const Dev& d, int nch, const double* a0, const double* a1,
-                                           const double* a2, int n, double* cbuf) {
-  const double* arr[3] = {a0, a1, a2};
-  if ((int)gridDim.x >= nch) {
-    if ((int)blockIdx.x < nch) {
-      const double v = block_chain(arr[blockIdx.x], n, cbuf);
-      if (threadIdx.x == 0) d.scal[S_CH0 + blockIdx.x] = v;
-    }
-  } else if (blockIdx.x == 0) {
-    for (int w = 0; w < nch; w++) {
-      const double v = block_chain(arr[w], n, cbuf);
-      if (threadIdx.x == 0) d.scal[S_CH0 + w] = v;
-    }
-  }
-}
-// One chain into scal[slot], on block 0.
-__device__ __forceinline__ void run_chain1(const Dev& d, const double* a, int n, int slot, double* cbuf) {
-  if (blockIdx.x == 0) {
-    const double v = block_chain(a, n, cbuf);
-    if (threadIdx.x == 0) d.scal[slot] = v;
-  }
-}
-
-__global__ void __launch_bounds__(kThreads) k_pcg(PcgArgs A) {
-  cg::grid_group grid = cg::this_grid();
-  __shared__ double sm[32];
-  __shared__ double bc[2];
-  __shared__ double cbuf[2 * kChunk];
-  const Dev& d = A.d;
-  const int n3 = d.n * 3;
-  const int tid = blockIdx.x * blockDim.x + threadIdx.x, nth = gridDim.x * blockDim.x;
-  const bool jacobi = d.precond == 0;
-  // ---- init: r = filter(b), z = M^-1 r, p = z (pcg.ts:27-55) ----
-  for (int i = tid; i < n3; i += nth) {
-    const double bi = -d.g[i];
-    d.T0[i] = bi * bi;
-    const double ri = d.pinned[i / 3] ? 0.0 : bi;
-    d.r[i] = ri;
-    d.dx[i] = 0;
-    d.T1[i] = ri * ri;
-    if (jacobi) {
-      double zi = d.diag[i] > 1e-12 ? ri / d.diag[i] : ri;
-      if (d.pinned[i / 3]) zi = 0;
-      d.z[i] = zi;
-      d.p[i] = zi;
-      d.T2[i] = ri * zi;
-    }
-  }
-  grid.sync();
-  if (!jacobi) {
-    for (int dom = tid; dom < d.D; dom += nth) schwarz_apply_domain(d, dom);
-    grid.sync();
-    for (int i = tid; i < n3; i += nth) d.p[i] = d.z[i];
-  }
-  // chains: rz (T2), |b|^2 (T0), |r|^2 (T1)
-  run_chains(d, 3, d.T2, d.T0, d.T1, n3, cbuf);
-  grid.sync();
-  double rz = d.scal[S_CH0];
-  const double bNorm = sqrt(d.scal[S_CH1]);
-  const double absTol = js_max(A.tol * js_max(bNorm, 1e-12), 1e-12);
-  double residual = sqrt(d.scal[S_CH2]);
-  int iters = 0;
-  bool done = residual < absTol;
-  if (!done) {
-    for (int i = tid; i < n3; i += nth) d.T3[i] = d.p[i] * d.p[i];
-    grid.sync();
-    run_chain1(d, d.T3, n3, S_CH3, cbuf);
-    grid.sync();
-  }
-  int k = 0;
-  for (; !done && k < A.maxIters; k++) {
-    // ---- Ap = M/h^2 p + membraneHvp (fem.ts:108-130) + contact HVP ----
-    const double pNorm = sqrt(d.scal[S_CH3]);
-    const double h = 1e-8 * (1 + pNorm);
-    for (int t = tid; t < d.m; t += nth) {
-      const uint32_t vi[3] = {d.idx[t * 3], d.idx[t * 3 + 1], d.idx[t * 3 + 2]};
-      double xp[9], xm[9];
-#pragma unroll
-      for (int c = 0; c < 3; c++)
-#pragma unroll
-        for (int q = 0; q < 3; q++) {
-          const double xx = d.x[vi[c] * 3 + q], pq = d.p[vi[c] * 3 + q];
-          xp[c * 3 + q] = xx + h * pq;
-          xm[c * 3 + q] = xx - h * pq;
-        }
-      const float4 iv = d.inv[t];
-      const double ar = d.area[t];
-      double e, gp[9], gm[9], E[3];
-      tri_grad<double>(xp, xp + 3, xp + 6, iv.x, iv.y, iv.z, iv.w, ar, d.mat, e, gp, E);
-      tri_grad<double>(xm, xm + 3, xm + 6, iv.x, iv.y, iv.z, iv.w, ar, d.mat, e, gm, E);
-      double* o = d.elem + (size_t)t * 18;
-#pragma unroll
-      for (int q = 0; q < 9; q++) { o[q] = gp[q]; o[9 + q] = gm[q]; }
-    }
-    if (d.hasContact) contact_hvp_coeffs(d, d.p, tid, nth);
-    grid.sync();
-    for (int v = tid; v < d.n; v += nth) {
-      double sp[3] = {0, 0, 0}, sn[3] = {0, 0, 0};
-      for (uint32_t q = d.memOff[v]; q < d.memOff[v + 1]; q++) {
-        const uint32_t rec = d.memRec[q];
-        const double* e = d.elem + (size_t)(rec >> 2) * 18 + (rec & 3) * 3;
-        sp[0] += e[0]; sp[1] += e[1]; sp[2] += e[2];
-        sn[0] += e[9]; sn[1] += e[10]; sn[2] += e[11];
-      }
-      double ch[3] = {0, 0, 0};
-      if (d.hasContact) contact_hvp_gather(d, v, ch);
-      const double M = d.mass[v];
-      const bool pin = d.pinned[v];
-#pragma unroll
-      for (int c = 0; c < 3; c++) {
-        const int i = v * 3 + c;
-        const double Hp = (sp[c] - sn[c]) / (2 * h);
-        double ap = M * d.p[i] * d.invH2 + Hp;
-        if (d.hasContact) ap += ch[c];
-        if (pin) ap = 0;
-        d.Ap[i] = ap;
-        d.T0[i] = d.p[i] * ap;
-      }
-    }
-    grid.sync();
-    run_chain1(d, d.T0, n3, S_CH1, cbuf);
-    grid.sync();
-    const double pAp = d.scal[S_CH1];
-    if (!(pAp > 1e-30)) { iters = k; done = true; break; }
-    const double alpha = rz / pAp;
-    for (int i = tid; i < n3; i += nth) {
-      const bool pin = d.pinned[i / 3];
-      double xi = d.dx[i] + alpha * d.p[i];
-      double ri = d.r[i] - alpha * d.Ap[i];
-      if (pin) { xi = 0; ri = 0; }
-      d.dx[i] = xi;
-      d.r[i] = ri;
-      d.T1[i] = ri * ri;
-      if (jacobi) {
-        double zi = d.diag[i] > 1e-12 ? ri / d.diag[i] : ri;
-        if (pin) zi = 0;
-        d.z[i] = zi;
-        d.T2[i] = ri * zi;
-      }
-    }
-    grid.sync();
-    run_chains(d, jacobi ? 2 : 1, d.T1, d.T2, d.T2, n3, cbuf);  // |r|^2 -> CH0, r.z -> CH1
-    grid.sync();
-    residual = sqrt(d.scal[S_CH0]);
-    if (residual < absTol) { iters = k + 1; done = true; break; }
-    if (!jacobi) {
-      for (int dom = tid; dom < d.D; dom += nth) schwarz_apply_domain(d, dom);
-      grid.sync();
-      run_chain1(d, d.T2, n3, S_CH1, cbuf);
-      grid.sync();
-    }
-    const double rzNew = d.scal[S_CH1];
-    const double beta = rzNew / rz;
-    for (int i = tid; i < n3; i += nth) {
-      const double pi = d.z[i] + beta * d.p[i];
-      d.p[i] = pi;
-      d.T3[i] = pi * pi;
-    }
-    rz = rzNew;
-    grid.sync();
-    run_chain1(d, d.T3, n3, S_CH3, cbuf);
-    grid.sync();
-  }
-  if (!done) iters = A.maxIters;
-  // ---- descent safeguard + trust region (newton.ts:152-179) ----
-  grid.sync();
-  for (int i = tid; i < n3; i += nth) d.T0[i] = d.g[i] * d.dx[i];
-  grid.sync();
-  run_chain1(d, d.T0, n3, S_CH2, cbuf);
-  grid.sync();
-  double gtdx = d.scal[S_CH2];
-  bool fallback = false;
-  if (!isfinite(gtdx) || gtdx >= 0) {
-    fallback = true;
-    for (int i = tid; i < n3; i += nth) {
-      const double di = -d.g[i] / d.diag[i];
-      d.dx[i] = di;
-      d.T1[i] = d.g[i] * di;
-    }
-    grid.sync();
-    run_chain1(d, d.T1, n3, S_CH3, cbuf);
-    grid.sync();
-    gtdx = d.scal[S_CH3];
-  }
-  double mx = 0;
-  for (int i = tid; i < n3; i += nth) {
-    const double a = fabs(d.dx[i]);
-    if (a > mx) mx = a;
-  }
-  const double bmx = block_max_nonan(mx, sm);
-  if (threadIdx.x == 0) d.part[6 * d.partStride + blockIdx.x] = bmx;
-  grid.sync();
-  const double maxDx = get_max_nonan(d, 6, bc);
-  const double TRUST = 0.002;
-  if (maxDx > TRUST) {
-    const double s = TRUST / maxDx;
-    for (int i = tid; i < n3; i += nth) d.dx[i] *= s;
-    gtdx *= s;
-  }
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    d.scal[S_PCG_ITERS] = iters;
-    d.scal[S_PCG_RES] = residual;
-    d.scal[S_GTDX] = gtdx;
-    d.scal[S_FALLBACK] = fallback ? 1 : 0;
-    d.scal[S_MAXDX] = maxDx;
-  }
-}
-
 // ---- standalone FD membrane HVP (fem.ts:108-130) -----------------------------------
 // out = (gradM(x + h p) - gradM(x - h p)) / (2h), h = 1e-8 (1 + |p|): the same
 // element and gather arithmetic as the PCG kernel's HVP phase, as plain kernels.
@@ -725,9 +346,9 @@ __global__ void k_hvp_terms(const double* p, int n3, double* T) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n3) T[i] = p[i] * p[i];
 }
-__global__ void __launch_bounds__(kThreads) k_hvp_h(const double* T, int n3, double* h) {
-  __shared__ double cbuf[2 * kChunk];
-  const double pp = block_chain(T, n3, cbuf);
+__global__ void __launch_bounds__(kOrdThreads) k_hvp_h(const double* T, int n3, double* h) {
+  __shared__ OrdSmem<kOrdThreads / 32> os;
+  const double pp = block_ordered_sum(T, n3, os);
   if (threadIdx.x == 0) *h = 1e-8 * (1 + sqrt(pp));
 }
 __device__ __forceinline__ void hvp_elem_tri(int t, const uint32_t* idx, const float4* inv, const float* area,
@@ -777,7 +398,7 @@ void launch_membrane_hvp(const uint32_t* idx, const float4* inv, const float* ar
                          int m, const uint32_t* memOff, const uint32_t* memRec, const double* x, const double* p,
                          double* out, double* T, double* h, double* elem, cudaStream_t s) {
   k_hvp_terms<<<nblk(n * 3), kThreads, 0, s>>>(p, n * 3, T);
-  k_hvp_h<<<1, kThreads, 0, s>>>(T, n * 3, h);
+  k_hvp_h<<<1, kOrdThreads, 0, s>>>(T, n * 3, h);
   k_hvp_elem<<<nblk(m), kThreads, 0, s>>>(idx, inv, area, mat, m, x, p, h, elem);
   k_hvp_gather<<<nblk(n), kThreads, 0, s>>>(memOff, memRec, n, elem, h, out);
 }
@@ -824,9 +445,9 @@ __global__ void __launch_bounds__(kThreads) k_gather_internal(Dev d, double* gra
 }
 // out[0] = the internal energy chain, out[1] = max strain over the triangle
 // partials (nbT of them; 0 when none were computed).
-__global__ void __launch_bounds__(kThreads) k_internal_final(Dev d, int nbT, double* out) {
-  __shared__ double cbuf[2 * kChunk];
-  const double e = block_chain(d.T1, d.m + (d.kb > 0 ? d.hg : 0), cbuf);
+__global__ void __launch_bounds__(kOrdThreads) k_internal_final(Dev d, int nbT, double* out) {
+  __shared__ OrdSmem<kOrdThreads / 32> os;
+  const double e = block_ordered_sum(d.T1, d.m + (d.kb > 0 ? d.hg : 0), os);
   if (threadIdx.x >= 32) return;
   const double ms = nbT > 0 ? warp_max_partials(d.part + 0 * d.partStride, nbT) : 0.0;
   if (threadIdx.x == 0) {
@@ -874,7 +495,7 @@ void launch_internal_eval(const Dev& d0, const double* x, double* grad, double* 
     k_gather_internal<<<nblk(d.n), kThreads, 0, s>>>(d, grad);
   }
   k_internal_energy_terms<<<nblk(std::max(d.m, d.hg)), kThreads, 0, s>>>(d, x);
-  k_internal_final<<<1, kThreads, 0, s>>>(d, nbT, out2);
+  k_internal_final<<<1, kOrdThreads, 0, s>>>(d, nbT, out2);
 }
 
 void launch_membrane_hvp_analytic(const Dev& d, const double* x, const double* p, double* out, cudaStream_t s) {
@@ -935,7 +556,7 @@ void launch_grad_terms(const Dev& d, cudaStream_t s, bool analyticBend) {
 }
 void launch_grad(const Dev& d, cudaStream_t s, bool analyticBend) {
   launch_grad_terms(d, s, analyticBend);
-  k_grad_final<<<1, kThreads, 0, s>>>(d, nblk(d.m));
+  k_grad_final<<<1, kOrdThreads, 0, s>>>(d, nblk(d.m));
 }
 void launch_energy_terms(const Dev& d, const double* x, cudaStream_t s) {
   const int nb = nblk(std::max(std::max(d.n, d.m), d.hg));
@@ -943,7 +564,7 @@ void launch_energy_terms(const Dev& d, const double* x, cudaStream_t s) {
 }
 void launch_energy(const Dev& d, const double* x, cudaStream_t s) {
   launch_energy_terms(d, x, s);
-  k_energy_chains<<<3, kThreads, 0, s>>>(d, d.hasContact ? d.c.nActive : 0);
+  k_energy_chains<<<3, kOrdThreads, 0, s>>>(d, d.hasContact ? d.c.nActive : 0);
   k_energy_final<<<1, 1, 0, s>>>(d);
 }
 void launch_diag_init(const Dev& d, double beta, cudaStream_t s) {
@@ -952,21 +573,6 @@ void launch_diag_init(const Dev& d, double beta, cudaStream_t s) {
 void launch_schwarz_factor(const Dev& d, cudaStream_t s) {
   k_schwarz_factor<<<(d.D + kSchwarzWarps - 1) / kSchwarzWarps, kSchwarzWarps * 32, 0, s>>>(d);
   if (d.precond == 2) k_coarse_diag<<<nblk(d.D), kThreads, 0, s>>>(d);
-}
-int pcg_grid_blocks(const Dev& d) {
-  int dev = 0, sms = 0, per = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_pcg, kThreads, 0);
-  const int want = nblk(std::max(d.n * 3, d.m));
-  int cap = per * sms;
-  if (cap < 1) cap = 1;
-  return std::max(1, std::min(want, std::min(cap, d.partStride)));
-}
-int launch_pcg(const Dev& d, int maxIters, double tol, int gridBlocks, cudaStream_t s) {
-  PcgArgs a{d, maxIters, tol};
-  void* args[] = {&a};
-  return (int)cudaLaunchCooperativeKernel((void*)k_pcg, dim3(gridBlocks), dim3(kThreads), args, 0, s);
 }
 void launch_trial(const Dev& d, double alpha, cudaStream_t s) {
   k_trial<<<nblk(d.n * 3), kThreads, 0, s>>>(d, alpha);

@@ -95,7 +95,7 @@ struct Dev {
   const int* domVerts;     // n (members, ascending per domain)
   const int* v2tOff;       // n+1 vertex -> incident triangles (ascending)
   const int* v2t;          // 3m
-  double* L;               // D x 576 (24x24 row-major), Cholesky or inverse diagonal
+  double* L;               // D x 576 (24x24 row-major), Cholesky factor with L^T above the diagonal, or inverse diagonal
   uint8_t* domFlag;        // D
   double* dcoarse;         // 3D: coarse diagonal of the two-level Schwarz (precond 2)
   int precond;             // 0 Jacobi, 1 one-level Schwarz, 2 two-level Schwarz (mas2)
@@ -120,7 +120,6 @@ void launch_energy_terms(const Dev& d, const double* x, cudaStream_t s);
 void launch_energy(const Dev& d, const double* x, cudaStream_t s);  // S_ENERGY_TRIAL
 void launch_diag_init(const Dev& d, double beta, cudaStream_t s);
 void launch_schwarz_factor(const Dev& d, cudaStream_t s);
-int launch_pcg(const Dev& d, int maxIters, double tol, int gridBlocks, cudaStream_t s);
 void launch_trial(const Dev& d, double alpha, cudaStream_t s);   // xt = x + alpha dx, pins
 void launch_velocity(const Dev& d, double damp, cudaStream_t s);
 // SimulationSession.doStep hand-off (sim-session.ts:132-150) on the device:
@@ -132,7 +131,6 @@ void launch_session_check(const double* x, double* stable, int n3, int* flag, cu
 void launch_internal_eval(const Dev& d, const double* x, double* grad, double* out2, cudaStream_t s);
 // evalMembraneHvp: analytic membrane Hessian-vector product at x along p.
 void launch_membrane_hvp_analytic(const Dev& d, const double* x, const double* p, double* out, cudaStream_t s);
-int pcg_grid_blocks(const Dev& d);
 // FD membrane HVP over device arrays (T: 3n terms, h: 1 double, elem: 18m scratch).
 void launch_membrane_hvp(const uint32_t* idx, const float4* inv, const float* area, const Mat<double>& mat, int n,
                          int m, const uint32_t* memOff, const uint32_t* memRec, const double* x, const double* p,

@@ -18,6 +18,7 @@
 #include "cluster_plan.hpp"
 #include "contact_host.hpp"
 #include "mixed.cuh"
+#include "pcg64.cuh"
 #include "plain.cuh"
 #include "setup.hpp"
 
@@ -103,7 +104,13 @@ class Solver {
   DBuf<uint8_t> domFlag;
   DBuf<double> dcoarse;
   double* hscal = nullptr;  // pinned host mirror of scal
-  int pcgBlocks = 1;
+  // linear solve of the FP64 path (pcg64.cu); built for FP64 solvers
+  Pcg64Host pcg;
+  DBuf<int> pcgSlotOff;
+  DBuf<int4> pcgSlots;
+  DBuf<uint32_t> pcgInc;
+  DBuf<double> pcgElem, pcgSums;
+  DBuf<OrdStage> pcgStages;
   // mixed-precision path
   DBuf<float> fr, fz, fp, fAp, fx, felem, ftris, fh9, fLinv, fp2;
   DBuf<float4> fvrec, fdc;
@@ -145,7 +152,7 @@ class Solver {
     return prev;
   }
 
-  // Algorithmic bytes of one k_pcg launch that ran `iters` iterations: per
+  // Algorithmic bytes of one k_pcg64 launch that ran `iters` iterations: per
   // iteration the FD HVP reads x, p (2 x 24 B per vertex), Dm^-1, area and 3
   // indices per triangle (32 B), writes and re-reads 18 element doubles
   // (2 x 144 B per triangle), reads mass (4 B) and writes Ap (24 B); the vector
@@ -295,7 +302,7 @@ class Solver {
     d.T0 = T0.p; d.T1 = T1.p; d.T2 = T2.p; d.T3 = T3.p; d.Tc = Tc.p;
     set_material(m);
     for (int k = 0; k < 3; k++) d.gravity[k] = gravity[k];
-    pcgBlocks = pcg_grid_blocks(d);
+    build_pcg64();
     if (precision == CS_PRECISION_MIXED) {
       for (DBuf<float>* b : {&fr, &fz, &fp, &fAp, &fx}) b->alloc(n3);
       felem.alloc((size_t)cm.m * 9);
@@ -333,6 +340,26 @@ class Solver {
     CK(cudaStreamSynchronize(stream));
     initEpoch++;
     ready = true;
+  }
+
+  void build_pcg64() {
+    int sms = 0;
+    CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
+    build_pcg64_plan(mesh, sms, pcg64_cluster_max(), precision == CS_PRECISION_FP64, pcg);
+    if (precision != CS_PRECISION_FP64) return;
+    Pcg64Plan& p = pcg.p;
+    pcgSlotOff.upload(pcg.slotOff.data(), pcg.slotOff.size(), stream);
+    pcgSlots.upload(pcg.slots.data(), pcg.slots.size(), stream);
+    pcgInc.upload(pcg.inc.data(), pcg.inc.size(), stream);
+    pcgElem.alloc(p.elemSmem ? 1 : (size_t)p.G * p.elemStride);
+    pcgStages.alloc(4 * (size_t)p.NS * kPcg64Stages);
+    pcgSums.alloc((size_t)kPcg64Rows * p.NS);
+    p.slotOff = pcgSlotOff.p;
+    p.slots = pcgSlots.p;
+    p.inc = pcgInc.p;
+    p.elem = pcgElem.p;
+    p.stages = pcgStages.p;
+    p.sums = pcgSums.p;
   }
 
   void set_pins(int k, const int* ids, const double* pos) {
@@ -482,7 +509,10 @@ class Solver {
                                               opts.pcg_max_iters, exactMixed ? std::max(newtonTol, kMixedTolFloor) : 1e-3,
                                               mxCluster, stream));
       else if (mixed()) CK((cudaError_t)mx_launch_pcg(d, mb, opts.pcg_max_iters, 1e-3, mxBlocks, stream));
-      else CK((cudaError_t)launch_pcg(d, opts.pcg_max_iters, 1e-3, pcgBlocks, stream));
+      else {
+        pcg.p.curv = contact ? contact->dd : nullptr;
+        CK((cudaError_t)launch_pcg64(d, pcg.p, opts.pcg_max_iters, 1e-3, stream));
+      }
       if (prof) { CK(cudaEventRecord(pev1, stream)); profPending = true; }
       lc += 1;
       double alpha = 1;

@@ -3,6 +3,14 @@
 // against the oracle. Built with -fmad=false like the FP64 device path.
 #include "../../closim_b200/csrc/contact_math.cuh"
 #include "../../closim_b200/csrc/adjoint_math.cuh"
+#include "../../closim_b200/csrc/div_rn.cuh"
+#include "../../closim_b200/csrc/ordered_sum.cuh"
+
+__global__ void __launch_bounds__(1024) k_hc_ordered(const double* t, int n, double* o) {
+  __shared__ cs::OrdSmem<32> os;
+  const double s = cs::block_ordered_sum(t, n, os);
+  if (threadIdx.x == 0) *o = s;
+}
 
 extern "C" {
 double hc_js_acos(double x) { return cs::js_acos(x); }
@@ -44,4 +52,40 @@ void hc_membrane_block9_psd(const double* x9, const double* inv4, double s, cons
                               true);
 }
 void hc_psd_stress(double* s3) { cs::psd_stress(s3[0], s3[1], s3[2]); }
+// The chunk maps of the ordered sum (ordered_sum.cuh), walked chunk by chunk
+// with starts guessed `rel` away from the true ones; covered = chunks whose map applied.
+double hc_ordered_maps(const double* t, int n, double rel, int* covered) {
+  long long b = cs::ord_bits(0.0);
+  *covered = 0;
+  for (int t0 = 0, c = 0; t0 < n; t0 += 4, c++) {
+    double ch[4] = {0, 0, 0, 0};
+    const int cnt = n - t0 < 4 ? n - t0 : 4;
+    for (int j = 0; j < cnt; j++) ch[j] = t[t0 + j];
+    cs::OrdStage s;
+    cs::ord_chunk<4>([&](int j) { return ch[j]; }, cnt, cs::ord_dbl(b) * (1 + (c % 7 - 3) * rel), s);
+    s.t0 = t0;
+    s.t1 = t0 + cnt;
+    const long long d = b - s.B;
+    *covered += s.type != cs::ORD_RAW && d >= -(long long)s.r && d <= (long long)s.r;
+    b = cs::ord_apply(s, b, t);
+  }
+  return cs::ord_dbl(b);
+}
+void hc_div_rn(const double* a, const double* b, int n, double* o) {
+  for (int i = 0; i < n; i++) o[i] = cs::div_rn_divisor(b[i]) && cs::div_rn_dividend(a[i]) ? cs::div_rn_fast(a[i], b[i], 1.0 / b[i]) : NAN;
+}
+// The block-wide ordered sum on the GPU; returns a cudaError_t.
+int hc_gpu_ordered_sum(const double* t, int n, double* out) {
+  double *dt = nullptr, *dout = nullptr;
+  cudaError_t e = cudaMalloc(&dt, (size_t)(n > 0 ? n : 1) * 8);
+  if (e == cudaSuccess) e = cudaMalloc(&dout, 8);
+  if (e == cudaSuccess && n > 0) e = cudaMemcpy(dt, t, (size_t)n * 8, cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) {
+    k_hc_ordered<<<1, 1024>>>(dt, n, dout);
+    e = cudaMemcpy(out, dout, 8, cudaMemcpyDeviceToHost);
+  }
+  cudaFree(dt);
+  cudaFree(dout);
+  return (int)e;
+}
 }
