@@ -8,18 +8,18 @@
 
 namespace cs {
 
-void build_cluster_plan(const HostMesh& me, int nrank, int warpsPerCta, ClusterPlanHost& p) {
+void build_cluster_plan(const HostMesh& me, int nrank, int warpsPerCta, ClusterPlanHost& p, bool domains) {
   p = ClusterPlanHost{};
   p.nrank = nrank;
   p.warpsPerCta = warpsPerCta;
   p.nwarps = nrank * warpsPerCta;
-  p.ok = nrank > 0 && warpsPerCta > 0 && me.D <= 3 * p.nwarps;
+  p.ok = nrank > 0 && warpsPerCta > 0 && (!domains || me.D <= 3 * p.nwarps);
   if (!p.ok) return;
   const int n = me.n;
   // phase B: domain slots per CTA and where each vertex's dofs live
   p.vDst.assign(n, -1);
   p.nSlots.assign(nrank, 0);
-  for (int dom = 0; dom < me.D; dom++) {
+  for (int dom = 0; domains && dom < me.D; dom++) {
     const int gw = dom % p.nwarps, u = dom / p.nwarps, r = gw / warpsPerCta, slot = u * warpsPerCta + gw % warpsPerCta;
     p.nSlots[r] = std::max(p.nSlots[r], slot + 1);
     for (int l = 0; l < me.domStart[dom + 1] - me.domStart[dom]; l++) {
@@ -28,7 +28,7 @@ void build_cluster_plan(const HostMesh& me, int nrank, int warpsPerCta, ClusterP
       p.vDst[v] = (r << 24) | (slot * 24 + l * 3);
     }
   }
-  for (int v = 0; v < n; v++)
+  for (int v = 0; domains && v < n; v++)
     if (p.vDst[v] < 0) { p.ok = false; return; }
   p.vb.resize(nrank + 1);
   for (int r = 0; r <= nrank; r++) p.vb[r] = (int)((int64_t)r * n / nrank);

@@ -89,6 +89,8 @@ struct ClusterPlanHost {
 
 // ok stays false when a halo needs more than 16-bit ids, when the domains do
 // not partition the vertices, or when some warp would own more than 3 domains.
-void build_cluster_plan(const HostMesh& me, int nrank, int warpsPerCta, ClusterPlanHost& p);
+// domains = false (the grid-wide kernel, whose phase B is not resident): no
+// domain slots, any number of domains per warp.
+void build_cluster_plan(const HostMesh& me, int nrank, int warpsPerCta, ClusterPlanHost& p, bool domains = true);
 
 }  // namespace cs

@@ -385,7 +385,7 @@ const int* Solver::contact_free_valid() {
 }
 
 bool Solver::step_graph(double h) {
-  if (!graphMode || !mixed() || mxCluster <= 0 || prof || profPhases) return false;
+  if (!graphMode || !mixed() || mxCluster <= 0 || mxGrid > 0 || prof || profPhases) return false;
   if (!gstep) gstep = new GraphStep();
   GraphStep& G = *gstep;
   if (G.failed) return false;

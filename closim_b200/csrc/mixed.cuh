@@ -72,6 +72,13 @@ int mx_cluster_size();
 bool mx_cluster_resident_ok(int clusterSize, size_t smemBytes);
 int mx_launch_pcg_cluster(const Dev& d, const MixBufs& mb, const ClPlan& plan, float* pA, float* pB, double* coef,
                           int maxIters, double tol, int clusterSize, cudaStream_t s);
+// The same PCG over the whole grid for sheets whose lists do not fit one
+// cluster's shared memory (mixed_cluster.cu): one CTA per rank of the plan, part
+// 8 x kMxGridMax doubles.
+constexpr int kMxGridMax = 256;
+bool mx_grid_ok(int ctas, size_t smemBytes);
+int mx_launch_pcg_grid(const Dev& d, const MixBufs& mb, const ClPlan& plan, float* pA, float* pB, double* coef,
+                       double* part, int maxIters, double tol, int ctas, cudaStream_t s);
 void mx_grad_final(const Dev& d, cudaStream_t s, int64_t* lc);
 void mx_energy_final(const Dev& d, cudaStream_t s, int64_t* lc);
 

@@ -990,6 +990,322 @@ __global__ void __launch_bounds__(kClT, 1) k_mx_pcg_cluster(ClArgs A) {
 #undef BC
 }
 
+// ---- the same solve on the whole grid ------------------------------------------------
+// Sheets whose per-CTA lists do not fit one cluster's shared memory (about
+// 4,300 vertices up): one CTA per SM owns a contiguous range of vertices, keeps
+// its triangles, hinges and incidence lists in shared memory for the whole solve
+// as the resident cluster kernel does, and exchanges p, Ap, r, z through L2 with
+// two cooperative grid barriers per iteration. Each vertex adds its incidences in
+// CSR order. On a B200, per iteration: 135 x 109 vertices (exact mode, floor
+// contact) 64 -> MXG_LARGE us against the cluster kernel gathering records from
+// global memory on 16 SMs; 256 x 256 (reference mode) 258 -> MXG_SPHERE us against the
+// element-scatter kernel with five grid barriers. Bound by the barriers and L2
+// round trips.
+struct GridArgs {
+  ClArgs c;
+  double* part;
+};
+
+template <int K>
+__device__ __forceinline__ void grid_put(const double* v, double* part, int row, double* wsm) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+  for (int k = 0; k < K; k++) {
+    double w = v[k];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) w += __shfl_down_sync(0xffffffffu, w, o);
+    if (lane == 0) wsm[k * 32 + warp] = w;
+  }
+  __syncthreads();
+  if (warp < K) {
+    double a = lane < (int)(blockDim.x >> 5) ? wsm[warp * 32 + lane] : 0.0;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) a += __shfl_down_sync(0xffffffffu, a, o);
+    if (lane == 0) part[(row + warp) * kMxGridMax + blockIdx.x] = a;
+  }
+}
+// Every warp adds the CTAs' partials in the same order: identical bits everywhere.
+__device__ __forceinline__ double grid_total(const double* part, int row) {
+  double s = 0;
+  for (int i = threadIdx.x & 31; i < (int)gridDim.x; i += 32) s += __ldcg(part + row * kMxGridMax + i);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  return s;
+}
+
+__global__ void __launch_bounds__(kClT, 1) k_mx_pcg_grid(GridArgs GA) {
+  cg::grid_group grid = cg::this_grid();
+  const ClArgs& A = GA.c;
+  double* const part = GA.part;
+  __shared__ double wsm[3 * 32];
+  __shared__ double sm[32];
+  const Dev& d = A.d;
+  const MixBufs& mb = A.mb;
+  const int n3 = d.n * 3;
+  const int rank = blockIdx.x, nrank = gridDim.x;
+  const int tid = rank * blockDim.x + threadIdx.x, nth = nrank * blockDim.x;
+  // neighbouring warps' domains lie in different CTAs, so a last partial round spreads
+  const int gwarp = (threadIdx.x >> 5) * nrank + rank, nwarps = nth >> 5;
+  const bool jacobi = d.precond == 0;
+  const float invH2 = (float)d.invH2;
+  const float C00 = mb.C00, C11 = mb.C11, C01 = mb.C01, G = mb.G;
+  extern __shared__ __align__(16) unsigned char cl_dyn[];
+  const ClPlan& P = A.plan;
+  const bool useHin = mb.hrec != nullptr;
+  const int vb0 = P.vb[rank], nOwn = P.vb[rank + 1] - vb0;
+  const int h0 = P.haloOff[rank], t0 = P.triOff[rank], g0 = P.hinOff[rank], i0 = P.incOff[vb0];
+  const int nHalo = P.haloOff[rank + 1] - h0, nTri = P.triOff[rank + 1] - t0;
+  const int nHin = useHin ? P.hinOff[rank + 1] - g0 : 0, nInc = P.incOff[vb0 + nOwn] - i0;
+  const ClSmem L = cl_smem_layout(nHalo, nTri, nHin, nInc, nOwn, 0, useHin, 0);
+  int* haloS = reinterpret_cast<int*>(cl_dyn + L.halo);
+  float4* pH = reinterpret_cast<float4*>(cl_dyn + L.pH);
+  float4* triD = reinterpret_cast<float4*>(cl_dyn + L.triD);
+  float* triO = reinterpret_cast<float*>(cl_dyn + L.triO);
+  float4* hinG = reinterpret_cast<float4*>(cl_dyn + L.hinG);
+  ushort4* hinL = reinterpret_cast<ushort4*>(cl_dyn + L.hinL);
+  float* hinS = reinterpret_cast<float*>(cl_dyn + L.hinS);
+  uint32_t* incS = reinterpret_cast<uint32_t*>(cl_dyn + L.inc);
+  int* incOffS = reinterpret_cast<int*>(cl_dyn + L.incOff);
+  int* incHinS = reinterpret_cast<int*>(cl_dyn + L.incHin);
+  int* ownHS = reinterpret_cast<int*>(cl_dyn + L.ownH);
+  float2* ownMP = reinterpret_cast<float2*>(cl_dyn + L.ownMP);
+  uint32_t* cOffS = reinterpret_cast<uint32_t*>(cl_dyn + L.cOff);
+  for (int i = threadIdx.x; i < nHalo; i += blockDim.x) haloS[i] = P.halo[h0 + i];
+  for (int sl = threadIdx.x; sl < nTri; sl += blockDim.x) {
+    const float4* src = reinterpret_cast<const float4*>(mb.tris) + (size_t)P.triId[t0 + sl] * 4;
+    const ushort4 lc = P.triLoc[t0 + sl];
+    float4 t3 = src[3];
+    t3.z = __uint_as_float((uint32_t)lc.x | ((uint32_t)lc.y << 16));
+    t3.w = __uint_as_float((uint32_t)lc.z);
+    triD[sl * 4] = src[0];
+    triD[sl * 4 + 1] = src[1];
+    triD[sl * 4 + 2] = src[2];
+    triD[sl * 4 + 3] = t3;
+  }
+  for (int sl = threadIdx.x; sl < nHin; sl += blockDim.x) {
+    const float4* src = mb.hrec + (size_t)P.hinId[g0 + sl] * 4;
+    hinG[sl * 3] = src[1];
+    hinG[sl * 3 + 1] = src[2];
+    hinG[sl * 3 + 2] = src[3];
+    hinL[sl] = P.hinLoc[g0 + sl];
+  }
+  for (int j = threadIdx.x; j < nInc; j += blockDim.x) incS[j] = P.inc[i0 + j];
+  for (int lv = threadIdx.x; lv <= nOwn; lv += blockDim.x) {
+    incOffS[lv] = P.incOff[vb0 + lv] - i0;
+    if (d.hasContact) cOffS[lv] = d.c.cOff[vb0 + lv];
+    if (lv < nOwn) {
+      incHinS[lv] = P.incHin[vb0 + lv] - i0;
+      ownHS[lv] = P.ownHalo[vb0 + lv];
+      ownMP[lv] = make_float2(d.mass[vb0 + lv], d.pinned[vb0 + lv] ? 1.f : 0.f);
+    }
+  }
+  DomFacts dfacts{{-1, -1, -1}, 0};
+  if (!jacobi && d.D <= 3 * nwarps) dfacts = cl_domain_facts(d, gwarp, nwarps);
+
+  double bb = 0, rr = 0, rz = 0;
+  for (int i = tid; i < n3; i += nth) {
+    const double bi = -d.g[i];
+    bb += bi * bi;
+  }
+  auto phaseB = [&](const float* pn, float alpha, bool init) {
+    if (jacobi)
+      for (int i = tid; i < n3; i += nth) cl_dof(d, mb, pn, alpha, init, i, rr, rz);
+    else
+      cl_all_domains(d, mb, pn, alpha, init, gwarp, nwarps, dfacts, rr, rz);
+  };
+  phaseB(nullptr, 0.f, true);
+  if (d.hasContact) {
+    const Contact& c = d.c;
+    for (int i = tid, na = n_active(c); i < na; i += nth) {
+      const double dist = js_max(frozen_dist(c, d.x, c.active[i]), 1e-12);
+      A.coef[i] = dist < c.dHat ? barrier_curvature(dist, c.dHat, c.kappa) : 0.0;
+    }
+  }
+  {
+    const double v3[3] = {bb, rr, rz};
+    grid_put<3>(v3, part, 1, wsm);
+  }
+  grid.sync();
+  const double bNorm = sqrt(grid_total(part, 1));
+  double residual = sqrt(grid_total(part, 2));
+  double rzCur = grid_total(part, 3);
+  const double absTol = fmax(A.tol * fmax(bNorm, 1e-12), 1e-12);
+  int iters = 0;
+  bool done = residual < absTol;
+  float beta = 0.f;
+  bool first = true;
+  float* pc = A.pA;  // p_{k-1}
+  float* pn = A.pB;  // p_k
+  int k = 0;
+  for (; !done && k < A.maxIters; k++) {
+    // ---- phase A: p_k on the halo, element HVPs, Ap_k, p.Ap ----
+    for (int i = threadIdx.x; i < nHalo; i += blockDim.x) {
+      const float3 pv = ld_p(mb.z, pc, beta, first, haloS[i]);
+      pH[i] = make_float4(pv.x, pv.y, pv.z, 0.f);
+    }
+    if (d.hasContact) cl_contact_records(d, mb, A.coef, pc, beta, first, cOffS[0], cOffS[nOwn]);
+    __syncthreads();
+    for (int e = threadIdx.x; e < nTri + nHin; e += blockDim.x) {
+      if (e < nTri) {
+        const float4 t3 = triD[e * 4 + 3];
+        const uint32_t l01 = __float_as_uint(t3.z), l2 = __float_as_uint(t3.w);
+        float g1[3], g2[3];
+        tri_hvp_g12(triD[e * 4], triD[e * 4 + 1], triD[e * 4 + 2], t3, pH[l01 & 0xffffu], pH[l01 >> 16], pH[l2], C00,
+                    C11, C01, G, g1, g2);
+        float* o = triO + e * 9;  // corner shares: -(g1 + g2), g1, g2
+#pragma unroll
+        for (int q = 0; q < 3; q++) {
+          o[q] = -(g1[q] + g2[q]);
+          o[3 + q] = g1[q];
+          o[6 + q] = g2[q];
+        }
+      } else {
+        const int sl = e - nTri;
+        const ushort4 l = hinL[sl];
+        const float4 P0 = pH[l.x], P1 = pH[l.y], P2 = pH[l.z], P3 = pH[l.w];
+        const float4 g0v = hinG[sl * 3], g1v = hinG[sl * 3 + 1], g2v = hinG[sl * 3 + 2];
+        hinS[sl] = g0v.x * P0.x + g0v.y * P0.y + g0v.z * P0.z + g0v.w * P1.x + g1v.x * P1.y + g1v.y * P1.z +
+                   g1v.z * P2.x + g1v.w * P2.y + g2v.x * P2.z + g2v.y * P3.x + g2v.z * P3.y + g2v.w * P3.z;
+      }
+    }
+    __syncthreads();
+    double pAp = 0;
+    for (int lv = threadIdx.x; lv < nOwn; lv += blockDim.x) {
+      float sp[3] = {0.f, 0.f, 0.f};
+      const int jh = incHinS[lv], je = incOffS[lv + 1];
+      for (int j = incOffS[lv]; j < jh; j++) {
+        const uint32_t rec = incS[j];
+        const float* o = triO + (rec >> 2) * 9 + (rec & 3) * 3;
+#pragma unroll
+        for (int q = 0; q < 3; q++) sp[q] += o[q];
+      }
+      if (useHin)
+        for (int j = jh; j < je; j++) {
+          const uint32_t rec = incS[j];
+          const float gs = hinS[rec >> 2];
+          const float* gc = reinterpret_cast<const float*>(hinG + (rec >> 2) * 3) + (rec & 3) * 3;
+          sp[0] += gs * gc[0];
+          sp[1] += gs * gc[1];
+          sp[2] += gs * gc[2];
+        }
+      double ch[3] = {0, 0, 0};
+      if (d.hasContact)
+        for (uint32_t q = cOffS[lv]; q < cOffS[lv + 1]; q++) {
+          const double* o = d.c.recScratch + (size_t)q * 3;
+          ch[0] += o[0]; ch[1] += o[1]; ch[2] += o[2];
+        }
+      const float4 pv = pH[ownHS[lv]];
+      const float2 mp = ownMP[lv];
+      const float pvv[3] = {pv.x, pv.y, pv.z};
+#pragma unroll
+      for (int q = 0; q < 3; q++) {
+        const int i = (vb0 + lv) * 3 + q;
+        float ap = mp.x * pvv[q] * invH2 + sp[q] + (float)ch[q];
+        if (mp.y != 0.f) ap = 0.f;
+        pn[i] = pvv[q];
+        mb.Ap[i] = ap;
+        pAp += (double)pvv[q] * ap;
+      }
+    }
+    grid_put<1>(&pAp, part, 0, wsm);
+    grid.sync();
+    const double pApT = grid_total(part, 0);
+    if (!(pApT > 1e-30)) { iters = k; done = true; break; }
+    // ---- phase B: x, r, z; r.r, r.z ----
+    rr = 0;
+    rz = 0;
+    phaseB(pn, (float)(rzCur / pApT), false);
+    {
+      const double v2[2] = {rr, rz};
+      grid_put<2>(v2, part, 1, wsm);
+    }
+    grid.sync();
+    residual = sqrt(grid_total(part, 1));
+    const double rzNew = grid_total(part, 2);
+    if (residual < absTol) { iters = k + 1; done = true; break; }
+    beta = (float)(rzNew / rzCur);
+    rzCur = rzNew;
+    first = false;
+    float* tmp = pc;
+    pc = pn;
+    pn = tmp;
+  }
+  if (!done) iters = A.maxIters;
+
+  // ---- descent safeguard + trust region in FP64 (newton.ts:152-179) ----
+  double gt = 0;
+  for (int i = tid; i < n3; i += nth) {
+    const double di = mb.x[i];
+    d.dx[i] = di;
+    gt += d.g[i] * di;
+  }
+  __syncthreads();
+  grid_put<1>(&gt, part, 4, wsm);
+  grid.sync();
+  double gtdx = grid_total(part, 4);
+  bool fallback = false;
+  if (!isfinite(gtdx) || gtdx >= 0) {
+    fallback = true;
+    gt = 0;
+    for (int i = tid; i < n3; i += nth) {
+      const double di = -d.g[i] / d.diag[i];
+      d.dx[i] = di;
+      gt += d.g[i] * di;
+    }
+    __syncthreads();
+    grid_put<1>(&gt, part, 5, wsm);
+    grid.sync();
+    gtdx = grid_total(part, 5);
+  }
+  double mxd = 0;
+  for (int i = tid; i < n3; i += nth) {
+    const double a = fabs(d.dx[i]);
+    if (a > mxd) mxd = a;
+  }
+  const double bmx = block_max(mxd, sm);
+  if (threadIdx.x == 0) part[6 * kMxGridMax + rank] = bmx;
+  grid.sync();
+  double maxDx = 0;
+  for (int i = 0; i < nrank; i++) {
+    const double v = __ldcg(part + 6 * kMxGridMax + i);
+    if (v > maxDx) maxDx = v;
+  }
+  if (maxDx > 0.002) {
+    const double s = 0.002 / maxDx;
+    for (int i = tid; i < n3; i += nth) d.dx[i] *= s;
+    gtdx *= s;
+  }
+  if (rank == 0 && threadIdx.x == 0) {
+    d.scal[S_PCG_ITERS] = iters;
+    d.scal[S_PCG_RES] = residual;
+    d.scal[S_GTDX] = gtdx;
+    d.scal[S_FALLBACK] = fallback ? 1 : 0;
+    d.scal[S_MAXDX] = maxDx;
+  }
+}
+
+bool mx_grid_ok(int ctas, size_t smemBytes) {
+  if (ctas < 1 || ctas > kMxGridMax || smemBytes > (size_t)kClMaxDynSmem) return false;
+  int dev = 0, sms = 0, per = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  // the largest the kernel may take: one limit for every mesh of the process
+  const bool ok = cudaFuncSetAttribute(k_mx_pcg_grid, cudaFuncAttributeMaxDynamicSharedMemorySize, kClMaxDynSmem) ==
+                      cudaSuccess &&
+                  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_mx_pcg_grid, kClT, smemBytes) == cudaSuccess &&
+                  per * sms >= ctas;
+  cudaGetLastError();
+  return ok;
+}
+
+int mx_launch_pcg_grid(const Dev& d, const MixBufs& mb, const ClPlan& plan, float* pA, float* pB, double* coef,
+                       double* part, int maxIters, double tol, int ctas, cudaStream_t s) {
+  GridArgs a{{d, mb, pA, pB, coef, maxIters, tol, plan}, part};
+  void* args[] = {&a};
+  return (int)cudaLaunchCooperativeKernel((void*)k_mx_pcg_grid, dim3(ctas), dim3(kClT), args, (size_t)plan.smemBytes,
+                                          s);
+}
+
 // Largest cluster (16, then 8, 4, 2, 1 CTAs) the device can co-schedule for
 // this kernel; 0 when none.
 int mx_cluster_size() {

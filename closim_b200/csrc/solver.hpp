@@ -117,6 +117,9 @@ class Solver {
   DBuf<uint32_t> triSlot;
   MixBufs mb{};
   int mxBlocks = 1;
+  int mxGrid = 0;     // CTAs of the resident grid-wide PCG (0: not used)
+  size_t mxGridSmem[2] = {0, 0};  // its dynamic shared memory without / with the bending term
+  DBuf<double> mxGridPart;
   int mxCluster = 0;  // CTAs of the one-cluster PCG (0: grid-wide cooperative PCG)
   // Per-CTA element lists of the one-cluster PCG's resident phase A; clRes[k]
   // (k = 1 with the Gauss-Newton bending term) says whether they fit.
@@ -320,8 +323,14 @@ class Solver {
       const char* env = std::getenv("CLOSIM_MX_PCG");
       const bool wantCluster = env ? std::string(env) == "cluster" : mesh.n <= 20000;
       mxCluster = wantCluster && mesh.maxDomain <= 8 ? mx_cluster_size() : 0;
+      mb.vrec = nullptr;
+      mb.triSlot = nullptr;
       if (mxCluster > 0) {
         fp2.alloc(n3);
+        build_cluster_resident();
+      }
+      build_grid_resident(env && std::string(env) == "cluster");
+      if (mxCluster > 0 && mxGrid == 0) {
         std::vector<uint32_t> slot(3 * (size_t)cm.m);
         for (size_t q = 0; q < mesh.memRec.size(); q++) {
           const uint32_t rec = mesh.memRec[q];
@@ -331,7 +340,6 @@ class Solver {
         fvrec.alloc(5 * 3 * (size_t)cm.m);
         mb.vrec = fvrec.p;
         mb.triSlot = triSlot.p;
-        build_cluster_resident();
       }
     }
     upload_pins();
@@ -504,6 +512,12 @@ class Solver {
                   opts.pcg_max_iters, newtonTol, adjOut.p};
         CK((cudaError_t)newton_exact_solve(a, adj_grid_blocks(d), stream));
         lc += 3;
+      } else if (mixed() && mxGrid > 0) {
+        ClPlan plan = clPlan;
+        plan.smemBytes = (int)mxGridSmem[mb.hrec ? 1 : 0];
+        CK((cudaError_t)mx_launch_pcg_grid(d, mb, plan, fp.p, fp2.p, d.hasContact ? d.c.dd : nullptr, mxGridPart.p,
+                                           opts.pcg_max_iters,
+                                           exactMixed ? std::max(newtonTol, kMixedTolFloor) : 1e-3, mxGrid, stream));
       } else if (mixed() && mxCluster > 0)
         CK((cudaError_t)mx_launch_pcg_cluster(d, mb, cluster_plan_for(mb), fp.p, fp2.p, d.hasContact ? d.c.dd : nullptr,
                                               opts.pcg_max_iters, exactMixed ? std::max(newtonTol, kMixedTolFloor) : 1e-3,
@@ -708,6 +722,36 @@ class Solver {
     clRes[1] = mx_cluster_resident_ok(mxCluster, clSmem[1]);
     clRes[0] = mx_cluster_resident_ok(mxCluster, clSmem[0]);
     if (!clRes[0] && !clRes[1]) return;
+    upload_cluster_plan();
+  }
+  // Sheets past kMxGridN vertices whose lists do not fit one cluster: the
+  // grid-wide resident PCG (mixed_cluster.cu), one CTA per SM. Below that the
+  // cluster's barrier and the captured step (a cooperative launch cannot be in
+  // one) are worth more: a 65 x 65 sheet is the first that does not fit.
+  static constexpr int kMxGridN = 4096;
+  void build_grid_resident(bool forceCluster) {
+    mxGrid = 0;
+    if (mxCluster <= 0) {
+      clRes[0] = clRes[1] = false;
+      clPlan = ClPlan{};
+    }
+    if (forceCluster || clRes[0] || clRes[1] || mesh.n <= kMxGridN || mesh.maxDomain > 8) return;
+    const char* env = std::getenv("CLOSIM_MX_RESIDENT");
+    if (env && std::string(env) == "0") return;
+    int sms = 0;
+    CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
+    const int ctas = std::min(std::min(sms, kMxGridMax), (mesh.n + 31) / 32);
+    build_cluster_plan(mesh, ctas, kClWarps, clHost, false);
+    const size_t most = mxCluster > 0 ? clHost.smemHinge : clHost.smemNoHinge;  // exact mode is FP64 without a cluster
+    if (!clHost.ok || !mx_grid_ok(ctas, most)) return;
+    mxGrid = ctas;
+    mxGridSmem[0] = clHost.smemNoHinge;
+    mxGridSmem[1] = clHost.smemHinge;
+    mxGridPart.alloc(8 * (size_t)kMxGridMax);
+    if (fp2.n < 3 * (size_t)mesh.n) fp2.alloc(3 * (size_t)mesh.n);
+    upload_cluster_plan();
+  }
+  void upload_cluster_plan() {
     auto up = [&](DBuf<int>& b, const std::vector<int>& v) {
       b.alloc(std::max<size_t>(v.size(), 1));
       b.upload(v.data(), v.size(), stream);
