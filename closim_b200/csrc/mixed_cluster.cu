@@ -347,31 +347,26 @@ __device__ __forceinline__ void cl_domains(const Dev& d, const MixBufs& mb, cons
       rr += (double)ri * ri;
     }
   }
-  // row `lane` of each 24x24 inverse: 96 bytes, in two halves of three 16-byte
-  // loads (all K domains' halves in flight together)
+  // Row `lane` of each 24x24 inverse, read as column `lane` of the symmetric
+  // matrix: a warp's loads are then contiguous (a row per lane touched 24 cache
+  // lines an instruction). Twelve loads of every domain in flight at a time.
   float zk[K];
 #pragma unroll
   for (int u = 0; u < K; u++) zk[u] = 0.f;
 #pragma unroll
   for (int h = 0; h < 2; h++) {
-    float4 L[K][3];
+    float Lc[K][12];
 #pragma unroll
     for (int u = 0; u < K; u++) {
-      const float4* Li = reinterpret_cast<const float4*>(mb.Linv + (size_t)(dom0 + u * step) * 576) + lane * 6 + h * 3;
+      const float* Li = mb.Linv + (size_t)(dom0 + u * step) * 576 + h * 12 * 24 + lane;
 #pragma unroll
-      for (int j4 = 0; j4 < 3; j4++) L[u][j4] = f.gi[u] >= 0 ? __ldg(Li + j4) : make_float4(0.f, 0.f, 0.f, 0.f);
+      for (int j = 0; j < 12; j++) Lc[u][j] = f.gi[u] >= 0 ? __ldg(Li + j * 24) : 0.f;
     }
 #pragma unroll
-    for (int u = 0; u < K; u++) {
+    for (int u = 0; u < K; u++)
 #pragma unroll
-      for (int j4 = 0; j4 < 3; j4++) {
-        const int c = 4 * (h * 3 + j4);
-        zk[u] = fmaf(L[u][j4].x, __shfl_sync(0xffffffffu, rv[u], c), zk[u]);
-        zk[u] = fmaf(L[u][j4].y, __shfl_sync(0xffffffffu, rv[u], c + 1), zk[u]);
-        zk[u] = fmaf(L[u][j4].z, __shfl_sync(0xffffffffu, rv[u], c + 2), zk[u]);
-        zk[u] = fmaf(L[u][j4].w, __shfl_sync(0xffffffffu, rv[u], c + 3), zk[u]);
-      }
-    }
+      for (int j = 0; j < 12; j++)
+        zk[u] = fmaf(Lc[u][j], __shfl_sync(0xffffffffu, rv[u], h * 12 + j), zk[u]);
   }
 #pragma unroll
   for (int u = 0; u < K; u++) {
@@ -997,8 +992,8 @@ __global__ void __launch_bounds__(kClT, 1) k_mx_pcg_cluster(ClArgs A) {
 // as the resident cluster kernel does, and exchanges p, Ap, r, z through L2 with
 // two cooperative grid barriers per iteration. Each vertex adds its incidences in
 // CSR order. On a B200, per iteration: 135 x 109 vertices (exact mode, floor
-// contact) 64 -> MXG_LARGE us against the cluster kernel gathering records from
-// global memory on 16 SMs; 256 x 256 (reference mode) 258 -> MXG_SPHERE us against the
+// contact) 64 -> 16 us against the cluster kernel gathering records from
+// global memory on 16 SMs; 256 x 256 (reference mode) 258 -> 28 us against the
 // element-scatter kernel with five grid barriers. Bound by the barriers and L2
 // round trips.
 struct GridArgs {
@@ -1024,14 +1019,27 @@ __device__ __forceinline__ void grid_put(const double* v, double* part, int row,
     if (lane == 0) part[(row + warp) * kMxGridMax + blockIdx.x] = a;
   }
 }
-// Every warp adds the CTAs' partials in the same order: identical bits everywhere.
-__device__ __forceinline__ double grid_total(const double* part, int row) {
-  double s = 0;
-  for (int i = threadIdx.x & 31; i < (int)gridDim.x; i += 32) s += __ldcg(part + row * kMxGridMax + i);
+// After the barrier, warp k of each CTA adds row `row + k` of the CTAs' partials in
+// one order, identical bits everywhere. (Every warp of every CTA reading the
+// partials instead queued 12,000 requests on a few L2 lines: 10,000 cycles.)
+template <int K>
+__device__ __forceinline__ void grid_totals(const double* part, int row, double* out, double* tot) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (warp < K) {
+    double s = 0;
+    for (int i = lane; i < (int)gridDim.x; i += 32) s += __ldcg(part + (row + warp) * kMxGridMax + i);
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  return s;
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane == 0) tot[warp] = s;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < K; k++) out[k] = tot[k];
 }
+
+constexpr int kGridDoms = 4;         // Schwarz domains per warp whose dofs are kept on chip
+constexpr int kGridSumWarps = 8;     // warps that sum vertices with many contacts
+constexpr uint32_t kGridLight = 4;   // contact records a vertex's own thread sums
 
 __global__ void __launch_bounds__(kClT, 1) k_mx_pcg_grid(GridArgs GA) {
   cg::grid_group grid = cg::this_grid();
@@ -1039,6 +1047,9 @@ __global__ void __launch_bounds__(kClT, 1) k_mx_pcg_grid(GridArgs GA) {
   double* const part = GA.part;
   __shared__ double wsm[3 * 32];
   __shared__ double sm[32];
+  __shared__ double tot[2][4];  // totals, alternating so that a slow reader is never overtaken
+  __shared__ int domS[kGridDoms][kClT];      // per warp and domain: the lane's dof (bit 30: pinned; -1: none)
+  __shared__ double rec32[kGridSumWarps][96];  // per summing warp: 32 contact records' shares
   const Dev& d = A.d;
   const MixBufs& mb = A.mb;
   const int n3 = d.n * 3;
@@ -1099,8 +1110,20 @@ __global__ void __launch_bounds__(kClT, 1) k_mx_pcg_grid(GridArgs GA) {
       ownMP[lv] = make_float2(d.mass[vb0 + lv], d.pinned[vb0 + lv] ? 1.f : 0.f);
     }
   }
-  DomFacts dfacts{{-1, -1, -1}, 0};
-  if (!jacobi && d.D <= 3 * nwarps) dfacts = cl_domain_facts(d, gwarp, nwarps);
+  const bool domsOnChip = d.D <= kGridDoms * nwarps;
+  if (!jacobi && domsOnChip)
+    for (int u = 0; u < kGridDoms; u++) {
+      const int dom = gwarp + u * nwarps, lane = threadIdx.x & 31;
+      int gi = -1;
+      if (dom < d.D) {
+        const int start = d.domStart[dom], dv = d.domStart[dom + 1] - start;
+        if (lane < 3 * dv) {
+          gi = d.domVerts[start + lane / 3] * 3 + lane % 3;
+          if (d.pinned[gi / 3]) gi |= 1 << 30;
+        }
+      }
+      domS[u][threadIdx.x] = gi;
+    }
 
   double bb = 0, rr = 0, rz = 0;
   for (int i = tid; i < n3; i += nth) {
@@ -1110,8 +1133,25 @@ __global__ void __launch_bounds__(kClT, 1) k_mx_pcg_grid(GridArgs GA) {
   auto phaseB = [&](const float* pn, float alpha, bool init) {
     if (jacobi)
       for (int i = tid; i < n3; i += nth) cl_dof(d, mb, pn, alpha, init, i, rr, rz);
-    else
-      cl_all_domains(d, mb, pn, alpha, init, gwarp, nwarps, dfacts, rr, rz);
+    else {
+      for (int dom = gwarp, u = 0; dom < d.D; dom += 2 * nwarps, u += 2) {
+        DomFacts f;
+        if (domsOnChip) {
+          f.meta = 0;
+#pragma unroll
+          for (int v = 0; v < 2; v++) {
+            const int gi = u + v < kGridDoms ? domS[u + v][threadIdx.x] : -1;
+            f.gi[v] = gi < 0 ? -1 : gi & ~(1 << 30);
+            if (gi >= 0 && (gi >> 30)) f.meta |= 1 << v;
+            f.meta |= (__popc(__ballot_sync(0xffffffffu, gi >= 0)) / 3) << (8 + 4 * v);
+          }
+        } else {
+          f = cl_domain_facts(d, dom, nwarps);
+        }
+        if (dom + nwarps < d.D) cl_domains<2>(d, mb, pn, alpha, init, dom, nwarps, f, rr, rz);
+        else cl_domains<1>(d, mb, pn, alpha, init, dom, nwarps, f, rr, rz);
+      }
+    }
   };
   phaseB(nullptr, 0.f, true);
   if (d.hasContact) {
@@ -1126,9 +1166,11 @@ __global__ void __launch_bounds__(kClT, 1) k_mx_pcg_grid(GridArgs GA) {
     grid_put<3>(v3, part, 1, wsm);
   }
   grid.sync();
-  const double bNorm = sqrt(grid_total(part, 1));
-  double residual = sqrt(grid_total(part, 2));
-  double rzCur = grid_total(part, 3);
+  double t3[3];
+  grid_totals<3>(part, 1, t3, tot[0]);
+  const double bNorm = sqrt(t3[0]);
+  double residual = sqrt(t3[1]);
+  double rzCur = t3[2];
   const double absTol = fmax(A.tol * fmax(bNorm, 1e-12), 1e-12);
   int iters = 0;
   bool done = residual < absTol;
@@ -1168,6 +1210,35 @@ __global__ void __launch_bounds__(kClT, 1) k_mx_pcg_grid(GridArgs GA) {
                    g1v.z * P2.x + g1v.w * P2.y + g2v.x * P2.z + g2v.y * P3.x + g2v.z * P3.y + g2v.w * P3.z;
       }
     }
+    if (d.hasContact) {
+      // A vertex may sit in hundreds of contacts: a warp sums its shares in order,
+      // 32 records loaded together, one lane per component (into the first three
+      // doubles of their scratch).
+      const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+      for (int lv = warp < kGridSumWarps ? warp : nOwn; lv < nOwn; lv += kGridSumWarps) {
+        const uint32_t q0 = cOffS[lv], q1 = cOffS[lv + 1];
+        if (q1 - q0 <= kGridLight) continue;
+        double* src = d.c.recScratch + (size_t)q0 * 3;
+        const int total = (int)(q1 - q0) * 3;
+        double* buf = rec32[warp];
+        double nx[3], acc = 0;
+#pragma unroll
+        for (int u = 0; u < 3; u++) nx[u] = u * 32 + lane < total ? src[u * 32 + lane] : 0.0;
+        for (int i = 0; i < total; i += 96) {
+          __syncwarp();
+#pragma unroll
+          for (int u = 0; u < 3; u++) buf[u * 32 + lane] = nx[u];
+          __syncwarp();
+#pragma unroll
+          for (int u = 0; u < 3; u++) nx[u] = i + 96 + u * 32 + lane < total ? src[i + 96 + u * 32 + lane] : 0.0;
+          if (lane < 3) {
+#pragma unroll 8
+            for (int u = 0; u < 32; u++) acc += buf[u * 3 + lane];  // zeros past the end
+          }
+        }
+        if (lane < 3) src[lane] = acc;
+      }
+    }
     __syncthreads();
     double pAp = 0;
     for (int lv = threadIdx.x; lv < nOwn; lv += blockDim.x) {
@@ -1190,8 +1261,8 @@ __global__ void __launch_bounds__(kClT, 1) k_mx_pcg_grid(GridArgs GA) {
         }
       double ch[3] = {0, 0, 0};
       if (d.hasContact)
-        for (uint32_t q = cOffS[lv]; q < cOffS[lv + 1]; q++) {
-          const double* o = d.c.recScratch + (size_t)q * 3;
+        for (uint32_t q0 = cOffS[lv], cnt = cOffS[lv + 1] - q0, u = 0; u < (cnt > kGridLight ? 1 : cnt); u++) {
+          const double* o = d.c.recScratch + (size_t)(q0 + u) * 3;
           ch[0] += o[0]; ch[1] += o[1]; ch[2] += o[2];
         }
       const float4 pv = pH[ownHS[lv]];
@@ -1209,7 +1280,8 @@ __global__ void __launch_bounds__(kClT, 1) k_mx_pcg_grid(GridArgs GA) {
     }
     grid_put<1>(&pAp, part, 0, wsm);
     grid.sync();
-    const double pApT = grid_total(part, 0);
+    double pApT;
+    grid_totals<1>(part, 0, &pApT, tot[1]);
     if (!(pApT > 1e-30)) { iters = k; done = true; break; }
     // ---- phase B: x, r, z; r.r, r.z ----
     rr = 0;
@@ -1220,8 +1292,10 @@ __global__ void __launch_bounds__(kClT, 1) k_mx_pcg_grid(GridArgs GA) {
       grid_put<2>(v2, part, 1, wsm);
     }
     grid.sync();
-    residual = sqrt(grid_total(part, 1));
-    const double rzNew = grid_total(part, 2);
+    double t2[2];
+    grid_totals<2>(part, 1, t2, tot[0]);
+    residual = sqrt(t2[0]);
+    const double rzNew = t2[1];
     if (residual < absTol) { iters = k + 1; done = true; break; }
     beta = (float)(rzNew / rzCur);
     rzCur = rzNew;
@@ -1242,7 +1316,8 @@ __global__ void __launch_bounds__(kClT, 1) k_mx_pcg_grid(GridArgs GA) {
   __syncthreads();
   grid_put<1>(&gt, part, 4, wsm);
   grid.sync();
-  double gtdx = grid_total(part, 4);
+  double gtdx;
+  grid_totals<1>(part, 4, &gtdx, tot[1]);
   bool fallback = false;
   if (!isfinite(gtdx) || gtdx >= 0) {
     fallback = true;
@@ -1255,7 +1330,7 @@ __global__ void __launch_bounds__(kClT, 1) k_mx_pcg_grid(GridArgs GA) {
     __syncthreads();
     grid_put<1>(&gt, part, 5, wsm);
     grid.sync();
-    gtdx = grid_total(part, 5);
+    grid_totals<1>(part, 5, &gtdx, tot[0]);
   }
   double mxd = 0;
   for (int i = tid; i < n3; i += nth) {
@@ -1285,12 +1360,13 @@ __global__ void __launch_bounds__(kClT, 1) k_mx_pcg_grid(GridArgs GA) {
 }
 
 bool mx_grid_ok(int ctas, size_t smemBytes) {
-  if (ctas < 1 || ctas > kMxGridMax || smemBytes > (size_t)kClMaxDynSmem) return false;
+  constexpr int kMaxDyn = 227 * 1024 - 17 * 1024;  // beside the kernel's static shared memory
+  if (ctas < 1 || ctas > kMxGridMax || smemBytes > (size_t)kMaxDyn) return false;
   int dev = 0, sms = 0, per = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   // the largest the kernel may take: one limit for every mesh of the process
-  const bool ok = cudaFuncSetAttribute(k_mx_pcg_grid, cudaFuncAttributeMaxDynamicSharedMemorySize, kClMaxDynSmem) ==
+  const bool ok = cudaFuncSetAttribute(k_mx_pcg_grid, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDyn) ==
                       cudaSuccess &&
                   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_mx_pcg_grid, kClT, smemBytes) == cudaSuccess &&
                   per * sms >= ctas;
