@@ -20,9 +20,13 @@
 // takes (the derivative of bending.ts:7-16).
 #include <cooperative_groups.h>
 
+#include <map>
+#include <mutex>
+
 #include "adjoint.cuh"
 #include "adjoint_math.cuh"
 #include "contact.cuh"
+#include "schwarz64.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -32,9 +36,9 @@ __device__ __forceinline__ void load3(const double* x, int v, double o[3]) {
   o[0] = x[v * 3]; o[1] = x[v * 3 + 1]; o[2] = x[v * 3 + 2];
 }
 
-__device__ __forceinline__ double adj_total(const Dev& d, int row, double* bc) {
+__device__ __forceinline__ double adj_total(const Dev& d, int row, int blocks, double* bc) {
   if (threadIdx.x < 32) {
-    const double s = warp_sum_partials(d.part + row * d.partStride, gridDim.x);
+    const double s = warp_sum_partials(d.part + row * d.partStride, blocks);
     if (threadIdx.x == 0) bc[0] = s;
   }
   __syncthreads();
@@ -45,63 +49,6 @@ __device__ __forceinline__ double adj_total(const Dev& d, int row, double* bc) {
 __device__ __forceinline__ void adj_put(const Dev& d, int row, double v, double* sm) {
   const double b = block_sum(v, sm);
   if (threadIdx.x == 0) d.part[row * d.partStride + blockIdx.x] = b;
-}
-
-// z = M^-1 r on one Schwarz domain with the FP64 factors in d.L (the
-// forward's Cholesky factor, or an inverse diagonal where it failed).
-__device__ double adj_schwarz(const Dev& d, const double* r, double* z, int dom) {
-  const int start = d.domStart[dom], dv = d.domStart[dom + 1] - start, dw = dv * 3;
-  const double* L = d.L + (size_t)dom * 576;
-  double rhs[24], y[24], sol[24];
-  for (int l = 0; l < dv; l++) {
-    const int v = d.domVerts[start + l];
-    for (int k = 0; k < 3; k++) rhs[l * 3 + k] = r[v * 3 + k];
-  }
-  if (d.domFlag[dom]) {
-    for (int i = 0; i < dw; i++) {
-      double s = rhs[i];
-      for (int j = 0; j < i; j++) s -= L[i * 24 + j] * y[j];
-      y[i] = s / L[i * 24 + i];
-    }
-    for (int i = dw - 1; i >= 0; i--) {
-      double s = y[i];
-      for (int j = i + 1; j < dw; j++) s -= L[j * 24 + i] * sol[j];
-      sol[i] = s / L[i * 24 + i];
-    }
-  } else {
-    for (int i = 0; i < dw; i++) {
-      double s = 0;
-      for (int j = 0; j < dw; j++) s += L[i * 24 + j] * rhs[j];
-      sol[i] = s;
-    }
-  }
-  double rz = 0;
-  for (int l = 0; l < dv; l++) {
-    const int v = d.domVerts[start + l];
-    const bool pin = d.pinned[v];
-    for (int k = 0; k < 3; k++) {
-      const double zz = pin ? 0.0 : sol[l * 3 + k];
-      z[v * 3 + k] = zz;
-      rz += rhs[l * 3 + k] * zz;
-    }
-  }
-  return rz;
-}
-
-__device__ __forceinline__ double adj_precond(const Dev& d, const AdjArgs& A, int tid, int nth) {
-  double rz = 0;
-  if (d.precond >= 1) {  // one-level Schwarz factors (the two-level coarse term is not applied here)
-    for (int dom = tid; dom < d.D; dom += nth) rz += adj_schwarz(d, A.r, A.z, dom);
-  } else {
-    for (int i = tid; i < d.n * 3; i += nth) {
-      const double ri = A.r[i];
-      double zi = d.diag[i] > 1e-12 ? ri / d.diag[i] : ri;
-      if (d.pinned[i / 3]) zi = 0;
-      A.z[i] = zi;
-      rz += ri * zi;
-    }
-  }
-  return rz;
 }
 
 // Membrane HVP in FP64 (membrane-hvp.ts:18-75). With psd set, the second
@@ -147,114 +94,174 @@ __device__ __forceinline__ void mem_hvp64(const double* x0, const double* x1, co
   }
 }
 
-// H p into A.Ap (element pass, grid barrier, gather); returns the partial p.Hp.
-__device__ double adj_hvp(cg::grid_group& grid, const Dev& d, const AdjArgs& A, int tid, int nth) {
-  for (int t = tid; t < d.m; t += nth) {
-    const uint32_t i0 = d.idx[t * 3], i1 = d.idx[t * 3 + 1], i2 = d.idx[t * 3 + 2];
-    double x0[3], x1[3], x2[3], v0[3], v1[3], v2[3];
-    load3(d.x, i0, x0); load3(d.x, i1, x1); load3(d.x, i2, x2);
-    load3(A.p, i0, v0); load3(A.p, i1, v1); load3(A.p, i2, v2);
-    const float4 iv = d.inv[t];
-    double o[9];
-    mem_hvp64(x0, x1, x2, v0, v1, v2, iv.x, iv.y, iv.z, iv.w, d.area[t], d.mat, A.psd != 0, o);
-    for (int k = 0; k < 9; k++) A.tri9[(size_t)t * 9 + k] = o[k];
-  }
-  if (A.kb > 0)
-    for (int hh = tid; hh < d.hg; hh += nth) {
-      const int4 hv = d.hinge[hh];
-      double q[12], v[12], o[12];
-      load3(d.x, hv.x, q); load3(d.x, hv.y, q + 3); load3(d.x, hv.z, q + 6); load3(d.x, hv.w, q + 9);
-      load3(A.p, hv.x, v); load3(A.p, hv.y, v + 3); load3(A.p, hv.z, v + 6); load3(A.p, hv.w, v + 9);
-      bend_hvp(q, v, d.hmeta[hh * 3], d.hmeta[hh * 3 + 1], d.hmeta[hh * 3 + 2], A.kb, o);
-      for (int k = 0; k < 12; k++) A.hin12[(size_t)hh * 12 + k] = o[k];
-    }
-  if (d.hasContact) contact_hvp_coeffs(d, A.p, tid, nth);
-  grid.sync();
-  double pAp = 0;
-  for (int v = tid; v < d.n; v += nth) {
-    double s[3] = {0, 0, 0};
-    for (uint32_t k = d.memOff[v]; k < d.memOff[v + 1]; k++) {
-      const uint32_t rec = d.memRec[k];
-      const double* e = A.tri9 + (size_t)(rec >> 2) * 9 + (rec & 3) * 3;
-      s[0] += e[0]; s[1] += e[1]; s[2] += e[2];
-    }
-    if (A.kb > 0)
-      for (uint32_t k = d.hinOff[v]; k < d.hinOff[v + 1]; k++) {
-        const uint32_t rec = d.hinRec[k];
-        const double* e = A.hin12 + (size_t)(rec >> 2) * 12 + (rec & 3) * 3;
-        s[0] += e[0]; s[1] += e[1]; s[2] += e[2];
-      }
-    double ch[3] = {0, 0, 0};
-    if (d.hasContact) contact_hvp_gather(d, v, ch);
-    const double M = d.mass[v];
-    const bool pin = d.pinned[v];
-    for (int k = 0; k < 3; k++) {
-      const int i = v * 3 + k;
-      const double ap = pin ? 0.0 : M * A.p[i] * d.invH2 + s[k] + ch[k];
-      A.Ap[i] = ap;
-      pAp += A.p[i] * ap;
-    }
-  }
-  return pAp;
-}
-
-// PCG on H mu = rhs (pcg.ts's recurrence, FP64 tree reductions), one
-// cooperative launch. out: [iterations, final residual, |rhs|].
-__global__ void __launch_bounds__(kThreads) k_adj_pcg(AdjArgs A) {
-  cg::grid_group grid = cg::this_grid();
+// PCG on H mu = rhs (pcg.ts's recurrence, FP64 tree reductions), one launch of C
+// CTAs. out: [iterations, final residual, |rhs|].
+//
+// Small sheets are bound by latency: the hinges' dual-number products and the
+// domains' substitutions are long dependent chains, and every phase ends in a
+// barrier. So all C CTAs share the elements and the domains (a warp each), and up
+// to 16 reducing blocks run as one thread-block cluster with its hardware barrier.
+// The reductions keep the shape of `blocks` blocks of kThreads, whatever C is: the
+// first `blocks` CTAs hold the vectors' elements, so results do not depend on how
+// the rest of the work is spread. On a B200, 19 x 16 vertices with Schwarz took
+// 65 us an iteration with a thread per domain on 4 cooperative blocks, 27 us now;
+// a fit's forward and backward pass 1.25 -> 0.51 s, the same bits.
+template <bool CLUSTER>
+__global__ void __launch_bounds__(kThreads) k_adj_pcg(AdjArgs A, int blocks) {
   __shared__ double sm[32];
   __shared__ double bc[2];
+  auto barrier = [&]() {
+    if constexpr (CLUSTER) cg::this_cluster().sync();
+    else cg::this_grid().sync();
+  };
   const Dev& d = A.d;
+  const bool reducing = (int)blockIdx.x < blocks;
   const int n3 = d.n * 3;
-  const int tid = blockIdx.x * blockDim.x + threadIdx.x, nth = gridDim.x * blockDim.x;
+  const int tid = blockIdx.x * blockDim.x + threadIdx.x, nthAll = gridDim.x * blockDim.x;
+  const int nth = blocks * blockDim.x;
+  const int i0 = reducing ? tid : n3, v0 = reducing ? tid : d.n;
+  const int gwarp = (threadIdx.x >> 5) * gridDim.x + blockIdx.x, nwarps = nthAll >> 5;
+  auto put = [&](int row, double v) {
+    if (reducing) adj_put(d, row, v, sm);
+  };
+  auto total = [&](int row) { return adj_total(d, row, blocks, bc); };
+  // z = M^-1 r (one-level Schwarz factors, or Jacobi); this thread's share of r.z.
+  // (The two-level coarse term is not applied here.)
+  auto precond = [&]() {
+    double rz = 0;
+    if (d.precond >= 1) {
+      for (int dom = gwarp; dom < d.D; dom += nwarps) {
+        const double s = domain_solve(d.L + (size_t)dom * 576, A.r, A.z, nullptr, domain_lane(d, dom));
+        if ((threadIdx.x & 31) == 0) A.domRz[dom] = s;
+      }
+      barrier();
+      for (int dom = reducing ? tid : d.D; dom < d.D; dom += nth) rz += __ldcg(A.domRz + dom);
+    } else {
+      for (int i = i0; i < n3; i += nth) {
+        const double ri = A.r[i];
+        double zi = d.diag[i] > 1e-12 ? ri / d.diag[i] : ri;
+        if (d.pinned[i / 3]) zi = 0;
+        A.z[i] = zi;
+        rz += ri * zi;
+      }
+    }
+    return rz;
+  };
   double bb = 0, rr = 0;
-  for (int i = tid; i < n3; i += nth) {
+  for (int i = i0; i < n3; i += nth) {
     const double ri = d.pinned[i / 3] ? 0.0 : A.rhs[i];
     bb += A.rhs[i] * A.rhs[i];
     A.r[i] = ri;
     A.mu[i] = 0;
     rr += ri * ri;
   }
-  grid.sync();
-  const double rz0 = adj_precond(d, A, tid, nth);
-  adj_put(d, 0, bb, sm);
-  adj_put(d, 1, rr, sm);
-  adj_put(d, 2, rz0, sm);
-  grid.sync();
-  for (int i = tid; i < n3; i += nth) A.p[i] = A.z[i];
-  const double bNorm = sqrt(adj_total(d, 0, bc));
-  double residual = sqrt(adj_total(d, 1, bc));
-  double rz = adj_total(d, 2, bc);
+  barrier();
+  const double rz0 = precond();
+  put(0, bb);
+  put(1, rr);
+  put(2, rz0);
+  barrier();
+  for (int i = i0; i < n3; i += nth) A.p[i] = __ldcg(A.z + i);
+  const double bNorm = sqrt(total(0));
+  double residual = sqrt(total(1));
+  double rz = total(2);
   const double absTol = fmax(A.tol * bNorm, 1e-300);
   int k = 0;
   bool done = !(residual > absTol);
-  grid.sync();
+  barrier();
   for (; !done && k < A.maxIters; k++) {
-    const double pAp = adj_hvp(grid, d, A, tid, nth);
-    adj_put(d, 3, pAp, sm);
-    grid.sync();
-    const double pApT = adj_total(d, 3, bc);
+    // ---- H p: elements on every CTA, then the vertex sums ----
+    const int nHin = A.kb > 0 ? d.hg : 0;
+    // whole warps of one kind of element: hinges first, they take longest
+    const int hinPad = (nHin + 31) & ~31;
+    for (int e = tid; e < hinPad + d.m; e += nthAll) {
+      if (e < nHin) {
+        const int4 hv = __ldg(d.hinge + e);
+        double q[12], v[12], o[12];
+        load3(d.x, hv.x, q); load3(d.x, hv.y, q + 3); load3(d.x, hv.z, q + 6); load3(d.x, hv.w, q + 9);
+        load3(A.p, hv.x, v); load3(A.p, hv.y, v + 3); load3(A.p, hv.z, v + 6); load3(A.p, hv.w, v + 9);
+        bend_hvp(q, v, d.hmeta[e * 3], d.hmeta[e * 3 + 1], d.hmeta[e * 3 + 2], A.kb, o);
+#pragma unroll
+        for (int c = 0; c < 12; c++) A.hin12[(size_t)e * 12 + c] = o[c];
+      } else if (e >= hinPad) {
+        const int t = e - hinPad;
+        const uint32_t t0 = __ldg(d.idx + t * 3), t1 = __ldg(d.idx + t * 3 + 1), t2 = __ldg(d.idx + t * 3 + 2);
+        double x0[3], x1[3], x2[3], w0[3], w1[3], w2[3];
+        load3(d.x, t0, x0); load3(d.x, t1, x1); load3(d.x, t2, x2);
+        load3(A.p, t0, w0); load3(A.p, t1, w1); load3(A.p, t2, w2);
+        const float4 iv = __ldg(d.inv + t);
+        double o[9];
+        mem_hvp64(x0, x1, x2, w0, w1, w2, iv.x, iv.y, iv.z, iv.w, d.area[t], d.mat, A.psd != 0, o);
+#pragma unroll
+        for (int c = 0; c < 9; c++) A.tri9[(size_t)t * 9 + c] = o[c];
+      }
+    }
+    if (d.hasContact) contact_hvp_coeffs(d, A.p, tid, nthAll);
+    barrier();
+    double pAp = 0;
+    for (int v = v0; v < d.n; v += nth) {
+      double s[3] = {0, 0, 0};
+      for (uint32_t q0 = d.memOff[v], q1 = d.memOff[v + 1]; q0 < q1; q0 += 4) {
+        double e[4][3];  // four incidences in flight, added in order
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+          const bool on = q0 + u < q1;
+          const uint32_t rec = on ? __ldg(d.memRec + q0 + u) : 0u;
+#pragma unroll
+          for (int c = 0; c < 3; c++) e[u][c] = on ? A.tri9[(size_t)(rec >> 2) * 9 + (rec & 3) * 3 + c] : 0.0;
+        }
+#pragma unroll
+        for (int u = 0; u < 4; u++) { s[0] += e[u][0]; s[1] += e[u][1]; s[2] += e[u][2]; }
+      }
+      if (A.kb > 0)
+        for (uint32_t q0 = d.hinOff[v], q1 = d.hinOff[v + 1]; q0 < q1; q0 += 4) {
+          double e[4][3];
+#pragma unroll
+          for (int u = 0; u < 4; u++) {
+            const bool on = q0 + u < q1;
+            const uint32_t rec = on ? __ldg(d.hinRec + q0 + u) : 0u;
+#pragma unroll
+            for (int c = 0; c < 3; c++) e[u][c] = on ? A.hin12[(size_t)(rec >> 2) * 12 + (rec & 3) * 3 + c] : 0.0;
+          }
+#pragma unroll
+          for (int u = 0; u < 4; u++) { s[0] += e[u][0]; s[1] += e[u][1]; s[2] += e[u][2]; }
+        }
+      double ch[3] = {0, 0, 0};
+      if (d.hasContact) contact_hvp_gather(d, v, ch);
+      const double M = d.mass[v];
+      const bool pin = d.pinned[v];
+#pragma unroll
+      for (int c = 0; c < 3; c++) {
+        const int i = v * 3 + c;
+        const double ap = pin ? 0.0 : M * A.p[i] * d.invH2 + s[c] + ch[c];
+        A.Ap[i] = ap;
+        pAp += A.p[i] * ap;
+      }
+    }
+    put(3, pAp);
+    barrier();
+    const double pApT = total(3);
     if (!(pApT > 0)) break;  // H not positive along p: stop with the current iterate
     const double alpha = rz / pApT;
     double rrn = 0;
-    for (int i = tid; i < n3; i += nth) {
+    for (int i = i0; i < n3; i += nth) {
       A.mu[i] += alpha * A.p[i];
       const double ri = A.r[i] - alpha * A.Ap[i];
       A.r[i] = ri;
       rrn += ri * ri;
     }
-    grid.sync();
-    const double rzn = adj_precond(d, A, tid, nth);
-    adj_put(d, 4, rrn, sm);
-    adj_put(d, 5, rzn, sm);
-    grid.sync();
-    residual = sqrt(adj_total(d, 4, bc));
-    const double rzNew = adj_total(d, 5, bc);
+    barrier();
+    const double rzn = precond();
+    put(4, rrn);
+    put(5, rzn);
+    barrier();
+    residual = sqrt(total(4));
+    const double rzNew = total(5);
     if (!(residual > absTol)) { k++; done = true; break; }
     const double beta = rzNew / rz;
     rz = rzNew;
-    for (int i = tid; i < n3; i += nth) A.p[i] = A.z[i] + beta * A.p[i];
-    grid.sync();
+    for (int i = i0; i < n3; i += nth) A.p[i] = __ldcg(A.z + i) + beta * A.p[i];
+    barrier();
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     A.out[0] = k;
@@ -386,21 +393,67 @@ int newton_exact_solve(const AdjArgs& a, int blocks, cudaStream_t s) {
 
 static inline int ablk(long n) { return (int)((n + kThreads - 1) / kThreads); }
 
-int adj_grid_blocks(const Dev& d) {
-  int dev = 0, sms = 0, per = 0;
+namespace {
+
+constexpr int kAdjCluster = 16;  // CTAs of the cluster launch, and the most blocks it reduces over
+
+struct AdjDevice {
+  int sms = 0, maxCtas = 0;
+  bool cluster = false;
+};
+void adj_cluster_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* attr) {
+  cfg.gridDim = dim3(kAdjCluster);
+  cfg.blockDim = dim3(kThreads);
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = kAdjCluster;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+}
+AdjDevice adj_device() {
+  static std::mutex mu;
+  static std::map<int, AdjDevice> known;  // per device
+  int dev = 0;
   cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_adj_pcg, kThreads, 0);
+  std::lock_guard<std::mutex> lock(mu);
+  const auto it = known.find(dev);
+  if (it != known.end()) return it->second;
+  AdjDevice a;
+  int per = 0, nc = 0;
+  cudaDeviceGetAttribute(&a.sms, cudaDevAttrMultiProcessorCount, dev);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_adj_pcg<false>, kThreads, 0);
+  a.maxCtas = std::max(1, per * a.sms);
+  cudaFuncSetAttribute(k_adj_pcg<true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  adj_cluster_config(cfg, attr);
+  a.cluster = cudaOccupancyMaxActiveClusters(&nc, k_adj_pcg<true>, &cfg) == cudaSuccess && nc >= 1;
+  cudaGetLastError();
+  known[dev] = a;
+  return a;
+}
+
+}  // namespace
+
+int adj_grid_blocks(const Dev& d) {
   const int want = ablk(std::max(std::max(d.n * 3, d.m), std::max(d.hg, d.D)));
-  int cap = per * sms;
-  if (cap < 1) cap = 1;
-  return std::max(1, std::min(want, std::min(cap, d.partStride)));
+  return std::max(1, std::min(want, std::min(adj_device().maxCtas, d.partStride)));
 }
 
 int adj_launch_pcg(const AdjArgs& a, int blocks, cudaStream_t s) {
+  const AdjDevice dv = adj_device();
   AdjArgs c = a;
-  void* args[] = {&c};
-  return (int)cudaLaunchCooperativeKernel((void*)k_adj_pcg, dim3(blocks), dim3(kThreads), args, 0, s);
+  if (blocks <= kAdjCluster && dv.cluster) {
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    adj_cluster_config(cfg, attr);
+    cfg.stream = s;
+    return (int)cudaLaunchKernelEx(&cfg, k_adj_pcg<true>, c, blocks);
+  }
+  void* args[] = {&c, &blocks};
+  const int ctas = std::min(dv.maxCtas, std::max(blocks, dv.sms));
+  return (int)cudaLaunchCooperativeKernel((void*)k_adj_pcg<false>, dim3(ctas), dim3(kThreads), args, 0, s);
 }
 
 void adj_theta(const Dev& d, const double* mu, double* terms, double* acc, cudaStream_t s) {

@@ -12,6 +12,7 @@ struct AdjArgs {
   double *r, *z, *p, *Ap;  // PCG work (3n each)
   double* tri9;          // 9m element HVP
   double* hin12;         // 12hg hinge HVP
+  double* domRz;         // D: r.z per Schwarz domain
   double kb;             // bending stiffness (0: no bending term)
   int psd;               // 1: positive part of the membrane stress in the geometric term (forward Newton matrix)
   int maxIters;
@@ -19,6 +20,7 @@ struct AdjArgs {
   double* out;           // [iterations, residual, |rhs|]
 };
 
+// Blocks of the PCG's reductions (the launch may use more CTAs).
 int adj_grid_blocks(const Dev& d);
 int adj_launch_pcg(const AdjArgs& a, int blocks, cudaStream_t s);
 // acc[0..4) -= mu . dg/d(C00, C11, G, k) at d.x; terms: 4 (m + hg) doubles.

@@ -508,7 +508,7 @@ class Solver {
       if (prof) CK(cudaEventRecord(pev0, stream));
       if (newtonMode == 1 && !exactMixed) {
         ensure_adj_buffers();
-        AdjArgs a{d, adjRhs.p, d.dx, adjR.p, adjZ.p, adjP.p, adjAp.p, adjTri.p, adjHin.p, d.kb, 1,
+        AdjArgs a{d, adjRhs.p, d.dx, adjR.p, adjZ.p, adjP.p, adjAp.p, adjTri.p, adjHin.p, adjDom.p, d.kb, 1,
                   opts.pcg_max_iters, newtonTol, adjOut.p};
         CK((cudaError_t)newton_exact_solve(a, adj_grid_blocks(d), stream));
         lc += 3;
@@ -684,7 +684,7 @@ class Solver {
     DBuf<double> xN, vN;     // state after the rollout
     bool valid = false;
   } ro;
-  DBuf<double> adjRhs, adjMu, adjR, adjZ, adjP, adjAp, adjTri, adjHin, adjTerms, adjLamX, adjLamV, adjAcc, adjOut;
+  DBuf<double> adjRhs, adjMu, adjR, adjZ, adjP, adjAp, adjTri, adjHin, adjTerms, adjLamX, adjLamV, adjAcc, adjOut, adjDom;
   AdjStats adjStats{};
   int adjMaxIters = 2000;
   double adjTol = 1e-10;
@@ -846,6 +846,7 @@ class Solver {
     if (adjHin.n < 12 * (size_t)std::max(mesh.hg, 1)) adjHin.alloc(12 * (size_t)std::max(mesh.hg, 1));
     if (adjTerms.n < 4 * (size_t)std::max(stride, 1)) adjTerms.alloc(4 * (size_t)std::max(stride, 1));
     if (adjAcc.n < 4) adjAcc.alloc(4);
+    if (adjDom.n < (size_t)std::max(mesh.D, 1)) adjDom.alloc(std::max(mesh.D, 1));
     if (adjOut.n < 3) adjOut.alloc(3);
   }
 
@@ -921,7 +922,7 @@ class Solver {
         launch_diag_init(d, beta, stream);
         if (d.precond >= 1) launch_schwarz_factor(d, stream);
         adj_rhs(d, adjLamX.p, adjLamV.p, damp, adjRhs.p, stream);
-        AdjArgs a{d, adjRhs.p, adjMu.p, adjR.p, adjZ.p, adjP.p, adjAp.p, adjTri.p, adjHin.p, d.kb, 0, maxIters, tol,
+        AdjArgs a{d, adjRhs.p, adjMu.p, adjR.p, adjZ.p, adjP.p, adjAp.p, adjTri.p, adjHin.p, adjDom.p, d.kb, 0, maxIters, tol,
                   adjOut.p};
         CK((cudaError_t)adj_launch_pcg(a, blocks, stream));
         adj_theta(d, adjMu.p, adjTerms.p, adjAcc.p, stream);
