@@ -1,18 +1,23 @@
 // Batched implicit step: one launch steps every sheet of a packed work list.
 //
-// Each sheet is an independent scene (no coupling), so a sheet maps to ONE
-// thread block that runs its whole step -- predictor and floor-CCD bisection,
+// Each sheet is an independent scene (no coupling), so a sheet maps to one
+// thread block, or one cluster of blocks (batch_class), that runs its whole
+// step -- predictor and floor-CCD bisection,
 // up to newtonIters Newton iterations (gradient, FP32 Jacobi-PCG with FP64 dot
 // products, descent safeguard, 2 mm trust region, CCD-gated Armijo search,
 // lagged-friction commit), velocity update and restitution -- with block
-// barriers only: no grid-wide synchronization and no host round trip. The
-// launch is persistent: blocks take sheets from a work list ordered largest
-// first. The algorithm per sheet is newton.ts:27-303 with the floor-contact
+// or cluster barriers only: no grid-wide synchronization and no host round trip.
+// The launch is persistent: groups take sheets from a work list ordered largest
+// first. A sheet's PCG is a chain of short passes over its vertices, bound by the
+// latency of its gathers; one SM per sheet left the batch waiting for its largest
+// sheet (96 sheets of 16 to 80 vertices a side: 84 ms a step, 44 with clusters). The algorithm per sheet is newton.ts:27-303 with the floor-contact
 // subset of contact-assembly.ts (kind 2: per-vertex barrier, lagged friction,
 // floor CCD, restitution); the bending gradient is the analytic gradient of
 // the hinge energy instead of its central difference (bending.ts:19-42).
-// Every reduction is a fixed-order block tree, so a sheet's result does not
-// depend on which block or how many blocks run it.
+// Every reduction is a fixed-order tree over the sheet's group, whose size depends
+// on the sheet alone, so a sheet's result does not depend on the rest of the batch.
+#include <cooperative_groups.h>
+
 #include "adjoint_math.cuh"
 #include "batch.cuh"
 #include "contact_math.cuh"
@@ -23,16 +28,121 @@ namespace cs {
 
 namespace {
 
+namespace cg = cooperative_groups;
+
 struct Range {
   int v0, v1, t0, t1, h0, h1;
 };
+
+constexpr int kParts = 12;  // up to three sums of four ranks
+
+// The CTAs that step one sheet: a thread-block cluster of `size` (1: one block).
+// `first` and `stride` spread a loop over all their threads.
+struct Group {
+  int size, rank, first, stride;
+  int virt;                 // 1, or the cluster size whose reductions a lone block reproduces
+  double* sm;               // block reduction scratch (32)
+  double (*part)[kParts][32];  // warp partials, two banks in turn
+  double (*bank)[3][8];     // the CTAs' partials, two banks in turn
+  int turn;
+};
+// Barrier over the group; what its threads wrote before is visible after.
+__device__ __forceinline__ void gsync(const Group& G) {
+  if (G.size > 1) cg::this_cluster().sync();
+  else __syncthreads();
+}
+// The CTAs' values of a block reduction: each is pushed into every peer's bank,
+// one cluster barrier, then all read their own bank. A bank is written again only
+// after the next call's barrier, which no CTA passes before it has read.
+template <class F>
+__device__ __forceinline__ double gcombine(Group& G, double v, const F& op) {
+  if (G.size == 1) return v;
+  cg::cluster_group cl = cg::this_cluster();
+  double* mine = G.bank[G.turn & 1][0];
+  if ((int)threadIdx.x < G.size) cl.map_shared_rank(mine, threadIdx.x)[G.rank] = v;
+  cl.sync();
+  double r = mine[0];
+  for (int q = 1; q < G.size; q++) r = op(r, mine[q]);
+  G.turn++;
+  return r;
+}
+// Sums over the group of what `share(first, stride, s)` leaves in s[0..K) for the
+// threads that start at `first` and step by `stride`, with one block barrier (and
+// one cluster barrier): warp trees, every warp (of a cluster: warp 0) adds the
+// warps' partials with the same tree, and the CTAs' totals are added in rank
+// order. A lone block that stands in for a cluster (virt > 1) evaluates each
+// rank's share and tree in turn, so it gets the cluster's bits. Also a barrier for
+// what the group's threads wrote before.
+template <int K, class F>
+__device__ __forceinline__ void gsums(double (&out)[K], Group& G, const F& share) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const int turn = G.turn & 1;
+  for (int r = 0; r < G.virt; r++) {
+    double v[K];
+#pragma unroll
+    for (int k = 0; k < K; k++) v[k] = 0;
+    share(G.first + r * (int)blockDim.x, G.stride * G.virt, v);
+#pragma unroll
+    for (int k = 0; k < K; k++) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_down_sync(0xffffffffu, v[k], o);
+      if (lane == 0) G.part[turn][r * K + k][warp] = v[k];
+    }
+  }
+  G.turn++;
+  __syncthreads();
+  if (G.size == 1) {
+#pragma unroll
+    for (int k = 0; k < K; k++) {
+      double w[4];
+#pragma unroll
+      for (int r = 0; r < 4; r++) w[r] = r < G.virt && lane < nw ? G.part[turn][r * K + k][lane] : 0.0;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int r = 0; r < 4; r++)
+          if (r < G.virt) w[r] += __shfl_down_sync(0xffffffffu, w[r], o);
+      double t = w[0];
+#pragma unroll
+      for (int r = 1; r < 4; r++)
+        if (r < G.virt) t += w[r];
+      out[k] = __shfl_sync(0xffffffffu, t, 0);
+    }
+    return;
+  }
+  cg::cluster_group cl = cg::this_cluster();
+  if (warp == 0) {
+#pragma unroll
+    for (int k = 0; k < K; k++) {
+      double w = lane < nw ? G.part[turn][k][lane] : 0.0;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) w += __shfl_down_sync(0xffffffffu, w, o);
+      w = __shfl_sync(0xffffffffu, w, 0);
+      if (lane < G.size) cl.map_shared_rank(G.bank[turn][k], lane)[G.rank] = w;
+    }
+  }
+  cl.sync();
+#pragma unroll
+  for (int k = 0; k < K; k++) {
+    double r = G.bank[turn][k][0];
+    for (int q = 1; q < G.size; q++) r += G.bank[turn][k][q];
+    out[k] = r;
+  }
+}
+
+__device__ __forceinline__ double gmax(double v, Group& G) {
+  return gcombine(G, block_max(v, G.sm), [](double a, double b) { return js_max(a, b); });
+}
+__device__ __forceinline__ double gmin(double v, Group& G) {
+  return gcombine(G, block_min(v, G.sm), [](double a, double b) { return fmin(a, b); });
+}
 
 __device__ __forceinline__ void ld3b(const double* x, int v, double o[3]) {
   o[0] = x[v * 3]; o[1] = x[v * 3 + 1]; o[2] = x[v * 3 + 2];
 }
 
-__device__ __forceinline__ void enforce_pins(const BatchDev& b, const Range& R, double* x) {
-  for (int v = R.v0 + threadIdx.x; v < R.v1; v += blockDim.x)
+__device__ __forceinline__ void enforce_pins(const BatchDev& b, const Range& R, const Group& G, double* x) {
+  for (int v = R.v0 + G.first; v < R.v1; v += G.stride)
     if (b.pinned[v])
       for (int k = 0; k < 3; k++) x[v * 3 + k] = b.pinPos[v * 3 + k];
 }
@@ -40,11 +150,11 @@ __device__ __forceinline__ void enforce_pins(const BatchDev& b, const Range& R, 
 // checkTrial restricted to the floor (contact-assembly.ts:489-553): the
 // smallest floor distance must exceed dMin and no vertex may cross the dMin
 // level during x0 -> xT.
-__device__ bool floor_trial_ok(const BatchDev& b, const Range& R, const double* xT, double* sm) {
+__device__ bool floor_trial_ok(const BatchDev& b, const Range& R, const double* xT, Group& G) {
   if (!b.hasFloor) return true;
   double mn = INFINITY;
   int bad = 0;
-  for (int v = R.v0 + threadIdx.x; v < R.v1; v += blockDim.x) {
+  for (int v = R.v0 + G.first; v < R.v1; v += G.stride) {
     const double yT = xT[v * 3 + 1] - b.floorY;
     if (yT < mn || yT != yT) mn = yT != yT ? -INFINITY : yT;
     const double y0 = b.x0[v * 3 + 1] - b.floorY;
@@ -54,51 +164,55 @@ __device__ bool floor_trial_ok(const BatchDev& b, const Range& R, const double* 
       if (toi < 1 - 1e-9) bad = 1;
     }
   }
-  const double m = block_min(mn, sm);
-  const double anyBad = block_max((double)bad, sm);
+  const double m = gmin(mn, G);
+  const double anyBad = gmax((double)bad, G);
   return !(m <= b.dMin) && anyBad == 0;
 }
 
-__device__ __forceinline__ void update_active(const BatchDev& b, const Range& R, const double* x) {
-  for (int v = R.v0 + threadIdx.x; v < R.v1; v += blockDim.x)
+__device__ __forceinline__ void update_active(const BatchDev& b, const Range& R, const Group& G, const double* x) {
+  for (int v = R.v0 + G.first; v < R.v1; v += G.stride)
     b.act[v] = b.hasFloor && (x[v * 3 + 1] - b.floorY < b.dHat) ? 1 : 0;
 }
 
 // totalEnergy (newton.ts:76-88): inertia + membrane + bending + barrier merit.
 __device__ double sheet_energy(const BatchDev& b, const Range& R, const double* x, const Mat<double>& mt, double kb,
-                               double* sm) {
-  double e = 0;
-  for (int v = R.v0 + threadIdx.x; v < R.v1; v += blockDim.x) {
-    const double M = b.mass[v];
-    for (int k = 0; k < 3; k++) {
-      const double d = x[v * 3 + k] - b.yHat[v * 3 + k];
-      e += 0.5 * M * d * d * b.invH2;
+                               Group& G) {
+  double out[1];
+  gsums<1>(out, G, [&](int first, int stride, double (&s)[1]) {
+    double e = 0;
+    for (int v = R.v0 + first; v < R.v1; v += stride) {
+      const double M = b.mass[v];
+      for (int k = 0; k < 3; k++) {
+        const double d = x[v * 3 + k] - b.yHat[v * 3 + k];
+        e += 0.5 * M * d * d * b.invH2;
+      }
+      if (b.act[v]) {
+        const double d = fmax(x[v * 3 + 1] - b.floorY, 1e-12);
+        if (d < b.dHat) e += b.kappa * barrier_value(d, b.dHat);
+      }
     }
-    if (b.act[v]) {
-      const double d = fmax(x[v * 3 + 1] - b.floorY, 1e-12);
-      if (d < b.dHat) e += b.kappa * barrier_value(d, b.dHat);
+    for (int t = R.t0 + first; t < R.t1; t += stride) {
+      double p0[3], p1[3], p2[3];
+      ld3b(x, b.idx[t * 3], p0); ld3b(x, b.idx[t * 3 + 1], p1); ld3b(x, b.idx[t * 3 + 2], p2);
+      const float4 iv = b.inv[t];
+      e += tri_energy<double>(p0, p1, p2, iv.x, iv.y, iv.z, iv.w, b.area[t], mt);
     }
-  }
-  for (int t = R.t0 + threadIdx.x; t < R.t1; t += blockDim.x) {
-    double p0[3], p1[3], p2[3];
-    ld3b(x, b.idx[t * 3], p0); ld3b(x, b.idx[t * 3 + 1], p1); ld3b(x, b.idx[t * 3 + 2], p2);
-    const float4 iv = b.inv[t];
-    e += tri_energy<double>(p0, p1, p2, iv.x, iv.y, iv.z, iv.w, b.area[t], mt);
-  }
-  if (kb > 0)
-    for (int hh = R.h0 + threadIdx.x; hh < R.h1; hh += blockDim.x) {
-      const int4 hv = b.hinge[hh];
-      double q[12], gdum[12];
-      ld3b(x, hv.x, q); ld3b(x, hv.y, q + 3); ld3b(x, hv.z, q + 6); ld3b(x, hv.w, q + 9);
-      e += bend_grad<double>(q, b.hmeta[hh * 3], b.hmeta[hh * 3 + 1], b.hmeta[hh * 3 + 2], kb, gdum);
-    }
-  return block_sum(e, sm);
+    if (kb > 0)
+      for (int hh = R.h0 + first; hh < R.h1; hh += stride) {
+        const int4 hv = b.hinge[hh];
+        double q[12], gdum[12];
+        ld3b(x, hv.x, q); ld3b(x, hv.y, q + 3); ld3b(x, hv.z, q + 6); ld3b(x, hv.w, q + 9);
+        e += bend_grad<double>(q, b.hmeta[hh * 3], b.hmeta[hh * 3 + 1], b.hmeta[hh * 3 + 2], kb, gdum);
+      }
+    s[0] = e;
+  });
+  return out[0];
 }
 
 // Newton gradient at b.x into b.g (filtered), the barrier curvature added to
 // the diagonal estimate; returns |g|.
-__device__ double sheet_gradient(const BatchDev& b, const Range& R, const Mat<double>& mt, double kb, double* sm) {
-  for (int t = R.t0 + threadIdx.x; t < R.t1; t += blockDim.x) {
+__device__ double sheet_gradient(const BatchDev& b, const Range& R, const Mat<double>& mt, double kb, Group& G) {
+  for (int t = R.t0 + G.first; t < R.t1; t += G.stride) {
     double p0[3], p1[3], p2[3];
     ld3b(b.x, b.idx[t * 3], p0); ld3b(b.x, b.idx[t * 3 + 1], p1); ld3b(b.x, b.idx[t * 3 + 2], p2);
     const float4 iv = b.inv[t];
@@ -107,57 +221,61 @@ __device__ double sheet_gradient(const BatchDev& b, const Range& R, const Mat<do
     for (int k = 0; k < 9; k++) b.elem[(size_t)t * 9 + k] = gg[k];
   }
   if (kb > 0)
-    for (int hh = R.h0 + threadIdx.x; hh < R.h1; hh += blockDim.x) {
+    for (int hh = R.h0 + G.first; hh < R.h1; hh += G.stride) {
       const int4 hv = b.hinge[hh];
       double q[12], gg[12];
       ld3b(b.x, hv.x, q); ld3b(b.x, hv.y, q + 3); ld3b(b.x, hv.z, q + 6); ld3b(b.x, hv.w, q + 9);
       bend_grad<double>(q, b.hmeta[hh * 3], b.hmeta[hh * 3 + 1], b.hmeta[hh * 3 + 2], kb, gg);
       for (int k = 0; k < 12; k++) b.helem[(size_t)hh * 12 + k] = gg[k];
     }
-  __syncthreads();
-  double gn = 0;
-  for (int v = R.v0 + threadIdx.x; v < R.v1; v += blockDim.x) {
-    double s[3] = {0, 0, 0};
-    for (uint32_t q = b.memOff[v]; q < b.memOff[v + 1]; q++) {
-      const uint32_t rec = b.memRec[q];
-      const double* e = b.elem + (size_t)(rec >> 2) * 9 + (rec & 3) * 3;
-      s[0] += e[0]; s[1] += e[1]; s[2] += e[2];
-    }
-    if (kb > 0)
-      for (uint32_t q = b.hinOff[v]; q < b.hinOff[v + 1]; q++) {
-        const uint32_t rec = b.hinRec[q];
-        const double* e = b.helem + (size_t)(rec >> 2) * 12 + (rec & 3) * 3;
+  gsync(G);
+  double out[1];
+  gsums<1>(out, G, [&](int first, int stride, double (&sum)[1]) {
+    double gn = 0;
+    for (int v = R.v0 + first; v < R.v1; v += stride) {
+      double s[3] = {0, 0, 0};
+      for (uint32_t q = b.memOff[v]; q < b.memOff[v + 1]; q++) {
+        const uint32_t rec = b.memRec[q];
+        const double* e = b.elem + (size_t)(rec >> 2) * 9 + (rec & 3) * 3;
         s[0] += e[0]; s[1] += e[1]; s[2] += e[2];
       }
-    if (b.act[v]) {
-      // barrier (addDistGrad) and lagged friction (addFrictionForce) of the floor contact
-      const double d = fmax(b.x[v * 3 + 1] - b.floorY, 1e-12);
-      if (d < b.dHat) {
-        s[1] += barrier_grad_scalar(d, b.dHat, b.kappa, 1);
-        const double lam = b.lagOk[v] ? b.lagLam[v] : barrier_normal_force(d, b.dHat, b.kappa, 1);
-        double u[3], fr[3];
-        for (int k = 0; k < 3; k++) u[k] = b.x[v * 3 + k] - b.x0[v * 3 + k];
-        coulomb_force(u, 0.0, 1.0, 0.0, lam, b.mu, b.eps, fr);
-        for (int k = 0; k < 3; k++) s[k] -= fr[k];
-        b.diag[v * 3 + 1] += barrier_curvature(d, b.dHat, b.kappa);  // addDiagEstimate (accumulates)
+      if (kb > 0)
+        for (uint32_t q = b.hinOff[v]; q < b.hinOff[v + 1]; q++) {
+          const uint32_t rec = b.hinRec[q];
+          const double* e = b.helem + (size_t)(rec >> 2) * 12 + (rec & 3) * 3;
+          s[0] += e[0]; s[1] += e[1]; s[2] += e[2];
+        }
+      if (b.act[v]) {
+        // barrier (addDistGrad) and lagged friction (addFrictionForce) of the floor contact
+        const double d = fmax(b.x[v * 3 + 1] - b.floorY, 1e-12);
+        if (d < b.dHat) {
+          s[1] += barrier_grad_scalar(d, b.dHat, b.kappa, 1);
+          const double lam = b.lagOk[v] ? b.lagLam[v] : barrier_normal_force(d, b.dHat, b.kappa, 1);
+          double u[3], fr[3];
+          for (int k = 0; k < 3; k++) u[k] = b.x[v * 3 + k] - b.x0[v * 3 + k];
+          coulomb_force(u, 0.0, 1.0, 0.0, lam, b.mu, b.eps, fr);
+          for (int k = 0; k < 3; k++) s[k] -= fr[k];
+          b.diag[v * 3 + 1] += barrier_curvature(d, b.dHat, b.kappa);  // addDiagEstimate (accumulates)
+        }
+      }
+      const double M = b.mass[v];
+      const bool pin = b.pinned[v];
+      for (int k = 0; k < 3; k++) {
+        const int i = v * 3 + k;
+        double gi = M * (b.x[i] - b.yHat[i]) * b.invH2 + s[k];
+        if (pin) gi = 0;
+        b.g[i] = gi;
+        gn += gi * gi;
       }
     }
-    const double M = b.mass[v];
-    const bool pin = b.pinned[v];
-    for (int k = 0; k < 3; k++) {
-      const int i = v * 3 + k;
-      double gi = M * (b.x[i] - b.yHat[i]) * b.invH2 + s[k];
-      if (pin) gi = 0;
-      b.g[i] = gi;
-      gn += gi * gi;
-    }
-  }
-  return sqrt(block_sum(gn, sm));
+    sum[0] = gn;
+  });
+  return sqrt(out[0]);
 }
 
 // FP32 state of every triangle for the matrix-free HVP (F, S, Dm^-1, s).
-__device__ void sheet_tristate(const BatchDev& b, const Range& R, const Mat<double>& m) {
-  for (int t = R.t0 + threadIdx.x; t < R.t1; t += blockDim.x) {
+__device__ void sheet_tristate(const BatchDev& b, const Range& R, const Group& G, const Mat<double>& m) {
+  for (int t = R.t0 + G.first; t < R.t1; t += G.stride) {
     double x0[3], x1[3], x2[3];
     ld3b(b.x, b.idx[t * 3], x0); ld3b(b.x, b.idx[t * 3 + 1], x1); ld3b(b.x, b.idx[t * 3 + 2], x2);
     const float4 iv = b.inv[t];
@@ -185,132 +303,152 @@ __device__ void sheet_tristate(const BatchDev& b, const Range& R, const Mat<doub
 // vertex adds the corner share of its incident triangles' HVP directly
 // (recomputed per corner from the stored FP32 state), so no per-triangle
 // result is written and read back and no barrier splits the product.
-__device__ double sheet_hvp(const BatchDev& b, const Range& R, float C00, float C11, float C01, float G,
-                            double* sm) {
-  double pAp = 0;
+__device__ double sheet_hvp(const BatchDev& b, const Range& R, float C00, float C11, float C01, float Gs,
+                            Group& G) {
   const float invH2 = (float)b.invH2;
-  for (int v = R.v0 + threadIdx.x; v < R.v1; v += blockDim.x) {
-    float sp[3] = {0.f, 0.f, 0.f};
-    for (uint32_t q = b.memOff[v]; q < b.memOff[v + 1]; q++) {
-      const uint32_t rec = __ldg(b.memRec + q);
-      const uint32_t t = rec >> 2;
-      const int i0 = (int)__ldg(b.idx + t * 3), i1 = (int)__ldg(b.idx + t * 3 + 1), i2 = (int)__ldg(b.idx + t * 3 + 2);
-      const float3 p0 = make_float3(b.p[i0 * 3], b.p[i0 * 3 + 1], b.p[i0 * 3 + 2]);
-      const float3 p1 = make_float3(b.p[i1 * 3], b.p[i1 * 3 + 1], b.p[i1 * 3 + 2]);
-      const float3 p2 = make_float3(b.p[i2 * 3], b.p[i2 * 3 + 1], b.p[i2 * 3 + 2]);
-      float o[3];
-      tri_hvp_corner(b.tris + (size_t)t * 16, p0, p1, p2, (int)(rec & 3), C00, C11, C01, G, o);
-      sp[0] += o[0]; sp[1] += o[1]; sp[2] += o[2];
+  double out[1];
+  gsums<1>(out, G, [&](int first, int stride, double (&s)[1]) {
+    double pAp = 0;
+    for (int v = R.v0 + first; v < R.v1; v += stride) {
+      float sp[3] = {0.f, 0.f, 0.f};
+      for (uint32_t q = b.memOff[v]; q < b.memOff[v + 1]; q++) {
+        const uint32_t rec = __ldg(b.memRec + q);
+        const uint32_t t = rec >> 2;
+        const int i0 = (int)__ldg(b.idx + t * 3), i1 = (int)__ldg(b.idx + t * 3 + 1);
+        const int i2 = (int)__ldg(b.idx + t * 3 + 2);
+        const float3 p0 = make_float3(b.p[i0 * 3], b.p[i0 * 3 + 1], b.p[i0 * 3 + 2]);
+        const float3 p1 = make_float3(b.p[i1 * 3], b.p[i1 * 3 + 1], b.p[i1 * 3 + 2]);
+        const float3 p2 = make_float3(b.p[i2 * 3], b.p[i2 * 3 + 1], b.p[i2 * 3 + 2]);
+        float o[3];
+        // plain loads: another CTA of the group may have written the record
+        tri_hvp_corner<false>(b.tris + (size_t)t * 16, p0, p1, p2, (int)(rec & 3), C00, C11, C01, Gs, o);
+        sp[0] += o[0]; sp[1] += o[1]; sp[2] += o[2];
+      }
+      float cy = 0.f;
+      if (b.act[v]) {
+        const double d = fmax(b.x[v * 3 + 1] - b.floorY, 1e-12);
+        if (d < b.dHat) cy = (float)(barrier_curvature(d, b.dHat, b.kappa) * (double)b.p[v * 3 + 1]);
+      }
+      const float M = b.mass[v];
+      const bool pin = b.pinned[v];
+      for (int q = 0; q < 3; q++) {
+        const int i = v * 3 + q;
+        float ap = M * b.p[i] * invH2 + sp[q] + (q == 1 ? cy : 0.f);
+        if (pin) ap = 0.f;
+        b.Ap[i] = ap;
+        pAp += (double)b.p[i] * ap;
+      }
     }
-    float cy = 0.f;
-    if (b.act[v]) {
-      const double d = fmax(b.x[v * 3 + 1] - b.floorY, 1e-12);
-      if (d < b.dHat) cy = (float)(barrier_curvature(d, b.dHat, b.kappa) * (double)b.p[v * 3 + 1]);
-    }
-    const float M = b.mass[v];
-    const bool pin = b.pinned[v];
-    for (int q = 0; q < 3; q++) {
-      const int i = v * 3 + q;
-      float ap = M * b.p[i] * invH2 + sp[q] + (q == 1 ? cy : 0.f);
-      if (pin) ap = 0.f;
-      b.Ap[i] = ap;
-      pAp += (double)b.p[i] * ap;
-    }
-  }
-  return block_sum(pAp, sm);
+    s[0] = pAp;
+  });
+  return out[0];
 }
 
 // pcg.ts:11-95 (Jacobi, tolerance 1e-3) and the newton.ts:152-179 epilogue;
 // the direction lands in b.dx. Returns the PCG iteration count.
-__device__ int sheet_pcg(const BatchDev& b, const Range& R, float C00, float C11, float C01, float G, double* sm,
+__device__ int sheet_pcg(const BatchDev& b, const Range& R, float C00, float C11, float C01, float Gs, Group& G,
                          double& gtdxOut) {
-  double bb = 0, rr = 0, rz = 0;
-  for (int i = 3 * R.v0 + threadIdx.x; i < 3 * R.v1; i += blockDim.x) {
-    const double bi = -b.g[i];
-    bb += bi * bi;
-    const bool pin = b.pinned[i / 3];
-    const float ri = pin ? 0.f : (float)bi;
-    b.r[i] = ri;
-    b.xs[i] = 0.f;
-    rr += (double)ri * ri;
-    const float di = pin ? 0.f : b.diag[i] > 1e-12 ? (float)(1.0 / b.diag[i]) : 1.f;
-    b.dinv[i] = di;
-    const float zi = ri * di;
-    b.z[i] = zi;
-    b.p[i] = zi;
-    rz += (double)ri * zi;
-  }
-  const double bNorm = sqrt(block_sum(bb, sm));
-  double residual = sqrt(block_sum(rr, sm));
-  rz = block_sum(rz, sm);
+  double s3[3];
+  gsums<3>(s3, G, [&](int first, int stride, double (&s)[3]) {
+    double bb = 0, rr = 0, rz = 0;
+    for (int i = 3 * R.v0 + first; i < 3 * R.v1; i += stride) {
+      const double bi = -b.g[i];
+      bb += bi * bi;
+      const bool pin = b.pinned[i / 3];
+      const float ri = pin ? 0.f : (float)bi;
+      b.r[i] = ri;
+      b.xs[i] = 0.f;
+      rr += (double)ri * ri;
+      const float di = pin ? 0.f : b.diag[i] > 1e-12 ? (float)(1.0 / b.diag[i]) : 1.f;
+      b.dinv[i] = di;
+      const float zi = ri * di;
+      b.z[i] = zi;
+      b.p[i] = zi;
+      rz += (double)ri * zi;
+    }
+    s[0] = bb; s[1] = rr; s[2] = rz;
+  });
+  const double bNorm = sqrt(s3[0]);
+  double residual = sqrt(s3[1]), rz = s3[2];
   const double absTol = fmax(1e-3 * fmax(bNorm, 1e-12), 1e-12);
   int iters = 0;
   bool done = residual < absTol;
   int k = 0;
   for (; !done && k < b.pcgMaxIters; k++) {
-    const double pAp = sheet_hvp(b, R, C00, C11, C01, G, sm);
+    const double pAp = sheet_hvp(b, R, C00, C11, C01, Gs, G);
     if (!(pAp > 1e-30)) { iters = k; done = true; break; }
     const float alpha = (float)(rz / pAp);
-    double rrn = 0, rzn = 0;
-    for (int i = 3 * R.v0 + threadIdx.x; i < 3 * R.v1; i += blockDim.x) {
-      const bool pin = b.pinned[i / 3];
-      float xi = b.xs[i] + alpha * b.p[i];
-      float ri = b.r[i] - alpha * b.Ap[i];
-      if (pin) { xi = 0.f; ri = 0.f; }
-      b.xs[i] = xi;
-      b.r[i] = ri;
-      rrn += (double)ri * ri;
-      const float zi = ri * b.dinv[i];
-      b.z[i] = zi;
-      rzn += (double)ri * zi;
-    }
-    residual = sqrt(block_sum(rrn, sm));
-    rzn = block_sum(rzn, sm);
+    double s2[2];
+    gsums<2>(s2, G, [&](int first, int stride, double (&s)[2]) {
+      double rrn = 0, rzn = 0;
+      for (int i = 3 * R.v0 + first; i < 3 * R.v1; i += stride) {
+        const bool pin = b.pinned[i / 3];
+        float xi = b.xs[i] + alpha * b.p[i];
+        float ri = b.r[i] - alpha * b.Ap[i];
+        if (pin) { xi = 0.f; ri = 0.f; }
+        b.xs[i] = xi;
+        b.r[i] = ri;
+        rrn += (double)ri * ri;
+        const float zi = ri * b.dinv[i];
+        b.z[i] = zi;
+        rzn += (double)ri * zi;
+      }
+      s[0] = rrn; s[1] = rzn;
+    });
+    residual = sqrt(s2[0]);
+    const double rzn = s2[1];
     if (residual < absTol) { iters = k + 1; done = true; break; }
     const float beta = (float)(rzn / rz);
     rz = rzn;
-    for (int i = 3 * R.v0 + threadIdx.x; i < 3 * R.v1; i += blockDim.x) b.p[i] = b.z[i] + beta * b.p[i];
-    __syncthreads();
+    for (int i = 3 * R.v0 + G.first; i < 3 * R.v1; i += G.stride) b.p[i] = b.z[i] + beta * b.p[i];
+    gsync(G);
   }
   if (!done) iters = b.pcgMaxIters;
-  double gt = 0;
-  for (int i = 3 * R.v0 + threadIdx.x; i < 3 * R.v1; i += blockDim.x) {
-    const double di = b.xs[i];
-    b.dx[i] = di;
-    gt += b.g[i] * di;
-  }
-  double gtdx = block_sum(gt, sm);
-  if (!isfinite(gtdx) || gtdx >= 0) {
-    gt = 0;
-    for (int i = 3 * R.v0 + threadIdx.x; i < 3 * R.v1; i += blockDim.x) {
-      const double di = -b.g[i] / b.diag[i];
+  double s1[1];
+  gsums<1>(s1, G, [&](int first, int stride, double (&s)[1]) {
+    double gt = 0;
+    for (int i = 3 * R.v0 + first; i < 3 * R.v1; i += stride) {
+      const double di = b.xs[i];
       b.dx[i] = di;
       gt += b.g[i] * di;
     }
-    gtdx = block_sum(gt, sm);
+    s[0] = gt;
+  });
+  double gtdx = s1[0];
+  if (!isfinite(gtdx) || gtdx >= 0) {
+    gsums<1>(s1, G, [&](int first, int stride, double (&s)[1]) {
+      double gt = 0;
+      for (int i = 3 * R.v0 + first; i < 3 * R.v1; i += stride) {
+        const double di = -b.g[i] / b.diag[i];
+        b.dx[i] = di;
+        gt += b.g[i] * di;
+      }
+      s[0] = gt;
+    });
+    gtdx = s1[0];
   }
   double mx = 0;
-  for (int i = 3 * R.v0 + threadIdx.x; i < 3 * R.v1; i += blockDim.x) mx = fmax(mx, fabs(b.dx[i]));
-  const double maxDx = block_max(mx, sm);
+  for (int i = 3 * R.v0 + G.first; i < 3 * R.v1; i += G.stride) mx = fmax(mx, fabs(b.dx[i]));
+  const double maxDx = gmax(mx, G);
   if (maxDx > 0.002) {
     const double sc = 0.002 / maxDx;
-    for (int i = 3 * R.v0 + threadIdx.x; i < 3 * R.v1; i += blockDim.x) b.dx[i] *= sc;
+    for (int i = 3 * R.v0 + G.first; i < 3 * R.v1; i += G.stride) b.dx[i] *= sc;
     gtdx *= sc;
-    __syncthreads();
+    gsync(G);
   }
   gtdxOut = gtdx;
   return iters;
 }
 
-__device__ void step_sheet(const BatchDev& b, int s, double* sm) {
+__device__ void step_sheet(const BatchDev& b, int s, Group& G) {
   const Range R{b.vStart[s], b.vStart[s + 1], b.tStart[s], b.tStart[s + 1], b.hStart[s], b.hStart[s + 1]};
   const double* mr = b.mat + (size_t)s * BM_N;
   const Mat<double> mt{mr[BM_C00], mr[BM_C11], mr[BM_C01], mr[BM_G], mr[BM_THICK]};
   const double kb = mr[BM_KB], damp = mr[BM_DAMP], beta = mr[BM_BETA];
-  const float C00 = (float)mr[BM_C00], C11 = (float)mr[BM_C11], C01 = (float)mr[BM_C01], G = (float)mr[BM_G];
+  const float C00 = (float)mr[BM_C00], C11 = (float)mr[BM_C11], C01 = (float)mr[BM_C01], Gs = (float)mr[BM_G];
   const double h = b.h;
   // predictor y_hat = x + h v + h^2 g, initial guess y_hat with pins (newton.ts:40-51)
-  for (int v = R.v0 + threadIdx.x; v < R.v1; v += blockDim.x)
+  for (int v = R.v0 + G.first; v < R.v1; v += G.stride)
     for (int k = 0; k < 3; k++) {
       const int i = v * 3 + k;
       const double xv = b.x[i];
@@ -319,72 +457,72 @@ __device__ void step_sheet(const BatchDev& b, int s, double* sm) {
       b.yHat[i] = y;
       b.x[i] = y;
     }
-  __syncthreads();
-  enforce_pins(b, R, b.x);
-  __syncthreads();
+  gsync(G);
+  enforce_pins(b, R, G, b.x);
+  gsync(G);
   int rejected = 0;
-  if (b.hasFloor && !floor_trial_ok(b, R, b.x, sm)) {
+  if (b.hasFloor && !floor_trial_ok(b, R, b.x, G)) {
     // bisect back along x0 -> y_hat to the largest CCD-valid fraction (newton.ts:53-72)
     double lo = 0, hi = 1;
     for (int it = 0; it < 8; it++) {
       const double mid = 0.5 * (lo + hi);
-      for (int i = 3 * R.v0 + threadIdx.x; i < 3 * R.v1; i += blockDim.x) b.xt[i] = b.x0[i] + mid * (b.x[i] - b.x0[i]);
-      __syncthreads();
-      enforce_pins(b, R, b.xt);
-      __syncthreads();
-      if (floor_trial_ok(b, R, b.xt, sm)) lo = mid;
+      for (int i = 3 * R.v0 + G.first; i < 3 * R.v1; i += G.stride) b.xt[i] = b.x0[i] + mid * (b.x[i] - b.x0[i]);
+      gsync(G);
+      enforce_pins(b, R, G, b.xt);
+      gsync(G);
+      if (floor_trial_ok(b, R, b.xt, G)) lo = mid;
       else hi = mid;
       if (hi - lo < 1e-4) break;
     }
-    for (int i = 3 * R.v0 + threadIdx.x; i < 3 * R.v1; i += blockDim.x) b.x[i] = b.x0[i] + lo * (b.x[i] - b.x0[i]);
-    __syncthreads();
-    enforce_pins(b, R, b.x);
-    __syncthreads();
+    for (int i = 3 * R.v0 + G.first; i < 3 * R.v1; i += G.stride) b.x[i] = b.x0[i] + lo * (b.x[i] - b.x0[i]);
+    gsync(G);
+    enforce_pins(b, R, G, b.x);
+    gsync(G);
   }
-  update_active(b, R, b.x);
-  __syncthreads();
-  double energy = sheet_energy(b, R, b.x, mt, kb, sm);
-  for (int v = R.v0 + threadIdx.x; v < R.v1; v += blockDim.x) {
+  update_active(b, R, G, b.x);
+  gsync(G);
+  double energy = sheet_energy(b, R, b.x, mt, kb, G);
+  for (int v = R.v0 + G.first; v < R.v1; v += G.stride) {
     const double d0 = b.mass[v] * b.invH2 + beta;
     b.diag[v * 3] = d0; b.diag[v * 3 + 1] = d0; b.diag[v * 3 + 2] = d0;
   }
-  __syncthreads();
+  gsync(G);
   double gradNorm = INFINITY;
   int used = 0, pcgTotal = 0, trials = 0, converged = 0;
   for (int ni = 0; ni < b.newtonIters; ni++) {
     used = ni + 1;
-    update_active(b, R, b.x);
-    __syncthreads();
-    gradNorm = sheet_gradient(b, R, mt, kb, sm);
+    update_active(b, R, G, b.x);
+    gsync(G);
+    gradNorm = sheet_gradient(b, R, mt, kb, G);
     if (!isfinite(gradNorm)) { converged = -1; break; }
     if (gradNorm < b.gradTol) { converged = 1; break; }
-    sheet_tristate(b, R, mt);
-    __syncthreads();
+    sheet_tristate(b, R, G, mt);
+    gsync(G);
     double gtdx;
-    pcgTotal += sheet_pcg(b, R, C00, C11, C01, G, sm, gtdx);
+    pcgTotal += sheet_pcg(b, R, C00, C11, C01, Gs, G, gtdx);
     double alpha = 1;
     bool accepted = false;
     for (int li = 0; li < b.lsIters; li++) {
       trials++;
-      for (int i = 3 * R.v0 + threadIdx.x; i < 3 * R.v1; i += blockDim.x) b.xt[i] = b.x[i] + alpha * b.dx[i];
-      __syncthreads();
-      enforce_pins(b, R, b.xt);
-      __syncthreads();
-      if (!floor_trial_ok(b, R, b.xt, sm)) { rejected++; alpha *= 0.5; continue; }
-      const double eNew = sheet_energy(b, R, b.xt, mt, kb, sm);
+      for (int i = 3 * R.v0 + G.first; i < 3 * R.v1; i += G.stride) b.xt[i] = b.x[i] + alpha * b.dx[i];
+      gsync(G);
+      enforce_pins(b, R, G, b.xt);
+      gsync(G);
+      if (!floor_trial_ok(b, R, b.xt, G)) { rejected++; alpha *= 0.5; continue; }
+      const double eNew = sheet_energy(b, R, b.xt, mt, kb, G);
       if (!isfinite(eNew)) { rejected++; alpha *= 0.5; continue; }
       if (eNew <= energy + 1e-4 * alpha * gtdx) {
-        for (int i = 3 * R.v0 + threadIdx.x; i < 3 * R.v1; i += blockDim.x) b.x[i] = b.xt[i];
+        for (int i = 3 * R.v0 + G.first; i < 3 * R.v1; i += G.stride) b.x[i] = b.xt[i];
         energy = eNew;
         accepted = true;
-        __syncthreads();
+        gsync(G);
         // commit: lagged normal force of every active floor contact (contact-assembly.ts:475-485)
-        for (int v = R.v0 + threadIdx.x; v < R.v1; v += blockDim.x)
+        for (int v = R.v0 + G.first; v < R.v1; v += G.stride)
           if (b.act[v]) {
             const double d = fmax(b.x[v * 3 + 1] - b.floorY, 1e-12);
             if (d < b.dHat) { b.lagLam[v] = barrier_normal_force(d, b.dHat, b.kappa, 1); b.lagOk[v] = 1; }
           }
-        __syncthreads();
+        gsync(G);
         break;
       }
       rejected++;
@@ -393,19 +531,20 @@ __device__ void step_sheet(const BatchDev& b, int s, double* sm) {
     if (!accepted || alpha < 1e-6) break;
   }
   // velocity update, restitution-0 on floor contacts (newton.ts:222-245)
-  for (int i = 3 * R.v0 + threadIdx.x; i < 3 * R.v1; i += blockDim.x) b.v[i] = ((b.x[i] - b.x0[i]) / h) * damp;
-  __syncthreads();
-  update_active(b, R, b.x);
-  __syncthreads();
+  for (int i = 3 * R.v0 + G.first; i < 3 * R.v1; i += G.stride) b.v[i] = ((b.x[i] - b.x0[i]) / h) * damp;
+  gsync(G);
+  update_active(b, R, G, b.x);
+  gsync(G);
   int nfloor = 0;
-  for (int v = R.v0 + threadIdx.x; v < R.v1; v += blockDim.x)
+  for (int v = R.v0 + G.first; v < R.v1; v += G.stride)
     if (b.act[v]) {
       nfloor++;
       if (b.v[v * 3 + 1] < 0) b.v[v * 3 + 1] = 0;
     }
-  enforce_pins(b, R, b.x);
-  const double nf = block_sum((double)nfloor, sm);
-  if (threadIdx.x == 0) {
+  enforce_pins(b, R, G, b.x);
+  double nf[1];
+  gsums<1>(nf, G, [&](int, int, double (&t)[1]) { t[0] += nfloor; nfloor = 0; });
+  if (G.rank == 0 && threadIdx.x == 0) {
     double* o = b.out + (size_t)s * BO_N;
     o[BO_NEWTON] = used;
     o[BO_PCG] = pcgTotal;
@@ -413,27 +552,51 @@ __device__ void step_sheet(const BatchDev& b, int s, double* sm) {
     o[BO_ENERGY] = energy;
     o[BO_CONVERGED] = converged;
     o[BO_TRIALS] = trials;
-    o[BO_FLOOR] = nf;
+    o[BO_FLOOR] = nf[0];
     o[BO_REJECTED] = rejected;
   }
-  __syncthreads();
+  gsync(G);
 }
 
 template <int T>
-__global__ void __launch_bounds__(T, 1) k_batch_step(BatchDev b) {
+__global__ void __launch_bounds__(T, 1) k_batch_step(BatchDev b, const int* order, int count, unsigned int* work,
+                                                     int size, int virt) {
   __shared__ double sm[32];
+  __shared__ double part[2][kParts][32];
+  __shared__ double bank[2][3][8];
   __shared__ int sheetSh;
-  for (int guard = 0; guard <= b.S; guard++) {
-    if (threadIdx.x == 0) {
-      const unsigned k = atomicAdd(b.work, 1u);
-      sheetSh = k < (unsigned)b.S ? b.order[k] : -1;
+  const int rank = size > 1 ? (int)cg::this_cluster().block_rank() : 0;
+  Group G{size, rank, rank * T + (int)threadIdx.x, size * T, virt, sm, part, bank, 0};
+  for (int guard = 0; guard <= count; guard++) {
+    if (rank == 0 && threadIdx.x == 0) {
+      const unsigned k = atomicAdd(work, 1u);
+      const int sheet = k < (unsigned)count ? order[k] : -1;
+      sheetSh = sheet;
+      for (int q = 1; q < size; q++) *cg::this_cluster().map_shared_rank(&sheetSh, q) = sheet;
     }
-    __syncthreads();
+    gsync(G);
     const int sheet = sheetSh;
-    __syncthreads();
+    gsync(G);
     if (sheet < 0) return;
-    step_sheet(b, sheet, sm);
+    step_sheet(b, sheet, G);
   }
+}
+
+template <int T>
+int launch_t(const BatchDev& b, const int* order, int count, unsigned int* work, int size, int virt, int ctas,
+             cudaStream_t s) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(ctas);
+  cfg.blockDim = dim3(T);
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = size;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = size > 1 ? 1 : 0;
+  return (int)cudaLaunchKernelEx(&cfg, k_batch_step<T>, b, order, count, work, size, virt);
 }
 
 }  // namespace
@@ -450,12 +613,11 @@ int batch_max_ctas(int threads) {
   return per * sms;
 }
 
-int batch_launch_step(const BatchDev& b, int threads, int ctas, cudaStream_t s) {
-  cudaMemsetAsync(b.work, 0, sizeof(unsigned int), s);
-  if (threads == 128) k_batch_step<128><<<ctas, 128, 0, s>>>(b);
-  else if (threads == 256) k_batch_step<256><<<ctas, 256, 0, s>>>(b);
-  else k_batch_step<512><<<ctas, 512, 0, s>>>(b);
-  return (int)cudaGetLastError();
+int batch_launch_step(const BatchDev& b, const int* order, int count, unsigned int* work, int size, int virt,
+                      int threads, int ctas, cudaStream_t s) {
+  if (threads == 128) return launch_t<128>(b, order, count, work, size, virt, ctas, s);
+  if (threads == 256) return launch_t<256>(b, order, count, work, size, virt, ctas, s);
+  return launch_t<512>(b, order, count, work, size, virt, ctas, s);
 }
 
 }  // namespace cs

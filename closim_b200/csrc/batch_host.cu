@@ -74,6 +74,12 @@ struct Batch {
   std::vector<double> matRows;  // S x BM_N, host copy
   int threads = 512;
   int ctas = 0;
+  // The size classes of the sheets (batch_class): their runs in `order`. Classes
+  // are independent launches; all but the first go to side streams between two
+  // events, so small sheets fill the SMs that the clusters leave free.
+  int classStart[kBatchClasses + 1] = {0, 0, 0, 0};
+  cudaStream_t side[kBatchClasses] = {};
+  cudaEvent_t fork = nullptr, join[kBatchClasses] = {};
   bool ready = false;
   cudaGraphExec_t graph = nullptr;
   int graphSteps = 0;
@@ -83,6 +89,11 @@ struct Batch {
 
   ~Batch() {
     if (graph) cudaGraphExecDestroy(graph);
+    for (int c = 0; c < kBatchClasses; c++) {
+      if (join[c]) cudaEventDestroy(join[c]);
+      if (side[c]) cudaStreamDestroy(side[c]);
+    }
+    if (fork) cudaEventDestroy(fork);
     if (stream) cudaStreamDestroy(stream);
   }
 
@@ -154,10 +165,21 @@ struct Batch {
     if (!stream) {
       BK(cudaSetDevice(device));
       BK(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
+      BK(cudaEventCreateWithFlags(&fork, cudaEventDisableTiming));
+      for (int c = 0; c < kBatchClasses; c++) {
+        BK(cudaStreamCreateWithFlags(&side[c], cudaStreamNonBlocking));
+        BK(cudaEventCreateWithFlags(&join[c], cudaEventDisableTiming));
+      }
     }
     std::vector<int> ord(S);
     std::iota(ord.begin(), ord.end(), 0);
-    std::stable_sort(ord.begin(), ord.end(), [&](int a, int b) { return ts[a + 1] - ts[a] > ts[b + 1] - ts[b]; });
+    auto classOf = [&](int a) { return batch_class(vs[a + 1] - vs[a]); };
+    std::stable_sort(ord.begin(), ord.end(), [&](int a, int b) {
+      if (classOf(a) != classOf(b)) return classOf(a) < classOf(b);
+      return ts[a + 1] - ts[a] > ts[b + 1] - ts[b];
+    });
+    for (int c = 0; c <= kBatchClasses; c++)
+      classStart[c] = (int)std::count_if(ord.begin(), ord.end(), [&](int a) { return classOf(a) < c; });
     cudaStream_t st = stream;
     vStart.up(vs.data(), vs.size(), st); tStart.up(ts.data(), ts.size(), st); hStart.up(hs.data(), hs.size(), st);
     order.up(ord.data(), ord.size(), st);
@@ -191,7 +213,7 @@ struct Batch {
     lagLam.alloc(N);
     out.alloc((size_t)S * BO_N);
     BK(cudaMemsetAsync(out.p, 0, (size_t)S * BO_N * 8, st));
-    work.alloc(1);
+    work.alloc(kBatchClasses);
     if (grav) for (int k = 0; k < 3; k++) gravity[k] = grav[k];
     BK(cudaStreamSynchronize(st));
     ctas = batch_max_ctas(threads);
@@ -200,7 +222,7 @@ struct Batch {
 
   void bind(double h) {
     d = BatchDev{};
-    d.S = S; d.vStart = vStart.p; d.tStart = tStart.p; d.hStart = hStart.p; d.order = order.p;
+    d.S = S; d.vStart = vStart.p; d.tStart = tStart.p; d.hStart = hStart.p;
     d.idx = idx.p; d.inv = inv.p; d.area = area.p; d.mass = mass.p; d.hinge = hinge.p; d.hmeta = hmeta.p;
     d.memOff = memOff.p; d.memRec = memRec.p; d.hinOff = hinOff.p; d.hinRec = hinRec.p;
     d.pinned = pinned.p; d.pinPos = pinPos.p; d.mat = mat.p;
@@ -214,13 +236,39 @@ struct Batch {
     for (int k = 0; k < 3; k++) d.gravity[k] = gravity[k];
     d.newtonIters = opts.newton_iters; d.pcgMaxIters = opts.pcg_max_iters; d.lsIters = opts.ls_iters;
     d.gradTol = opts.grad_tol;
-    d.out = out.p; d.work = work.p;
+    d.out = out.p;
   }
 
-  // One step = reset of the work list + one persistent launch.
+  // One step = reset of the work lists + one persistent launch per size class.
   void enqueue_step(double h) {
     bind(h);
-    BK((cudaError_t)batch_launch_step(d, threads, ctas, stream));
+    BK(cudaMemsetAsync(work.p, 0, kBatchClasses * sizeof(unsigned int), stream));
+    bool forked = false, used = false;
+    long wanted = 0;
+    for (int c = 0; c < kBatchClasses; c++) wanted += (long)(classStart[c + 1] - classStart[c]) * kBatchSize[c];
+    const bool lone = wanted > (long)kBatchFill * ctas;
+    for (int c = 0; c < kBatchClasses; c++) {
+      const int count = classStart[c + 1] - classStart[c];
+      const int size = lone ? 1 : kBatchSize[c], virt = lone ? kBatchSize[c] : 1;
+      if (count == 0) continue;
+      cudaStream_t st = stream;
+      if (used) {  // another class already runs on the main stream
+        st = side[c];
+        if (!forked) throw BErr(CS_E_CUDA, "batch streams not forked");
+        BK(cudaStreamWaitEvent(st, fork, 0));
+      } else {
+        BK(cudaEventRecord(fork, stream));
+        forked = true;
+      }
+      const int groups = std::max(1, std::min(count, ctas / size));
+      BK((cudaError_t)batch_launch_step(d, order.p + classStart[c], count, work.p + c, size, virt, threads,
+                                        groups * size, st));
+      if (used) {
+        BK(cudaEventRecord(join[c], st));
+        BK(cudaStreamWaitEvent(stream, join[c], 0));
+      }
+      used = true;
+    }
   }
 
   void step(double h, int steps) {

@@ -7,10 +7,13 @@ namespace cs {
 
 // Corner share of one triangle's membrane HVP (membrane-hvp.ts:18-75):
 // dF = Ds(p) Dm^-1, dE, dS, dP = dF S + F dS, force = -area * dP Dm^-T.
+// NC: the record is constant for the kernel (read-only cache); else a plain load.
+template <bool NC = true>
 __device__ __forceinline__ void tri_hvp_corner(const float* T, const float3 p0, const float3 p1, const float3 p2,
                                                int corner, float C00, float C11, float C01, float G, float o[3]) {
-  const float4 t0 = __ldg((const float4*)T), t1 = __ldg((const float4*)(T + 4)), t2 = __ldg((const float4*)(T + 8)),
-               t3 = __ldg((const float4*)(T + 12));
+  const float4* T4 = (const float4*)T;
+  const float4 t0 = NC ? __ldg(T4) : T4[0], t1 = NC ? __ldg(T4 + 1) : T4[1], t2 = NC ? __ldg(T4 + 2) : T4[2],
+               t3 = NC ? __ldg(T4 + 3) : T4[3];
   const float F0[3] = {t0.x, t0.y, t0.z}, F1[3] = {t0.w, t1.x, t1.y};
   const float S00 = t1.z, S11 = t1.w, S01 = t2.x;
   const float a = t2.y, b = t2.z, c = t2.w, dd = t3.x, s = t3.y;

@@ -132,3 +132,17 @@ def test_batch_matches_the_oracle_exact_mode_when_converged():
               f"oracle {co}/{steps}")
         assert co == steps and conv[i] >= steps - 1, (conv[i], co)
         assert err <= 1e-7, err
+
+
+@pytest.mark.parametrize("side,count", [(55, 160), (39, 320), (38, 3)])
+def test_sheet_is_the_same_in_a_cluster_and_by_a_lone_block(side, count):
+    """A sheet's reductions have the shape of its size class whether a cluster
+    steps it (a small batch) or a lone block does (a batch that fills the
+    device): 55 x 55 and 39 x 39 are the smallest sheets of the classes of four
+    and two blocks, 38 x 38 the largest of the class of one."""
+    sheets = configs.batch_sheets(count=count, side_min=side, side_max=side)
+    full, alone = BatchSolver(sheets), BatchSolver([sheets[count // 2]])
+    full.step(0.01, steps=2)
+    alone.step(0.01, steps=2)
+    assert np.array_equal(full.positions(count // 2), alone.positions(0))
+    assert full.stats()[count // 2] == alone.stats()[0]
