@@ -337,8 +337,9 @@ __device__ __forceinline__ long long ord_after(const OrdStage& s) {
 // dependent chain is five integer operations per list; the windows are checked
 // eight lists at a time. Lists without a step, or whose window does not hold,
 // are applied stage by stage.
-static __device__ __noinline__ long long ord_walk(long long b, int n, const OrdStage* w, int stride, const OrdStage* more,
-                                              int moreStride, const OrdStep* st, const double* T) {
+static __device__ __noinline__ long long ord_walk(long long b, int n, const OrdStage* w, int stride,
+                                                  const OrdStage* more, int moreStride, const OrdStep* st,
+                                                  const double* T) {
   int i = 0;
   while (i < n) {
     const long long dl = b - w[(size_t)i * stride].B;

@@ -15,8 +15,8 @@
 // earlier, so each costs one barrier. Sheets up to kPcg64ClusterN vertices run
 // in one 16-CTA cluster (hardware barrier), larger ones on the whole grid.
 // Whole steps on a B200 against one-thread chains on a cooperative grid: 41 x 9
-// strip (Jacobi, two steps) 47.6 -> 38.5 ms, 64 x 64 drape (Schwarz) 86.0 ->
-// 20.6 ms, 121 x 95 garment on a sphere (Jacobi) 458 -> 54 ms, the same bits. An
+// strip (Jacobi, two steps) 43.7 -> 31.4 ms, 64 x 64 drape (Schwarz) 54.0 ->
+// 14.7 ms, 121 x 95 garment on a sphere (Jacobi) 411 -> 61 ms, the same bits. An
 // iteration is now bound by its barriers and the stage walks (5,000-8,000
 // cycles per dot product), with Schwarz by the domains' substitution chains.
 #include <cooperative_groups.h>
@@ -76,12 +76,24 @@ __device__ __noinline__ double seg_before(const double* row, int seg) {
   return wsum(s);
 }
 
-// Publishes at `out` the stages of a segment, as one map where they collapse: the
+// The same for three rows (`stride` apart) combined with weights, their loads in flight together.
+__device__ __noinline__ double seg_before3(const double* row, size_t stride, int seg, double w1, double w2) {
+  const int lane = threadIdx.x & 31;
+  double s = 0;
+  for (int i = lane; i < seg; i += 32) {
+    const double a = __ldcg(row + i), b = __ldcg(row + stride + i), c = __ldcg(row + 2 * stride + i);
+    s += a + w1 * b + w2 * c;
+  }
+  return wsum(s);
+}
+
+// Publishes the stages of a segment, as one map where they collapse: the first at
+// `head` (contiguous over the segments, all a walk usually reads), a longer list at `out`. The
 // lane's chunk of the local terms t, g0 + c.l0 its place in the whole sum, `before`
 // the approximate sum before the segment (first: it begins the sum). mine: one
 // warp's scratch.
-__device__ __noinline__ void seg_order(OrdStage* out, const double* t, int g0, Chunk c, double before, bool first,
-                                       OrdStage* mine) {
+__device__ __noinline__ void seg_order(OrdStage* head, OrdStage* out, const double* t, int g0, Chunk c, double before,
+                                       bool first, OrdStage* mine) {
   const int lane = threadIdx.x & 31;
   if (first) {
     const int end = __shfl_sync(0xffffffffu, c.l0 + c.cnt, 31);
@@ -102,20 +114,22 @@ __device__ __noinline__ void seg_order(OrdStage* out, const double* t, int g0, C
     ord_collapse(mine);
   }
   __syncwarp();
-  for (int i = lane, n = mine[0].count * 4; i < n; i += 32)
+  const int n = mine[0].count;
+  if (lane < 4) reinterpret_cast<int4*>(head)[lane] = reinterpret_cast<const int4*>(mine)[lane];
+  for (int i = lane; n > 1 && i < n * 4; i += 32)
     reinterpret_cast<int4*>(out)[i] = reinterpret_cast<const int4*>(mine)[i];
   __syncwarp();
 }
 
-// The exact sums of nk (1 or 2) kinds (stages st, global terms T): every thread of the CTA
+// The exact sums of nk (1 or 2) kinds (heads h, lists st, global terms T): every thread of the CTA
 // calls it, warp q walks kind q. wst holds the first stage of each segment, loaded
 // together (a longer list's rest is read as it is reached), stp their steps.
-__device__ __noinline__ void walk(const OrdStage* st0, const OrdStage* st1, int nk, int NS, const double* T0,
-                                  const double* T1, OrdStage* wst, OrdStep* stp, double* res) {
+__device__ __noinline__ void walk(const OrdStage* h0, const OrdStage* h1, const OrdStage* st0, const OrdStage* st1,
+                                  int nk, int NS, const double* T0, const double* T1, OrdStage* wst, OrdStep* stp,
+                                  double* res) {
   for (int i = threadIdx.x; i < nk * NS * 4; i += blockDim.x) {
-    const int seg = i >> 2;
-    const OrdStage* src = seg >= NS ? st1 + (size_t)(seg - NS) * kPcg64Stages : st0 + (size_t)seg * kPcg64Stages;
-    reinterpret_cast<int4*>(wst + seg)[i & 3] = __ldcg(reinterpret_cast<const int4*>(src) + (i & 3));
+    const int4* src = reinterpret_cast<const int4*>(i >= NS * 4 ? h1 - NS : h0);
+    reinterpret_cast<int4*>(wst)[i] = __ldcg(src + i);
   }
   __syncthreads();
   const int q = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -175,14 +189,21 @@ __global__ void __launch_bounds__(kPcg64T, 1) k_pcg64(const __grid_constant__ Ar
     if (vs) glob[g0 + i] = v;
   };
   auto stages = [&](int kind) { return P.stages + (size_t)kind * NS * kPcg64Stages; };
+  auto heads = [&](int kind) { return P.heads + (size_t)kind * NS; };
   auto order = [&](int kind, int r, const double* t, double before) {
     const int seg = b * R + r;
-    seg_order(stages(kind) + (size_t)seg * kPcg64Stages, t, g0, seg_chunk(P, r, nt), before, seg == 0, mine[warp]);
+    seg_order(heads(kind) + seg, stages(kind) + (size_t)seg * kPcg64Stages, t, g0, seg_chunk(P, r, nt), before,
+              seg == 0, mine[warp]);
   };
   auto before = [&](int row, int r) { return seg_before(P.sums + (size_t)row * NS, b * R + r); };
-  auto walk1 = [&](int kind, const double* T0) { walk(stages(kind), nullptr, 1, NS, T0, nullptr, wst, stp, res); };
+  auto before3 = [&](int row, int r, double w1, double w2) {
+    return seg_before3(P.sums + (size_t)row * NS, NS, b * R + r, w1, w2);
+  };
+  auto walk1 = [&](int kind, const double* T0) {
+    walk(heads(kind), nullptr, stages(kind), nullptr, 1, NS, T0, nullptr, wst, stp, res);
+  };
   auto walk2 = [&](int k0, int k1, const double* T0, const double* T1) {
-    walk(stages(k0), stages(k1), 2, NS, T0, T1, wst, stp, res);
+    walk(heads(k0), heads(k1), stages(k0), stages(k1), 2, NS, T0, T1, wst, stp, res);
   };
   // Warps q * R .. q * R + R - 1 order the segments of the q-th pending sum.
   auto segment = [&](int q) { return warp - q * R; };
@@ -448,14 +469,13 @@ __global__ void __launch_bounds__(kPcg64T, 1) k_pcg64(const __grid_constant__ Ar
       const int q = warp / R, r = segment(q);
       if (q < 2) {
         const int row = q ? W_RZ : W_RR;
-        order(q ? D_RZ : D_RR, r, q ? t2 : t1,
-              before(row, r) - 2 * alpha * before(row + 1, r) + alpha * alpha * before(row + 2, r));
+        order(q ? D_RZ : D_RR, r, q ? t2 : t1, before3(row, r, -2 * alpha, alpha * alpha));
       } else {
         direction_sums(r);
       }
     }
     barrier();
-    walk(stages(D_RR), stages(D_RZ), jacobi ? 2 : 1, NS, d.T1, d.T2, wst, stp, res);
+    walk(heads(D_RR), heads(D_RZ), stages(D_RR), stages(D_RZ), jacobi ? 2 : 1, NS, d.T1, d.T2, wst, stp, res);
     residual = sqrt(res[0]);
     double rzNew = res[1];
     if (residual < absTol) { iters = k + 1; done = true; break; }
@@ -497,8 +517,7 @@ __global__ void __launch_bounds__(kPcg64T, 1) k_pcg64(const __grid_constant__ Ar
     rz = rzNew;
     __syncthreads();
     if (warp < R) {
-      order(D_PP, warp, t3,
-            before(W_ZZ, warp) + 2 * beta * before(W_ZP, warp) + beta * beta * before(W_PP, warp));
+      order(D_PP, warp, t3, before3(W_ZZ, warp, 2 * beta, beta * beta));
     }
     barrier();
     walk1(D_PP, d.T3);
@@ -639,7 +658,8 @@ void build_pcg64_plan(const HostMesh& me, int sms, int clusterMax, bool lists, P
   }
   p.nv = (me.n + p.G - 1) / p.G;
   const int terms = 3 * p.nv;
-  p.R = p.G == 1 ? 4 : p.G <= 16 ? 2 : 1;
+  // fewer segments to walk against fewer terms per lane to map
+  p.R = p.G == 1 ? 4 : p.G <= 16 && terms > 160 ? 2 : 1;
   p.K = ((terms + p.R * 32 - 1) / (p.R * 32)) | 1;
   p.NS = p.G * p.R;
   out.slotOff.assign(1, 0);
@@ -667,7 +687,8 @@ void build_pcg64_plan(const HostMesh& me, int sms, int clusterMax, bool lists, P
     out.slotOff.push_back((int)out.slots.size());
   }
   p.elemStride = 18 * (size_t)std::max(most, 1);
-  const size_t walk = 2 * (size_t)p.NS * (sizeof(OrdStage) + sizeof(OrdStep)), vec = 9 * (size_t)terms * 8, elem = p.elemStride * 8;
+  const size_t walk = 2 * (size_t)p.NS * (sizeof(OrdStage) + sizeof(OrdStep));
+  const size_t vec = 9 * (size_t)terms * 8, elem = p.elemStride * 8;
   const size_t offs = ((size_t)(p.nv + 1) * 4 + 15) & ~(size_t)15;
   p.vecSmem = walk + offs + vec <= kMaxDyn;
   p.elemSmem = walk + offs + (p.vecSmem ? vec : 0) + elem <= kMaxDyn;

@@ -29,7 +29,8 @@ struct Pcg64Plan {
   const int4* slots = nullptr;    // per CTA: its incident triangles (i0, i1, i2, triangle)
   const uint32_t* inc = nullptr;  // 3m, memRec's order: CTA slot << 2 | corner
   double* elem = nullptr;         // G * elemStride when not in shared memory
-  OrdStage* stages = nullptr;     // 4 x NS x kPcg64Stages
+  OrdStage* heads = nullptr;      // 4 x NS: the first stage of each segment
+  OrdStage* stages = nullptr;     // 4 x NS x kPcg64Stages: lists of more than one
   double* sums = nullptr;         // kPcg64Rows x NS
   double* curv = nullptr;         // barrier curvature per active contact
 };

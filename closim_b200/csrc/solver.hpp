@@ -123,11 +123,43 @@ class Solver {
   int mxCluster = 0;  // CTAs of the one-cluster PCG (0: grid-wide cooperative PCG)
   // Per-CTA element lists of the one-cluster PCG's resident phase A; clRes[k]
   // (k = 1 with the Gauss-Newton bending term) says whether they fit.
-  ClusterPlanHost clHost;
-  DBuf<int> clVb, clHaloOff, clHalo, clTriOff, clTriId, clHinOff, clHinId, clIncOff, clIncHin, clOwnHalo, clVDst;
-  DBuf<uint16_t> clTriLoc, clHinLoc;
-  DBuf<uint32_t> clInc;
-  ClPlan clPlan{};
+  // Per-CTA lists of a resident PCG and their device copies: cl for the cluster,
+  // grl for the grid-wide kernel.
+  struct ClLists {
+    ClusterPlanHost host;
+    DBuf<int> vb, haloOff, halo, triOff, triId, hinOff, hinId, incOff, incHin, ownHalo, vDst;
+    DBuf<uint16_t> triLoc, hinLoc;
+    DBuf<uint32_t> inc;
+    ClPlan plan{};
+    void upload(cudaStream_t st) {
+      auto up = [&](DBuf<int>& d, const std::vector<int>& v) {
+        d.alloc(std::max<size_t>(v.size(), 1));
+        d.upload(v.data(), v.size(), st);
+        return (const int*)d.p;
+      };
+      plan.vb = up(vb, host.vb);
+      plan.haloOff = up(haloOff, host.haloOff);
+      plan.halo = up(halo, host.halo);
+      plan.triOff = up(triOff, host.triOff);
+      plan.triId = up(triId, host.triId);
+      plan.hinOff = up(hinOff, host.hinOff);
+      plan.hinId = up(hinId, host.hinId);
+      plan.incOff = up(incOff, host.incOff);
+      plan.incHin = up(incHin, host.incHin);
+      plan.ownHalo = up(ownHalo, host.ownHalo);
+      plan.vDst = up(vDst, host.vDst);
+      triLoc.alloc(std::max<size_t>(host.triLoc.size(), 4));
+      triLoc.upload(host.triLoc.data(), host.triLoc.size(), st);
+      hinLoc.alloc(std::max<size_t>(host.hinLoc.size(), 4));
+      hinLoc.upload(host.hinLoc.data(), host.hinLoc.size(), st);
+      inc.alloc(std::max<size_t>(host.inc.size(), 1));
+      inc.upload(host.inc.data(), host.inc.size(), st);
+      plan.triLoc = reinterpret_cast<const ushort4*>(triLoc.p);
+      plan.hinLoc = reinterpret_cast<const ushort4*>(hinLoc.p);
+      plan.inc = inc.p;
+    }
+  };
+  ClLists cl, grl;
   bool clRes[2] = {false, false};
   size_t clSmem[2] = {0, 0};  // launch's dynamic shared memory
   int clCap[2] = {0, 0};      // on-chip contact records per CTA
@@ -360,13 +392,14 @@ class Solver {
     pcgSlots.upload(pcg.slots.data(), pcg.slots.size(), stream);
     pcgInc.upload(pcg.inc.data(), pcg.inc.size(), stream);
     pcgElem.alloc(p.elemSmem ? 1 : (size_t)p.G * p.elemStride);
-    pcgStages.alloc(4 * (size_t)p.NS * kPcg64Stages);
+    pcgStages.alloc(4 * (size_t)p.NS * (kPcg64Stages + 1));
     pcgSums.alloc((size_t)kPcg64Rows * p.NS);
     p.slotOff = pcgSlotOff.p;
     p.slots = pcgSlots.p;
     p.inc = pcgInc.p;
     p.elem = pcgElem.p;
-    p.stages = pcgStages.p;
+    p.heads = pcgStages.p;
+    p.stages = pcgStages.p + 4 * (size_t)p.NS;
     p.sums = pcgSums.p;
   }
 
@@ -512,8 +545,8 @@ class Solver {
                   opts.pcg_max_iters, newtonTol, adjOut.p};
         CK((cudaError_t)newton_exact_solve(a, adj_grid_blocks(d), stream));
         lc += 3;
-      } else if (mixed() && mxGrid > 0) {
-        ClPlan plan = clPlan;
+      } else if (mixed() && grid_pcg(mb.hrec != nullptr)) {
+        ClPlan plan = grl.plan;
         plan.smemBytes = (int)mxGridSmem[mb.hrec ? 1 : 0];
         CK((cudaError_t)mx_launch_pcg_grid(d, mb, plan, fp.p, fp2.p, d.hasContact ? d.c.dd : nullptr, mxGridPart.p,
                                            opts.pcg_max_iters,
@@ -684,7 +717,8 @@ class Solver {
     DBuf<double> xN, vN;     // state after the rollout
     bool valid = false;
   } ro;
-  DBuf<double> adjRhs, adjMu, adjR, adjZ, adjP, adjAp, adjTri, adjHin, adjTerms, adjLamX, adjLamV, adjAcc, adjOut, adjDom;
+  DBuf<double> adjRhs, adjMu, adjR, adjZ, adjP, adjAp, adjTri, adjHin, adjTerms, adjLamX, adjLamV, adjAcc, adjOut;
+  DBuf<double> adjDom;
   AdjStats adjStats{};
   int adjMaxIters = 2000;
   double adjTol = 1e-10;
@@ -707,22 +741,21 @@ class Solver {
   // largest CTA's share fits in shared memory (CLOSIM_MX_RESIDENT=0 turns it off).
   void build_cluster_resident() {
     clRes[0] = clRes[1] = false;
-    clPlan = ClPlan{};
+    cl.plan = ClPlan{};
     const char* env = std::getenv("CLOSIM_MX_RESIDENT");
     if (env && std::string(env) == "0") return;
-    build_cluster_plan(mesh, mxCluster, kClWarps, clHost);
-    if (!clHost.ok) return;
+    build_cluster_plan(mesh, mxCluster, kClWarps, cl.host);
+    if (!cl.host.ok) return;
     // the shared memory left over holds contact records (up to 8192 per CTA)
     for (int k = 0; k < 2; k++) {
-      const size_t base = k ? clHost.smemHinge : clHost.smemNoHinge;
+      const size_t base = k ? cl.host.smemHinge : cl.host.smemNoHinge;
       const long room = (long)kClMaxDynSmem - (long)base - 32;
       clCap[k] = room > 0 ? (int)std::min<long>(room / kClRecBytes, 8192) : 0;
       clSmem[k] = base + 32 + (size_t)clCap[k] * kClRecBytes;
     }
     clRes[1] = mx_cluster_resident_ok(mxCluster, clSmem[1]);
     clRes[0] = mx_cluster_resident_ok(mxCluster, clSmem[0]);
-    if (!clRes[0] && !clRes[1]) return;
-    upload_cluster_plan();
+    if (clRes[0] || clRes[1]) cl.upload(stream);
   }
   // Sheets past kMxGridN vertices whose lists do not fit one cluster: the
   // grid-wide resident PCG (mixed_cluster.cu), one CTA per SM. Below that the
@@ -733,56 +766,34 @@ class Solver {
     mxGrid = 0;
     if (mxCluster <= 0) {
       clRes[0] = clRes[1] = false;
-      clPlan = ClPlan{};
+      cl.plan = ClPlan{};
     }
-    if (forceCluster || clRes[0] || clRes[1] || mesh.n <= kMxGridN || mesh.maxDomain > 8) return;
+    if (forceCluster || (clRes[0] && clRes[1]) || mesh.n <= kMxGridN || mesh.maxDomain > 8) return;
     const char* env = std::getenv("CLOSIM_MX_RESIDENT");
     if (env && std::string(env) == "0") return;
     int sms = 0;
     CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
     const int ctas = std::min(std::min(sms, kMxGridMax), (mesh.n + 31) / 32);
-    build_cluster_plan(mesh, ctas, kClWarps, clHost, false);
-    const size_t most = mxCluster > 0 ? clHost.smemHinge : clHost.smemNoHinge;  // exact mode is FP64 without a cluster
-    if (!clHost.ok || !mx_grid_ok(ctas, most)) return;
+    build_cluster_plan(mesh, ctas, kClWarps, grl.host, false);
+    // without a cluster (past 20,000 vertices) exact mode solves in FP64
+    const size_t most = mxCluster > 0 ? grl.host.smemHinge : grl.host.smemNoHinge;
+    if (!grl.host.ok || !mx_grid_ok(ctas, most)) return;
     mxGrid = ctas;
-    mxGridSmem[0] = clHost.smemNoHinge;
-    mxGridSmem[1] = clHost.smemHinge;
+    mxGridSmem[0] = grl.host.smemNoHinge;
+    mxGridSmem[1] = grl.host.smemHinge;
     mxGridPart.alloc(8 * (size_t)kMxGridMax);
     if (fp2.n < 3 * (size_t)mesh.n) fp2.alloc(3 * (size_t)mesh.n);
-    upload_cluster_plan();
+    grl.upload(stream);
   }
-  void upload_cluster_plan() {
-    auto up = [&](DBuf<int>& b, const std::vector<int>& v) {
-      b.alloc(std::max<size_t>(v.size(), 1));
-      b.upload(v.data(), v.size(), stream);
-      return (const int*)b.p;
-    };
-    clPlan.vb = up(clVb, clHost.vb);
-    clPlan.haloOff = up(clHaloOff, clHost.haloOff);
-    clPlan.halo = up(clHalo, clHost.halo);
-    clPlan.triOff = up(clTriOff, clHost.triOff);
-    clPlan.triId = up(clTriId, clHost.triId);
-    clPlan.hinOff = up(clHinOff, clHost.hinOff);
-    clPlan.hinId = up(clHinId, clHost.hinId);
-    clPlan.incOff = up(clIncOff, clHost.incOff);
-    clPlan.incHin = up(clIncHin, clHost.incHin);
-    clPlan.ownHalo = up(clOwnHalo, clHost.ownHalo);
-    clPlan.vDst = up(clVDst, clHost.vDst);
-    clTriLoc.alloc(std::max<size_t>(clHost.triLoc.size(), 4));
-    clTriLoc.upload(clHost.triLoc.data(), clHost.triLoc.size(), stream);
-    clHinLoc.alloc(std::max<size_t>(clHost.hinLoc.size(), 4));
-    clHinLoc.upload(clHost.hinLoc.data(), clHost.hinLoc.size(), stream);
-    clInc.alloc(std::max<size_t>(clHost.inc.size(), 1));
-    clInc.upload(clHost.inc.data(), clHost.inc.size(), stream);
-    clPlan.triLoc = reinterpret_cast<const ushort4*>(clTriLoc.p);
-    clPlan.hinLoc = reinterpret_cast<const ushort4*>(clHinLoc.p);
-    clPlan.inc = clInc.p;
-  }
+  // Whether a mixed solve takes the grid-wide kernel: its lists exist and the
+  // cluster's do not fit in this mode (hinges: with the bending term), or the
+  // preconditioner is Jacobi, which the resident cluster kernel does not have.
+  bool grid_pcg(bool hinges) const { return mxGrid > 0 && !(clRes[hinges ? 1 : 0] && precond_code() >= 1); }
   // The plan for a launch: resident when this launch's lists fit.
   ClPlan cluster_plan_for(const MixBufs& m) const {
-    ClPlan p = clPlan;
+    ClPlan p = cl.plan;
     const int k = m.hrec ? 1 : 0;
-    p.resident = clRes[k] && clHost.nrank == mxCluster && d.precond >= 1 ? 1 : 0;
+    p.resident = clRes[k] && cl.host.nrank == mxCluster && d.precond >= 1 ? 1 : 0;
     p.smemBytes = p.resident ? (int)clSmem[k] : 0;
     p.cCap = p.resident ? clCap[k] : 0;
     return p;
@@ -922,7 +933,8 @@ class Solver {
         launch_diag_init(d, beta, stream);
         if (d.precond >= 1) launch_schwarz_factor(d, stream);
         adj_rhs(d, adjLamX.p, adjLamV.p, damp, adjRhs.p, stream);
-        AdjArgs a{d, adjRhs.p, adjMu.p, adjR.p, adjZ.p, adjP.p, adjAp.p, adjTri.p, adjHin.p, adjDom.p, d.kb, 0, maxIters, tol,
+        AdjArgs a{d, adjRhs.p, adjMu.p, adjR.p, adjZ.p, adjP.p, adjAp.p, adjTri.p, adjHin.p, adjDom.p, d.kb, 0,
+                  maxIters, tol,
                   adjOut.p};
         CK((cudaError_t)adj_launch_pcg(a, blocks, stream));
         adj_theta(d, adjMu.p, adjTerms.p, adjAcc.p, stream);

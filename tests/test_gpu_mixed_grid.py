@@ -1,0 +1,53 @@
+"""The grid-wide resident PCG of the mixed path (k_mx_pcg_grid) against the
+kernels it replaces there (the gathering cluster kernel, and past 20,000
+vertices the element-scatter kernel), forced by CLOSIM_MX_RESIDENT=0.
+
+Every vertex and element does the same FP32 operations in the same order; only
+the FP64 dot products are summed in another order, which moves an FP32 alpha or
+beta by an ulp when their ratio lies within 1e-16 of a rounding boundary, about
+once in 1e8 iterations. So one step at the reference budget agrees to 1e-9 of
+the positions' size, and a converged step to what gradTol leaves."""
+import numpy as np
+import pytest
+
+import closim_b200 as cb
+from closim_b200 import configs
+
+pytestmark = pytest.mark.gpu
+
+
+def one_step(monkeypatch, resident, cfg, mode, **opts):
+    if resident:
+        monkeypatch.delenv("CLOSIM_MX_RESIDENT", raising=False)
+    else:
+        monkeypatch.setenv("CLOSIM_MX_RESIDENT", "0")
+    s = cb.CudaSolver("mixed", **{**cfg["options"], **opts})
+    sc = configs.make_scene(cfg)
+    s.initialize(sc)
+    s.setGraphMode(False)
+    s.setNewtonMode(mode, 3e-4)
+    s.step(cfg["h"])
+    info, st = s.launchInfo(), s.lastStats
+    s.close()
+    return sc.positions.copy(), st, info
+
+
+@pytest.mark.parametrize("nx,ny,precond,mode", [
+    (65, 64, "mas2", "exact"),           # just past the cluster's lists in this mode
+    (99, 84, "schwarz", "reference"),
+    (1050, 3, "schwarz", "exact"),       # a ribbon: many vertices of the halo per owned one
+    (79, 71, "jacobi", "reference"),
+    (150, 140, "schwarz", "reference"),  # past 20,000 vertices
+    (255, 252, "schwarz", "reference"),  # near the most shared memory takes
+])
+def test_grid_pcg_matches_the_kernels_it_replaces(monkeypatch, nx, ny, precond, mode):
+    cfg = configs.floor_drape(nx=nx, ny=ny, w=0.0127 * nx, hgt=0.0127 * ny, height=0.002, precond=precond)
+    cfg["v"] = np.tile([0.3, -0.1, 0.1], cfg["x"].size // 3)
+    cfg["fixed_pins"] = [0, nx]
+    opts = dict(newtonIters=30, pcgMaxIters=2000, gradTol=1e-9) if mode == "exact" else {}
+    x1, st1, info = one_step(monkeypatch, True, cfg, mode, **opts)
+    x0, st0, old = one_step(monkeypatch, False, cfg, mode, **opts)
+    assert info["pcgGridCtas"] <= 148 and old["pcgGridCtas"] != info["pcgGridCtas"]
+    assert st1.contact["floorPairs"] > 0
+    assert st1.newtonItersUsed == st0.newtonItersUsed and st1.pcgIters == st0.pcgIters
+    assert np.max(np.abs(x1 - x0)) <= 1e-9 * np.max(np.abs(x0))
