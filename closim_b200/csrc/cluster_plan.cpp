@@ -8,7 +8,8 @@
 
 namespace cs {
 
-void build_cluster_plan(const HostMesh& me, int nrank, int warpsPerCta, ClusterPlanHost& p, bool domains) {
+void build_cluster_plan(const HostMesh& me, int nrank, int warpsPerCta, ClusterPlanHost& p, bool domains,
+                        bool hinges) {
   p = ClusterPlanHost{};
   p.nrank = nrank;
   p.warpsPerCta = warpsPerCta;
@@ -48,7 +49,7 @@ void build_cluster_plan(const HostMesh& me, int nrank, int warpsPerCta, ClusterP
     for (int v = v0; v < v1; v++) {
       halo.push_back(v);
       for (uint32_t q = me.memOff[v]; q < me.memOff[v + 1]; q++) tris.push_back((int)(me.memRec[q] >> 2));
-      for (uint32_t q = me.hinOff[v]; q < me.hinOff[v + 1]; q++) hins.push_back((int)(me.hinRec[q] >> 2));
+      for (uint32_t q = me.hinOff[v]; hinges && q < me.hinOff[v + 1]; q++) hins.push_back((int)(me.hinRec[q] >> 2));
     }
     std::sort(tris.begin(), tris.end());
     tris.erase(std::unique(tris.begin(), tris.end()), tris.end());
@@ -81,7 +82,7 @@ void build_cluster_plan(const HostMesh& me, int nrank, int warpsPerCta, ClusterP
         p.inc.push_back(((uint32_t)tslot[rec >> 2] << 2) | (rec & 3));
       }
       p.incHin[v] = (int)p.inc.size();
-      for (uint32_t q = me.hinOff[v]; q < me.hinOff[v + 1]; q++) {
+      for (uint32_t q = me.hinOff[v]; hinges && q < me.hinOff[v + 1]; q++) {
         const uint32_t rec = me.hinRec[q];
         p.inc.push_back(((uint32_t)hslot[rec >> 2] << 2) | (rec & 3));
       }

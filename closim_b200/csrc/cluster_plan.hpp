@@ -90,7 +90,9 @@ struct ClusterPlanHost {
 // ok stays false when a halo needs more than 16-bit ids, when the domains do
 // not partition the vertices, or when some warp would own more than 3 domains.
 // domains = false (the grid-wide kernel, whose phase B is not resident): no
-// domain slots, any number of domains per warp.
-void build_cluster_plan(const HostMesh& me, int nrank, int warpsPerCta, ClusterPlanHost& p, bool domains = true);
+// domain slots, any number of domains per warp. hinges = false: no hinge lists (a
+// sheet whose exact mode solves elsewhere), a smaller halo.
+void build_cluster_plan(const HostMesh& me, int nrank, int warpsPerCta, ClusterPlanHost& p, bool domains = true,
+                        bool hinges = true);
 
 }  // namespace cs

@@ -774,8 +774,8 @@ class Solver {
     int sms = 0;
     CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
     const int ctas = std::min(std::min(sms, kMxGridMax), (mesh.n + 31) / 32);
-    build_cluster_plan(mesh, ctas, kClWarps, grl.host, false);
     // without a cluster (past 20,000 vertices) exact mode solves in FP64
+    build_cluster_plan(mesh, ctas, kClWarps, grl.host, false, mxCluster > 0);
     const size_t most = mxCluster > 0 ? grl.host.smemHinge : grl.host.smemNoHinge;
     if (!grl.host.ok || !mx_grid_ok(ctas, most)) return;
     mxGrid = ctas;
