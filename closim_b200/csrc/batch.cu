@@ -10,7 +10,8 @@
 // The launch is persistent: groups take sheets from a work list ordered largest
 // first. A sheet's PCG is a chain of short passes over its vertices, bound by the
 // latency of its gathers; one SM per sheet left the batch waiting for its largest
-// sheet (96 sheets of 16 to 80 vertices a side: 84 ms a step, 44 with clusters). The algorithm per sheet is newton.ts:27-303 with the floor-contact
+// sheet (96 sheets of 16 to 80 vertices a side: 84 ms a step, 44 with clusters).
+// The algorithm per sheet is newton.ts:27-303 with the floor-contact
 // subset of contact-assembly.ts (kind 2: per-vertex barrier, lagged friction,
 // floor CCD, restitution); the bending gradient is the analytic gradient of
 // the hinge energy instead of its central difference (bending.ts:19-42).
