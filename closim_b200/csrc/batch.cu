@@ -568,6 +568,9 @@ __global__ void __launch_bounds__(T, 1) k_batch_step(BatchDev b, const int* orde
   __shared__ int sheetSh;
   const int rank = size > 1 ? (int)cg::this_cluster().block_rank() : 0;
   Group G{size, rank, rank * T + (int)threadIdx.x, size * T, virt, sm, part, bank, 0};
+  // Shared memory of a peer may be touched once every CTA of the cluster has
+  // started, which co-scheduling alone does not promise.
+  gsync(G);
   for (int guard = 0; guard <= count; guard++) {
     if (rank == 0 && threadIdx.x == 0) {
       const unsigned k = atomicAdd(work, 1u);

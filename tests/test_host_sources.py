@@ -1,5 +1,7 @@
-"""The TypeScript host (host/ts/cuda-solver.ts) and its N-API addon
-(host/napi/addon.cc) against each other and against the C ABI, on the CPU.
+"""What can be read off the sources on the CPU: the TypeScript host
+(host/ts/cuda-solver.ts) and its N-API addon (host/napi/addon.cc) against each
+other and against the C ABI, and the order of cluster barriers in the kernels
+that use distributed shared memory.
 
 No Node toolchain exists here, so these checks stand in for a build: every
 addon function the TS class calls is exported by the addon, every cs_* call
@@ -56,3 +58,30 @@ def test_addon_compiles_against_napi_declarations():
     r = subprocess.run(["g++", "-std=c++17", "-Wall", "-Wextra", "-Werror", "-fsyntax-only", "-I", stub, "-I",
                         os.path.join(ROOT, "include"), ADDON], capture_output=True, text=True)
     assert r.returncode == 0, r.stderr
+
+
+CSRC = os.path.join(ROOT, "closim_b200", "csrc")
+
+
+def kernel_body(path, name):
+    """The text between the braces of the __global__ function `name`, without comments."""
+    src = re.sub(r"//[^\n]*", "", open(path).read())
+    i = re.search(rf"__global__[^;{{]*\b{name}\(", src).end()
+    i = j = src.index("{", i)
+    depth = 0
+    while True:
+        depth += {"{": 1, "}": -1}.get(src[j], 0)
+        j += 1
+        if depth == 0:
+            return src[i:j]
+
+
+@pytest.mark.parametrize("file,kernel,barrier,remote", [
+    ("batch.cu", "k_batch_step", r"\bgsync\(G\)", r"map_shared_rank|\bstep_sheet\("),
+])
+def test_cluster_barrier_precedes_the_first_remote_access(file, kernel, barrier, remote):
+    """A CTA's shared memory may be reached by its cluster's peers only once all
+    of them have started: a cluster barrier comes before the first access."""
+    body = kernel_body(os.path.join(CSRC, file), kernel)
+    first = re.search(remote, body)
+    assert first and re.search(barrier, body[:first.start()]), (kernel, body[:200])
