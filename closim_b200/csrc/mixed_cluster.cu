@@ -487,6 +487,9 @@ __device__ __forceinline__ void cl_dof(const Dev& d, const MixBufs& mb, const fl
 template <bool RES>
 __global__ void __launch_bounds__(kClT, 1) k_mx_pcg_cluster(ClArgs A) {
   cg::cluster_group cl = cg::this_cluster();
+  // Shared memory of a peer may be touched once every CTA of the cluster has
+  // started, which co-scheduling alone does not promise: waited for before the first push.
+  cl.barrier_arrive();
   __shared__ double sm[32];
   // Partials alternate between two banks: a bank is rewritten only after the
   // cluster barrier that follows every CTA's read of it.
@@ -624,6 +627,7 @@ __global__ void __launch_bounds__(kClT, 1) k_mx_pcg_cluster(ClArgs A) {
   }
   {
     const double v3[3] = {bb, rr, rz};
+    cl.barrier_wait();
     block_partials<3>(cl, v3, red[round & 1], rank, nrank, wsm);
   }
   cl.sync();

@@ -78,6 +78,7 @@ def kernel_body(path, name):
 
 @pytest.mark.parametrize("file,kernel,barrier,remote", [
     ("batch.cu", "k_batch_step", r"\bgsync\(G\)", r"map_shared_rank|\bstep_sheet\("),
+    ("mixed_cluster.cu", "k_mx_pcg_cluster", r"\bcl\.(sync|barrier_wait)\(\)", r"map_shared_rank|\bblock_partials<"),
 ])
 def test_cluster_barrier_precedes_the_first_remote_access(file, kernel, barrier, remote):
     """A CTA's shared memory may be reached by its cluster's peers only once all
