@@ -179,10 +179,12 @@ __global__ void __launch_bounds__(kPcg64T, 1) k_pcg64(const __grid_constant__ Ar
   double* const t3 = vs ? vecS + 8 * len : d.T3 + g0;
   double* const el = P.elemSmem ? vecS + (vs ? 9 * len : 0) : P.elem + (size_t)b * P.elemStride;
   const int s0 = P.slotOff[b], nSlot = P.slotOff[b + 1] - s0;
-  // this launch's contact-record offsets of the owned vertices
+  // this launch's contact-record offsets of the owned vertices, at the end of the
+  // shared memory where they fit
   uint32_t* const cOffS = reinterpret_cast<uint32_t*>(dyn + P.smem) - (P.nv + 1);
-  if (d.hasContact)
+  if (d.hasContact && P.offSmem)
     for (int i = threadIdx.x; i <= nOwn; i += T) cOffS[i] = d.c.cOff[vb0 + i];
+  auto cOff = [&](int lv) { return P.offSmem ? cOffS[lv] : __ldg(d.c.cOff + vb0 + lv); };
   // A term in the CTA's copy and (for a walk's fallback) in memory.
   auto term = [&](double* loc, double* glob, int i, double v) {
     loc[i] = v;
@@ -311,7 +313,7 @@ __global__ void __launch_bounds__(kPcg64T, 1) k_pcg64(const __grid_constant__ Ar
     if (d.hasContact) {
       // the shares of the owned vertices' contact records, one record per thread
       const Contact& c = d.c;
-      for (uint32_t q = cOffS[0] + threadIdx.x, q1 = cOffS[nOwn]; q < q1; q += T) {
+      for (uint32_t q = cOff(0) + threadIdx.x, q1 = cOff(nOwn); q < q1; q += T) {
         const uint32_t rec = c.cRec[q];
         const double cv = __ldcg(P.curv + (rec >> 2));
         double o[3] = {0, 0, 0};
@@ -329,7 +331,7 @@ __global__ void __launch_bounds__(kPcg64T, 1) k_pcg64(const __grid_constant__ Ar
       // A vertex may sit in hundreds of contacts: a warp sums its shares in order,
       // 32 records loaded together, one lane per component (into t2, free until the update).
       for (int lv = warp; lv < nOwn; lv += W) {
-        const uint32_t q0 = cOffS[lv], q1 = cOffS[lv + 1];
+        const uint32_t q0 = cOff(lv), q1 = cOff(lv + 1);
         if (q1 - q0 <= kLight) continue;
         const int lane = threadIdx.x & 31;
         const double* src = d.c.recScratch + (size_t)q0 * 3;
@@ -371,7 +373,7 @@ __global__ void __launch_bounds__(kPcg64T, 1) k_pcg64(const __grid_constant__ Ar
       if (!on || sg) continue;
       double ch[3] = {0, 0, 0};
       if (d.hasContact) {
-        const uint32_t q0 = cOffS[lv], cnt = cOffS[lv + 1] - q0;
+        const uint32_t q0 = cOff(lv), cnt = cOff(lv + 1) - q0;
         if (cnt > kLight) {
 #pragma unroll
           for (int c = 0; c < 3; c++) ch[c] = t2[lv * 3 + c];
@@ -690,9 +692,15 @@ void build_pcg64_plan(const HostMesh& me, int sms, int clusterMax, bool lists, P
   const size_t walk = 2 * (size_t)p.NS * (sizeof(OrdStage) + sizeof(OrdStep));
   const size_t vec = 9 * (size_t)terms * 8, elem = p.elemStride * 8;
   const size_t offs = ((size_t)(p.nv + 1) * 4 + 15) & ~(size_t)15;
-  p.vecSmem = walk + offs + vec <= kMaxDyn;
-  p.elemSmem = walk + offs + (p.vecSmem ? vec : 0) + elem <= kMaxDyn;
-  p.smem = walk + offs + (p.vecSmem ? vec : 0) + (p.elemSmem ? elem : 0);
+  p.smem = walk;
+  auto fits = [&](size_t bytes) {
+    if (p.smem + bytes > kMaxDyn) return 0;
+    p.smem += bytes;
+    return 1;
+  };
+  p.offSmem = fits(offs);  // up to about 6.7 million vertices
+  p.vecSmem = fits(vec);
+  p.elemSmem = fits(elem);
 }
 
 int launch_pcg64(const Dev& d, const Pcg64Plan& p, int maxIters, double tol, cudaStream_t s) {

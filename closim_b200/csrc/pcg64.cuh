@@ -22,7 +22,8 @@ struct Pcg64Plan {
   int R = 1;         // segments (ordering warps) per CTA
   int K = 1;         // terms per lane of a segment (odd: conflict-free shared reads)
   int NS = 0;        // G * R segments
-  int vecSmem = 0, elemSmem = 0;  // whether the CTA's vectors / element results fit in shared memory
+  int offSmem = 0, vecSmem = 0, elemSmem = 0;  // whether the CTA's contact-record offsets / vectors / element
+                                               // results fit in shared memory
   size_t smem = 0;
   size_t elemStride = 0;          // element results per CTA (doubles)
   const int* slotOff = nullptr;   // G + 1

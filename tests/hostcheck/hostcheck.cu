@@ -5,6 +5,7 @@
 #include "../../closim_b200/csrc/adjoint_math.cuh"
 #include "../../closim_b200/csrc/div_rn.cuh"
 #include "../../closim_b200/csrc/ordered_sum.cuh"
+#include "../../closim_b200/csrc/pcg64.cu"
 
 __global__ void __launch_bounds__(1024) k_hc_ordered(const double* t, int n, double* o) {
   __shared__ cs::OrdSmem<32> os;
@@ -73,6 +74,17 @@ double hc_ordered_maps(const double* t, int n, double rel, int* covered) {
 }
 void hc_div_rn(const double* a, const double* b, int n, double* o) {
   for (int i = 0; i < n; i++) o[i] = cs::div_rn_divisor(b[i]) && cs::div_rn_dividend(a[i]) ? cs::div_rn_fast(a[i], b[i], 1.0 / b[i]) : NAN;
+}
+// Shared memory of the FP64 solve's launch for n vertices (no triangles) on a device
+// with 148 SMs and clusters of 16; parts: 1 offsets, 2 vectors, 4 element results kept there.
+int64_t hc_pcg64_smem(int n, int* parts) {
+  cs::HostMesh me;
+  me.n = n;
+  me.memOff.assign((size_t)n + 1, 0u);
+  cs::Pcg64Host h;
+  cs::build_pcg64_plan(me, 148, 16, true, h);
+  *parts = h.p.offSmem | (h.p.vecSmem << 1) | (h.p.elemSmem << 2);
+  return (int64_t)h.p.smem;
 }
 // The block-wide ordered sum on the GPU; returns a cudaError_t.
 int hc_gpu_ordered_sum(const double* t, int n, double* out) {

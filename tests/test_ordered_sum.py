@@ -23,6 +23,7 @@ def hc():
     L.hc_ordered_maps.argtypes = [PTR, C.c_int, C.c_double, C.POINTER(C.c_int)]
     L.hc_gpu_ordered_sum.argtypes = [PTR, C.c_int, PTR]
     L.hc_div_rn.argtypes = [PTR, PTR, C.c_int, PTR]
+    L.hc_pcg64_smem.restype = C.c_int64
     return L
 
 
@@ -88,6 +89,18 @@ def test_division(hc):
     said = ~np.isnan(out)  # the range it answers for
     assert said[:-6].all() and said[-6] and not said[-5:].any()
     assert np.array_equal(out[said], want[said])
+
+
+@pytest.mark.parametrize("n,parts", [
+    (1, 7), (4096, 7), (4097, 7), (120000, 7), (150000, 5), (6000000, 5), (6710000, 5), (6800000, 4),
+    (7000000, 4), (30000000, 4),
+])
+def test_solve_fits_shared_memory_at_any_size(hc, n, parts):
+    """The launch never asks for more than a CTA may take (227 KB less the kernel's
+    static 22 KB): what does not fit stays in global memory."""
+    kept = C.c_int(0)
+    assert 0 < hc.hc_pcg64_smem(n, C.byref(kept)) <= (227 - 22) * 1024
+    assert kept.value == parts
 
 
 @pytest.mark.gpu
