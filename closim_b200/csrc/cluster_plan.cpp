@@ -8,6 +8,45 @@
 
 namespace cs {
 
+namespace {
+
+// A set of ids below `n` that empties itself in ascending order: marking is one
+// bit, and a CTA's ids lie close together, so the scan is short.
+struct IdSet {
+  std::vector<uint64_t> words;
+  size_t lo, hi;
+  explicit IdSet(int n) : words((size_t)n / 64 + 1, 0), lo(words.size()), hi(0) {}
+  void add(int id) {
+    const size_t w = (size_t)id >> 6;
+    words[w] |= 1ull << (id & 63);
+    lo = std::min(lo, w);
+    hi = std::max(hi, w + 1);
+  }
+  void drain(std::vector<int>& out) {
+    out.clear();
+    for (size_t w = lo; w < hi; w++) {
+      for (uint64_t b = words[w]; b; b &= b - 1) out.push_back((int)(w * 64 + (size_t)__builtin_ctzll(b)));
+      words[w] = 0;
+    }
+    lo = words.size();
+    hi = 0;
+  }
+};
+
+int range_begin(int n, int nrank, int r) { return (int)((int64_t)r * n / nrank); }
+
+}  // namespace
+
+size_t cluster_plan_least_smem(const HostMesh& me, int nrank, bool hinges) {
+  size_t least = 0;
+  for (int r = 0; r < nrank; r++) {
+    const int v0 = range_begin(me.n, nrank, r), v1 = range_begin(me.n, nrank, r + 1);
+    const int ti = (int)(me.memOff[v1] - me.memOff[v0]), hi = hinges ? (int)(me.hinOff[v1] - me.hinOff[v0]) : 0;
+    least = std::max(least, (size_t)cl_smem_layout(v1 - v0, ti / 3, hi / 4, ti + hi, v1 - v0, 0, hinges).total);
+  }
+  return least;
+}
+
 void build_cluster_plan(const HostMesh& me, int nrank, int warpsPerCta, ClusterPlanHost& p, bool domains,
                         bool hinges) {
   p = ClusterPlanHost{};
@@ -32,35 +71,30 @@ void build_cluster_plan(const HostMesh& me, int nrank, int warpsPerCta, ClusterP
   for (int v = 0; domains && v < n; v++)
     if (p.vDst[v] < 0) { p.ok = false; return; }
   p.vb.resize(nrank + 1);
-  for (int r = 0; r <= nrank; r++) p.vb[r] = (int)((int64_t)r * n / nrank);
+  for (int r = 0; r <= nrank; r++) p.vb[r] = range_begin(n, nrank, r);
   p.haloOff.assign(1, 0);
   p.triOff.assign(1, 0);
   p.hinOff.assign(1, 0);
   p.incOff.assign(n + 1, 0);
   p.incHin.assign(n, 0);
   p.ownHalo.assign(n, 0);
+  p.inc.reserve(me.memRec.size() + (hinges ? me.hinRec.size() : 0));
   std::vector<int> loc(n, -1), tslot(me.m, -1), hslot(me.hg, -1);
   std::vector<int> tris, hins, halo;
+  IdSet triSet(me.m), hinSet(me.hg), haloSet(n);
   for (int r = 0; r < nrank; r++) {
     const int v0 = p.vb[r], v1 = p.vb[r + 1];
-    tris.clear();
-    hins.clear();
-    halo.clear();
-    for (int v = v0; v < v1; v++) {
-      halo.push_back(v);
-      for (uint32_t q = me.memOff[v]; q < me.memOff[v + 1]; q++) tris.push_back((int)(me.memRec[q] >> 2));
-      for (uint32_t q = me.hinOff[v]; hinges && q < me.hinOff[v + 1]; q++) hins.push_back((int)(me.hinRec[q] >> 2));
-    }
-    std::sort(tris.begin(), tris.end());
-    tris.erase(std::unique(tris.begin(), tris.end()), tris.end());
-    std::sort(hins.begin(), hins.end());
-    hins.erase(std::unique(hins.begin(), hins.end()), hins.end());
+    for (int v = v0; v < v1; v++) haloSet.add(v);
+    for (uint32_t q = me.memOff[v0]; q < me.memOff[v1]; q++) triSet.add((int)(me.memRec[q] >> 2));
+    if (hinges)
+      for (uint32_t q = me.hinOff[v0]; q < me.hinOff[v1]; q++) hinSet.add((int)(me.hinRec[q] >> 2));
+    triSet.drain(tris);
+    hinSet.drain(hins);
     for (int t : tris)
-      for (int c = 0; c < 3; c++) halo.push_back((int)me.idx[3 * (size_t)t + c]);
+      for (int c = 0; c < 3; c++) haloSet.add((int)me.idx[3 * (size_t)t + c]);
     for (int h : hins)
-      for (int c = 0; c < 4; c++) halo.push_back(me.hinge[4 * (size_t)h + c]);
-    std::sort(halo.begin(), halo.end());
-    halo.erase(std::unique(halo.begin(), halo.end()), halo.end());
+      for (int c = 0; c < 4; c++) haloSet.add(me.hinge[4 * (size_t)h + c]);
+    haloSet.drain(halo);
     if (halo.size() > 65535) p.ok = false;
     for (size_t i = 0; i < halo.size(); i++) loc[halo[i]] = (int)i;
     for (size_t s = 0; s < tris.size(); s++) {

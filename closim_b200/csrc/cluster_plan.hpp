@@ -94,5 +94,10 @@ struct ClusterPlanHost {
 // sheet whose exact mode solves elsewhere), a smaller halo.
 void build_cluster_plan(const HostMesh& me, int nrank, int warpsPerCta, ClusterPlanHost& p, bool domains = true,
                         bool hinges = true);
+// The least dynamic shared memory of the largest CTA that any plan of these ranges
+// needs, from the incidence counts alone (a list holds at least a third of its
+// triangle incidences, a quarter of its hinge incidences): when it is over the
+// limit there is nothing to build.
+size_t cluster_plan_least_smem(const HostMesh& me, int nrank, bool hinges);
 
 }  // namespace cs

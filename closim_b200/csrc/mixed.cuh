@@ -76,6 +76,7 @@ int mx_launch_pcg_cluster(const Dev& d, const MixBufs& mb, const ClPlan& plan, f
 // cluster's shared memory (mixed_cluster.cu): one CTA per rank of the plan, part
 // 8 x kMxGridMax doubles.
 constexpr int kMxGridMax = 256;
+constexpr int kMxGridMaxDyn = 227 * 1024 - 17 * 1024;  // dynamic shared memory beside the kernel's static one
 bool mx_grid_ok(int ctas, size_t smemBytes);
 int mx_launch_pcg_grid(const Dev& d, const MixBufs& mb, const ClPlan& plan, float* pA, float* pB, double* coef,
                        double* part, int maxIters, double tol, int ctas, cudaStream_t s);

@@ -1364,14 +1364,13 @@ __global__ void __launch_bounds__(kClT, 1) k_mx_pcg_grid(GridArgs GA) {
 }
 
 bool mx_grid_ok(int ctas, size_t smemBytes) {
-  constexpr int kMaxDyn = 227 * 1024 - 17 * 1024;  // beside the kernel's static shared memory
-  if (ctas < 1 || ctas > kMxGridMax || smemBytes > (size_t)kMaxDyn) return false;
+  if (ctas < 1 || ctas > kMxGridMax || smemBytes > (size_t)kMxGridMaxDyn) return false;
   int dev = 0, sms = 0, per = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   // the largest the kernel may take: one limit for every mesh of the process
-  const bool ok = cudaFuncSetAttribute(k_mx_pcg_grid, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDyn) ==
-                      cudaSuccess &&
+  const bool ok = cudaFuncSetAttribute(k_mx_pcg_grid, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       kMxGridMaxDyn) == cudaSuccess &&
                   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_mx_pcg_grid, kClT, smemBytes) == cudaSuccess &&
                   per * sms >= ctas;
   cudaGetLastError();

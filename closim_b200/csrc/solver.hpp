@@ -744,6 +744,7 @@ class Solver {
     cl.plan = ClPlan{};
     const char* env = std::getenv("CLOSIM_MX_RESIDENT");
     if (env && std::string(env) == "0") return;
+    if (cluster_plan_least_smem(mesh, mxCluster, false) > (size_t)kClMaxDynSmem) return;
     build_cluster_plan(mesh, mxCluster, kClWarps, cl.host);
     if (!cl.host.ok) return;
     // the shared memory left over holds contact records (up to 8192 per CTA)
@@ -775,6 +776,7 @@ class Solver {
     CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
     const int ctas = std::min(std::min(sms, kMxGridMax), (mesh.n + 31) / 32);
     // without a cluster (past 20,000 vertices) exact mode solves in FP64
+    if (cluster_plan_least_smem(mesh, ctas, mxCluster > 0) > (size_t)kMxGridMaxDyn) return;
     build_cluster_plan(mesh, ctas, kClWarps, grl.host, false, mxCluster > 0);
     const size_t most = mxCluster > 0 ? grl.host.smemHinge : grl.host.smemNoHinge;
     if (!grl.host.ok || !mx_grid_ok(ctas, most)) return;

@@ -8,14 +8,38 @@
 #include "../../closim_b200/csrc/cluster_plan.hpp"
 #include "../../closim_b200/csrc/setup.hpp"
 
-extern "C" int pc_check(int n, int m, int hg, const uint32_t* idx, const int* hinge, const float* rest, int nrank,
-                        int64_t* info) {
-  // info: smem without / with hinges, ok, halo, triangle and hinge list sizes, domains
-  cs::HostMesh me;
+static void fill(cs::HostMesh& me, int n, int m, int hg, const uint32_t* idx, const int* hinge) {
   me.n = n; me.m = m; me.hg = hg;
   me.idx.assign(idx, idx + 3 * (size_t)m);
   me.hinge.assign(hinge, hinge + 4 * (size_t)hg);
   cs::build_topology(me);
+}
+
+// The counted lower bound of the lists' shared memory and what the built lists
+// (without domains) need, without and with hinges. Returns 1 when a list is not
+// strictly ascending.
+extern "C" int pc_least(int n, int m, int hg, const uint32_t* idx, const int* hinge, int nrank, int64_t* info) {
+  cs::HostMesh me;
+  fill(me, n, m, hg, idx, hinge);
+  for (int h = 0; h < 2; h++) {
+    cs::ClusterPlanHost p;
+    cs::build_cluster_plan(me, nrank, 16, p, false, h == 1);
+    info[2 * h] = (int64_t)cs::cluster_plan_least_smem(me, nrank, h == 1);
+    info[2 * h + 1] = (int64_t)(h ? p.smemHinge : p.smemNoHinge);
+    const std::vector<int>* lists[3][2] = {{&p.triOff, &p.triId}, {&p.hinOff, &p.hinId}, {&p.haloOff, &p.halo}};
+    for (auto& l : lists)
+      for (int r = 0; r < nrank; r++)
+        for (int i = (*l[0])[r] + 1; i < (*l[0])[r + 1]; i++)
+          if ((*l[1])[i] <= (*l[1])[i - 1]) return 1;
+  }
+  return 0;
+}
+
+extern "C" int pc_check(int n, int m, int hg, const uint32_t* idx, const int* hinge, const float* rest, int nrank,
+                        int64_t* info) {
+  // info: smem without / with hinges, ok, halo, triangle and hinge list sizes, domains
+  cs::HostMesh me;
+  fill(me, n, m, hg, idx, hinge);
   me.rest.assign(rest, rest + 3 * (size_t)n);
   cs::build_schwarz(me, 8, 1);
   cs::ClusterPlanHost p;

@@ -84,3 +84,21 @@ def test_plan_more_ctas_than_vertices(lib):
     cfg = configs.floor_drape(nx=2, ny=2, w=0.1, hgt=0.1, steps=2)
     rc, info = check(lib, scene_mesh(cfg), 16)
     assert rc == 0, rc
+
+
+@pytest.mark.parametrize("nx,ny,nrank,fits", [
+    (63, 63, 16, True), (99, 84, 16, True), (134, 108, 16, False),  # one cluster (its domains aside)
+    (134, 108, 148, True), (255, 255, 148, True), (419, 419, 148, False), (1050, 3, 100, True),
+])
+def test_counted_bound_of_the_lists(lib, nx, ny, nrank, fits):
+    """The bound that spares building lists which cannot fit is one: never above
+    what the built lists need, and above the limit where they are far from fitting."""
+    mesh = scene_mesh(configs.floor_drape(nx=nx, ny=ny, w=0.0127 * nx, hgt=0.0127 * ny))
+    idx = np.ascontiguousarray(mesh.indices, dtype=np.uint32)
+    hin = np.ascontiguousarray(np.asarray(mesh.hinges, dtype=np.int32).reshape(-1))
+    info = np.zeros(4, dtype=np.int64)
+    rc = lib.pc_least(len(mesh.restPositions) // 3, len(idx) // 3, len(hin) // 4, idx.ctypes.data_as(ctypes.c_void_p),
+                      hin.ctypes.data_as(ctypes.c_void_p), nrank, info.ctypes.data_as(ctypes.c_void_p))
+    assert rc == 0
+    assert 0 < info[0] <= info[1] and 0 < info[2] <= info[3] and info[0] <= info[2]
+    assert (info[0] <= SMEM_LIMIT) == fits, info
