@@ -37,27 +37,36 @@ struct Range {
 
 constexpr int kParts = 12;  // up to three sums of four ranks
 
-// The CTAs that step one sheet: a thread-block cluster of `size` (1: one block).
-// `first` and `stride` spread a loop over all their threads.
+// The threads that step one sheet: a thread-block cluster (CL) or one block, which
+// may reproduce the reductions of a cluster of VIRT blocks. The shape is part of the
+// type: with the stride and the barriers known at compile time 148 sheets of 38
+// vertices a side take 19.85 ms a step instead of 20.3.
+// `first` and `stride` spread a loop over all the threads.
+template <int T, bool CL, int VIRT>
 struct Group {
-  int size, rank, first, stride;
-  int virt;                 // 1, or the cluster size whose reductions a lone block reproduces
-  double* sm;               // block reduction scratch (32)
+  static_assert(VIRT == 1 || VIRT == 2 || VIRT == 4, "the shares turn by one place");
+  static constexpr bool kCluster = CL;
+  static constexpr int kVirt = VIRT;
+  int size, rank;
+  double* sm;                  // block reduction scratch (32)
   double (*part)[kParts][32];  // warp partials, two banks in turn
-  double (*bank)[3][8];     // the CTAs' partials, two banks in turn
+  double (*bank)[3][8];        // the CTAs' partials, two banks in turn
   int turn;
+  __device__ __forceinline__ int first() const { return CL ? rank * T + (int)threadIdx.x : (int)threadIdx.x; }
+  __device__ __forceinline__ int stride() const { return CL ? size * T : T; }
 };
 // Barrier over the group; what its threads wrote before is visible after.
-__device__ __forceinline__ void gsync(const Group& G) {
-  if (G.size > 1) cg::this_cluster().sync();
+template <class GR>
+__device__ __forceinline__ void gsync(const GR& G) {
+  if constexpr (GR::kCluster) cg::this_cluster().sync();
   else __syncthreads();
 }
 // The CTAs' values of a block reduction: each is pushed into every peer's bank,
 // one cluster barrier, then all read their own bank. A bank is written again only
 // after the next call's barrier, which no CTA passes before it has read.
-template <class F>
-__device__ __forceinline__ double gcombine(Group& G, double v, const F& op) {
-  if (G.size == 1) return v;
+template <class GR, class F>
+__device__ __forceinline__ double gcombine(GR& G, double v, const F& op) {
+  if constexpr (!GR::kCluster) return v;
   cg::cluster_group cl = cg::this_cluster();
   double* mine = G.bank[G.turn & 1][0];
   if ((int)threadIdx.x < G.size) cl.map_shared_rank(mine, threadIdx.x)[G.rank] = v;
@@ -67,46 +76,91 @@ __device__ __forceinline__ double gcombine(Group& G, double v, const F& op) {
   G.turn++;
   return r;
 }
-// Sums over the group of what `share(first, stride, s)` leaves in s[0..K) for the
-// threads that start at `first` and step by `stride`, with one block barrier (and
-// one cluster barrier): warp trees, every warp (of a cluster: warp 0) adds the
-// warps' partials with the same tree, and the CTAs' totals are added in rank
-// order. A lone block that stands in for a cluster (virt > 1) evaluates each
-// rank's share and tree in turn, so it gets the cluster's bits. Also a barrier for
-// what the group's threads wrote before.
-template <int K, class F>
-__device__ __forceinline__ void gsums(double (&out)[K], Group& G, const F& share) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  const int turn = G.turn & 1;
-  for (int r = 0; r < G.virt; r++) {
-    double v[K];
+// A thread's part of the sums of gsums: v[r][k] belongs to rank r of the cluster
+// that a lone block stands in for (a rank of a real one has only its own, v[0]).
+template <int K, int VIRT>
+struct Shares {
+  double v[VIRT][K];
+};
+// f(i, s) adds item i's terms to s for the thread's items of [i0, i1). Rank r of a
+// cluster takes the items first + (r + j * VIRT) * stride, so a lone block that
+// stands in for it walks all items in memory order and gives each in turn to the
+// next rank's share: unrolled by VIRT in the short passes of the PCG (UNROLL), by
+// turning the shares one place an item in the long ones, whose code would outgrow
+// the instruction cache. 512 sheets of 16 to 128 vertices a side, ms a step on a B200: 387
+// with a pass per rank, 386 turning everywhere, 387 unrolled everywhere, 384
+// this way; 381 with one share and no clusters at all.
+template <bool UNROLL = false, int K, class GR, class F>
+__device__ __forceinline__ void geach(const GR& G, Shares<K, GR::kVirt>& S, int i0, int i1, const F& f) {
+  constexpr int V = GR::kVirt;
+  if constexpr (UNROLL && V > 1) {
+    for (int i = i0 + G.first(); i < i1; i += V * G.stride()) {
 #pragma unroll
-    for (int k = 0; k < K; k++) v[k] = 0;
-    share(G.first + r * (int)blockDim.x, G.stride * G.virt, v);
+      for (int r = 0; r < V; r++)
+        if (r == 0 || i + r * G.stride() < i1) f(i + r * G.stride(), S.v[r]);
+    }
+    return;
+  }
+  auto turn = [&]() {
 #pragma unroll
     for (int k = 0; k < K; k++) {
+      const double t = S.v[0][k];
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_down_sync(0xffffffffu, v[k], o);
-      if (lane == 0) G.part[turn][r * K + k][warp] = v[k];
+      for (int r = 1; r < V; r++) S.v[r - 1][k] = S.v[r][k];
+      S.v[V - 1][k] = t;
+    }
+  };
+  int place = 0;
+  for (int i = i0 + G.first(); i < i1; i += G.stride()) {
+    f(i, S.v[0]);
+    if constexpr (V > 1) {
+      turn();
+      place++;
     }
   }
-  G.turn++;
-  __syncthreads();
-  if (G.size == 1) {
+  if constexpr (V > 1)
+    for (; place & (V - 1); place++) turn();
+}
+// Sums over the group of the terms that `share(S)` leaves in S (by geach), with one
+// block barrier (and one cluster barrier): warp trees, every warp (of a cluster:
+// warp 0) adds the warps' partials with the same tree, and the CTAs' totals are
+// added in rank order. A lone block that stands in for a cluster (virt > 1) does so
+// with each rank's shares, so it gets the cluster's bits. Also a barrier for
+// what the group's threads wrote before.
+template <int K, class GR, class F>
+__device__ __forceinline__ void gsums(double (&out)[K], GR& G, const F& share) {
+  constexpr int V = GR::kVirt;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const int turn = G.turn & 1;
+  Shares<K, V> S;
+#pragma unroll
+  for (int r = 0; r < V; r++)
+#pragma unroll
+    for (int k = 0; k < K; k++) S.v[r][k] = 0;
+  share(S);
+#pragma unroll
+  for (int r = 0; r < V; r++)
 #pragma unroll
     for (int k = 0; k < K; k++) {
-      double w[4];
 #pragma unroll
-      for (int r = 0; r < 4; r++) w[r] = r < G.virt && lane < nw ? G.part[turn][r * K + k][lane] : 0.0;
+      for (int o = 16; o > 0; o >>= 1) S.v[r][k] += __shfl_down_sync(0xffffffffu, S.v[r][k], o);
+      if (lane == 0) G.part[turn][r * K + k][warp] = S.v[r][k];
+    }
+  G.turn++;
+  __syncthreads();
+  if constexpr (!GR::kCluster) {
+#pragma unroll
+    for (int k = 0; k < K; k++) {
+      double w[V];
+#pragma unroll
+      for (int r = 0; r < V; r++) w[r] = lane < nw ? G.part[turn][r * K + k][lane] : 0.0;
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1)
 #pragma unroll
-        for (int r = 0; r < 4; r++)
-          if (r < G.virt) w[r] += __shfl_down_sync(0xffffffffu, w[r], o);
+        for (int r = 0; r < V; r++) w[r] += __shfl_down_sync(0xffffffffu, w[r], o);
       double t = w[0];
 #pragma unroll
-      for (int r = 1; r < 4; r++)
-        if (r < G.virt) t += w[r];
+      for (int r = 1; r < V; r++) t += w[r];
       out[k] = __shfl_sync(0xffffffffu, t, 0);
     }
     return;
@@ -131,10 +185,12 @@ __device__ __forceinline__ void gsums(double (&out)[K], Group& G, const F& share
   }
 }
 
-__device__ __forceinline__ double gmax(double v, Group& G) {
+template <class GR>
+__device__ __forceinline__ double gmax(double v, GR& G) {
   return gcombine(G, block_max(v, G.sm), [](double a, double b) { return js_max(a, b); });
 }
-__device__ __forceinline__ double gmin(double v, Group& G) {
+template <class GR>
+__device__ __forceinline__ double gmin(double v, GR& G) {
   return gcombine(G, block_min(v, G.sm), [](double a, double b) { return fmin(a, b); });
 }
 
@@ -142,8 +198,9 @@ __device__ __forceinline__ void ld3b(const double* x, int v, double o[3]) {
   o[0] = x[v * 3]; o[1] = x[v * 3 + 1]; o[2] = x[v * 3 + 2];
 }
 
-__device__ __forceinline__ void enforce_pins(const BatchDev& b, const Range& R, const Group& G, double* x) {
-  for (int v = R.v0 + G.first; v < R.v1; v += G.stride)
+template <class GR>
+__device__ __forceinline__ void enforce_pins(const BatchDev& b, const Range& R, const GR& G, double* x) {
+  for (int v = R.v0 + G.first(); v < R.v1; v += G.stride())
     if (b.pinned[v])
       for (int k = 0; k < 3; k++) x[v * 3 + k] = b.pinPos[v * 3 + k];
 }
@@ -151,11 +208,12 @@ __device__ __forceinline__ void enforce_pins(const BatchDev& b, const Range& R, 
 // checkTrial restricted to the floor (contact-assembly.ts:489-553): the
 // smallest floor distance must exceed dMin and no vertex may cross the dMin
 // level during x0 -> xT.
-__device__ bool floor_trial_ok(const BatchDev& b, const Range& R, const double* xT, Group& G) {
+template <class GR>
+__device__ bool floor_trial_ok(const BatchDev& b, const Range& R, const double* xT, GR& G) {
   if (!b.hasFloor) return true;
   double mn = INFINITY;
   int bad = 0;
-  for (int v = R.v0 + G.first; v < R.v1; v += G.stride) {
+  for (int v = R.v0 + G.first(); v < R.v1; v += G.stride()) {
     const double yT = xT[v * 3 + 1] - b.floorY;
     if (yT < mn || yT != yT) mn = yT != yT ? -INFINITY : yT;
     const double y0 = b.x0[v * 3 + 1] - b.floorY;
@@ -170,18 +228,20 @@ __device__ bool floor_trial_ok(const BatchDev& b, const Range& R, const double* 
   return !(m <= b.dMin) && anyBad == 0;
 }
 
-__device__ __forceinline__ void update_active(const BatchDev& b, const Range& R, const Group& G, const double* x) {
-  for (int v = R.v0 + G.first; v < R.v1; v += G.stride)
+template <class GR>
+__device__ __forceinline__ void update_active(const BatchDev& b, const Range& R, const GR& G, const double* x) {
+  for (int v = R.v0 + G.first(); v < R.v1; v += G.stride())
     b.act[v] = b.hasFloor && (x[v * 3 + 1] - b.floorY < b.dHat) ? 1 : 0;
 }
 
 // totalEnergy (newton.ts:76-88): inertia + membrane + bending + barrier merit.
+template <class GR>
 __device__ double sheet_energy(const BatchDev& b, const Range& R, const double* x, const Mat<double>& mt, double kb,
-                               Group& G) {
+                               GR& G) {
   double out[1];
-  gsums<1>(out, G, [&](int first, int stride, double (&s)[1]) {
-    double e = 0;
-    for (int v = R.v0 + first; v < R.v1; v += stride) {
+  gsums<1>(out, G, [&](Shares<1, GR::kVirt>& S) {
+    geach(G, S, R.v0, R.v1, [&](int v, double (&s)[1]) {
+      double e = s[0];
       const double M = b.mass[v];
       for (int k = 0; k < 3; k++) {
         const double d = x[v * 3 + k] - b.yHat[v * 3 + k];
@@ -191,29 +251,30 @@ __device__ double sheet_energy(const BatchDev& b, const Range& R, const double* 
         const double d = fmax(x[v * 3 + 1] - b.floorY, 1e-12);
         if (d < b.dHat) e += b.kappa * barrier_value(d, b.dHat);
       }
-    }
-    for (int t = R.t0 + first; t < R.t1; t += stride) {
+      s[0] = e;
+    });
+    geach(G, S, R.t0, R.t1, [&](int t, double (&s)[1]) {
       double p0[3], p1[3], p2[3];
       ld3b(x, b.idx[t * 3], p0); ld3b(x, b.idx[t * 3 + 1], p1); ld3b(x, b.idx[t * 3 + 2], p2);
       const float4 iv = b.inv[t];
-      e += tri_energy<double>(p0, p1, p2, iv.x, iv.y, iv.z, iv.w, b.area[t], mt);
-    }
+      s[0] += tri_energy<double>(p0, p1, p2, iv.x, iv.y, iv.z, iv.w, b.area[t], mt);
+    });
     if (kb > 0)
-      for (int hh = R.h0 + first; hh < R.h1; hh += stride) {
+      geach(G, S, R.h0, R.h1, [&](int hh, double (&s)[1]) {
         const int4 hv = b.hinge[hh];
         double q[12], gdum[12];
         ld3b(x, hv.x, q); ld3b(x, hv.y, q + 3); ld3b(x, hv.z, q + 6); ld3b(x, hv.w, q + 9);
-        e += bend_grad<double>(q, b.hmeta[hh * 3], b.hmeta[hh * 3 + 1], b.hmeta[hh * 3 + 2], kb, gdum);
-      }
-    s[0] = e;
+        s[0] += bend_grad<double>(q, b.hmeta[hh * 3], b.hmeta[hh * 3 + 1], b.hmeta[hh * 3 + 2], kb, gdum);
+      });
   });
   return out[0];
 }
 
 // Newton gradient at b.x into b.g (filtered), the barrier curvature added to
 // the diagonal estimate; returns |g|.
-__device__ double sheet_gradient(const BatchDev& b, const Range& R, const Mat<double>& mt, double kb, Group& G) {
-  for (int t = R.t0 + G.first; t < R.t1; t += G.stride) {
+template <class GR>
+__device__ double sheet_gradient(const BatchDev& b, const Range& R, const Mat<double>& mt, double kb, GR& G) {
+  for (int t = R.t0 + G.first(); t < R.t1; t += G.stride()) {
     double p0[3], p1[3], p2[3];
     ld3b(b.x, b.idx[t * 3], p0); ld3b(b.x, b.idx[t * 3 + 1], p1); ld3b(b.x, b.idx[t * 3 + 2], p2);
     const float4 iv = b.inv[t];
@@ -222,7 +283,7 @@ __device__ double sheet_gradient(const BatchDev& b, const Range& R, const Mat<do
     for (int k = 0; k < 9; k++) b.elem[(size_t)t * 9 + k] = gg[k];
   }
   if (kb > 0)
-    for (int hh = R.h0 + G.first; hh < R.h1; hh += G.stride) {
+    for (int hh = R.h0 + G.first(); hh < R.h1; hh += G.stride()) {
       const int4 hv = b.hinge[hh];
       double q[12], gg[12];
       ld3b(b.x, hv.x, q); ld3b(b.x, hv.y, q + 3); ld3b(b.x, hv.z, q + 6); ld3b(b.x, hv.w, q + 9);
@@ -231,9 +292,8 @@ __device__ double sheet_gradient(const BatchDev& b, const Range& R, const Mat<do
     }
   gsync(G);
   double out[1];
-  gsums<1>(out, G, [&](int first, int stride, double (&sum)[1]) {
-    double gn = 0;
-    for (int v = R.v0 + first; v < R.v1; v += stride) {
+  gsums<1>(out, G, [&](Shares<1, GR::kVirt>& S) {
+    geach(G, S, R.v0, R.v1, [&](int v, double (&sum)[1]) {
       double s[3] = {0, 0, 0};
       for (uint32_t q = b.memOff[v]; q < b.memOff[v + 1]; q++) {
         const uint32_t rec = b.memRec[q];
@@ -266,17 +326,17 @@ __device__ double sheet_gradient(const BatchDev& b, const Range& R, const Mat<do
         double gi = M * (b.x[i] - b.yHat[i]) * b.invH2 + s[k];
         if (pin) gi = 0;
         b.g[i] = gi;
-        gn += gi * gi;
+        sum[0] += gi * gi;
       }
-    }
-    sum[0] = gn;
+    });
   });
   return sqrt(out[0]);
 }
 
 // FP32 state of every triangle for the matrix-free HVP (F, S, Dm^-1, s).
-__device__ void sheet_tristate(const BatchDev& b, const Range& R, const Group& G, const Mat<double>& m) {
-  for (int t = R.t0 + G.first; t < R.t1; t += G.stride) {
+template <class GR>
+__device__ void sheet_tristate(const BatchDev& b, const Range& R, const GR& G, const Mat<double>& m) {
+  for (int t = R.t0 + G.first(); t < R.t1; t += G.stride()) {
     double x0[3], x1[3], x2[3];
     ld3b(b.x, b.idx[t * 3], x0); ld3b(b.x, b.idx[t * 3 + 1], x1); ld3b(b.x, b.idx[t * 3 + 2], x2);
     const float4 iv = b.inv[t];
@@ -304,13 +364,13 @@ __device__ void sheet_tristate(const BatchDev& b, const Range& R, const Group& G
 // vertex adds the corner share of its incident triangles' HVP directly
 // (recomputed per corner from the stored FP32 state), so no per-triangle
 // result is written and read back and no barrier splits the product.
+template <class GR>
 __device__ double sheet_hvp(const BatchDev& b, const Range& R, float C00, float C11, float C01, float Gs,
-                            Group& G) {
+                            GR& G) {
   const float invH2 = (float)b.invH2;
   double out[1];
-  gsums<1>(out, G, [&](int first, int stride, double (&s)[1]) {
-    double pAp = 0;
-    for (int v = R.v0 + first; v < R.v1; v += stride) {
+  gsums<1>(out, G, [&](Shares<1, GR::kVirt>& S) {
+    geach<true>(G, S, R.v0, R.v1, [&](int v, double (&s)[1]) {
       float sp[3] = {0.f, 0.f, 0.f};
       for (uint32_t q = b.memOff[v]; q < b.memOff[v + 1]; q++) {
         const uint32_t rec = __ldg(b.memRec + q);
@@ -337,37 +397,35 @@ __device__ double sheet_hvp(const BatchDev& b, const Range& R, float C00, float 
         float ap = M * b.p[i] * invH2 + sp[q] + (q == 1 ? cy : 0.f);
         if (pin) ap = 0.f;
         b.Ap[i] = ap;
-        pAp += (double)b.p[i] * ap;
+        s[0] += (double)b.p[i] * ap;
       }
-    }
-    s[0] = pAp;
+    });
   });
   return out[0];
 }
 
 // pcg.ts:11-95 (Jacobi, tolerance 1e-3) and the newton.ts:152-179 epilogue;
 // the direction lands in b.dx. Returns the PCG iteration count.
-__device__ int sheet_pcg(const BatchDev& b, const Range& R, float C00, float C11, float C01, float Gs, Group& G,
+template <class GR>
+__device__ int sheet_pcg(const BatchDev& b, const Range& R, float C00, float C11, float C01, float Gs, GR& G,
                          double& gtdxOut) {
   double s3[3];
-  gsums<3>(s3, G, [&](int first, int stride, double (&s)[3]) {
-    double bb = 0, rr = 0, rz = 0;
-    for (int i = 3 * R.v0 + first; i < 3 * R.v1; i += stride) {
+  gsums<3>(s3, G, [&](Shares<3, GR::kVirt>& S) {
+    geach<true>(G, S, 3 * R.v0, 3 * R.v1, [&](int i, double (&s)[3]) {
       const double bi = -b.g[i];
-      bb += bi * bi;
+      s[0] += bi * bi;
       const bool pin = b.pinned[i / 3];
       const float ri = pin ? 0.f : (float)bi;
       b.r[i] = ri;
       b.xs[i] = 0.f;
-      rr += (double)ri * ri;
+      s[1] += (double)ri * ri;
       const float di = pin ? 0.f : b.diag[i] > 1e-12 ? (float)(1.0 / b.diag[i]) : 1.f;
       b.dinv[i] = di;
       const float zi = ri * di;
       b.z[i] = zi;
       b.p[i] = zi;
-      rz += (double)ri * zi;
-    }
-    s[0] = bb; s[1] = rr; s[2] = rz;
+      s[2] += (double)ri * zi;
+    });
   });
   const double bNorm = sqrt(s3[0]);
   double residual = sqrt(s3[1]), rz = s3[2];
@@ -380,60 +438,54 @@ __device__ int sheet_pcg(const BatchDev& b, const Range& R, float C00, float C11
     if (!(pAp > 1e-30)) { iters = k; done = true; break; }
     const float alpha = (float)(rz / pAp);
     double s2[2];
-    gsums<2>(s2, G, [&](int first, int stride, double (&s)[2]) {
-      double rrn = 0, rzn = 0;
-      for (int i = 3 * R.v0 + first; i < 3 * R.v1; i += stride) {
+    gsums<2>(s2, G, [&](Shares<2, GR::kVirt>& S) {
+      geach<true>(G, S, 3 * R.v0, 3 * R.v1, [&](int i, double (&s)[2]) {
         const bool pin = b.pinned[i / 3];
         float xi = b.xs[i] + alpha * b.p[i];
         float ri = b.r[i] - alpha * b.Ap[i];
         if (pin) { xi = 0.f; ri = 0.f; }
         b.xs[i] = xi;
         b.r[i] = ri;
-        rrn += (double)ri * ri;
+        s[0] += (double)ri * ri;
         const float zi = ri * b.dinv[i];
         b.z[i] = zi;
-        rzn += (double)ri * zi;
-      }
-      s[0] = rrn; s[1] = rzn;
+        s[1] += (double)ri * zi;
+      });
     });
     residual = sqrt(s2[0]);
     const double rzn = s2[1];
     if (residual < absTol) { iters = k + 1; done = true; break; }
     const float beta = (float)(rzn / rz);
     rz = rzn;
-    for (int i = 3 * R.v0 + G.first; i < 3 * R.v1; i += G.stride) b.p[i] = b.z[i] + beta * b.p[i];
+    for (int i = 3 * R.v0 + G.first(); i < 3 * R.v1; i += G.stride()) b.p[i] = b.z[i] + beta * b.p[i];
     gsync(G);
   }
   if (!done) iters = b.pcgMaxIters;
   double s1[1];
-  gsums<1>(s1, G, [&](int first, int stride, double (&s)[1]) {
-    double gt = 0;
-    for (int i = 3 * R.v0 + first; i < 3 * R.v1; i += stride) {
+  gsums<1>(s1, G, [&](Shares<1, GR::kVirt>& S) {
+    geach<true>(G, S, 3 * R.v0, 3 * R.v1, [&](int i, double (&s)[1]) {
       const double di = b.xs[i];
       b.dx[i] = di;
-      gt += b.g[i] * di;
-    }
-    s[0] = gt;
+      s[0] += b.g[i] * di;
+    });
   });
   double gtdx = s1[0];
   if (!isfinite(gtdx) || gtdx >= 0) {
-    gsums<1>(s1, G, [&](int first, int stride, double (&s)[1]) {
-      double gt = 0;
-      for (int i = 3 * R.v0 + first; i < 3 * R.v1; i += stride) {
+    gsums<1>(s1, G, [&](Shares<1, GR::kVirt>& S) {
+      geach<true>(G, S, 3 * R.v0, 3 * R.v1, [&](int i, double (&s)[1]) {
         const double di = -b.g[i] / b.diag[i];
         b.dx[i] = di;
-        gt += b.g[i] * di;
-      }
-      s[0] = gt;
+        s[0] += b.g[i] * di;
+      });
     });
     gtdx = s1[0];
   }
   double mx = 0;
-  for (int i = 3 * R.v0 + G.first; i < 3 * R.v1; i += G.stride) mx = fmax(mx, fabs(b.dx[i]));
+  for (int i = 3 * R.v0 + G.first(); i < 3 * R.v1; i += G.stride()) mx = fmax(mx, fabs(b.dx[i]));
   const double maxDx = gmax(mx, G);
   if (maxDx > 0.002) {
     const double sc = 0.002 / maxDx;
-    for (int i = 3 * R.v0 + G.first; i < 3 * R.v1; i += G.stride) b.dx[i] *= sc;
+    for (int i = 3 * R.v0 + G.first(); i < 3 * R.v1; i += G.stride()) b.dx[i] *= sc;
     gtdx *= sc;
     gsync(G);
   }
@@ -441,7 +493,8 @@ __device__ int sheet_pcg(const BatchDev& b, const Range& R, float C00, float C11
   return iters;
 }
 
-__device__ void step_sheet(const BatchDev& b, int s, Group& G) {
+template <class GR>
+__device__ void step_sheet(const BatchDev& b, int s, GR& G) {
   const Range R{b.vStart[s], b.vStart[s + 1], b.tStart[s], b.tStart[s + 1], b.hStart[s], b.hStart[s + 1]};
   const double* mr = b.mat + (size_t)s * BM_N;
   const Mat<double> mt{mr[BM_C00], mr[BM_C11], mr[BM_C01], mr[BM_G], mr[BM_THICK]};
@@ -449,7 +502,7 @@ __device__ void step_sheet(const BatchDev& b, int s, Group& G) {
   const float C00 = (float)mr[BM_C00], C11 = (float)mr[BM_C11], C01 = (float)mr[BM_C01], Gs = (float)mr[BM_G];
   const double h = b.h;
   // predictor y_hat = x + h v + h^2 g, initial guess y_hat with pins (newton.ts:40-51)
-  for (int v = R.v0 + G.first; v < R.v1; v += G.stride)
+  for (int v = R.v0 + G.first(); v < R.v1; v += G.stride())
     for (int k = 0; k < 3; k++) {
       const int i = v * 3 + k;
       const double xv = b.x[i];
@@ -467,7 +520,7 @@ __device__ void step_sheet(const BatchDev& b, int s, Group& G) {
     double lo = 0, hi = 1;
     for (int it = 0; it < 8; it++) {
       const double mid = 0.5 * (lo + hi);
-      for (int i = 3 * R.v0 + G.first; i < 3 * R.v1; i += G.stride) b.xt[i] = b.x0[i] + mid * (b.x[i] - b.x0[i]);
+      for (int i = 3 * R.v0 + G.first(); i < 3 * R.v1; i += G.stride()) b.xt[i] = b.x0[i] + mid * (b.x[i] - b.x0[i]);
       gsync(G);
       enforce_pins(b, R, G, b.xt);
       gsync(G);
@@ -475,7 +528,7 @@ __device__ void step_sheet(const BatchDev& b, int s, Group& G) {
       else hi = mid;
       if (hi - lo < 1e-4) break;
     }
-    for (int i = 3 * R.v0 + G.first; i < 3 * R.v1; i += G.stride) b.x[i] = b.x0[i] + lo * (b.x[i] - b.x0[i]);
+    for (int i = 3 * R.v0 + G.first(); i < 3 * R.v1; i += G.stride()) b.x[i] = b.x0[i] + lo * (b.x[i] - b.x0[i]);
     gsync(G);
     enforce_pins(b, R, G, b.x);
     gsync(G);
@@ -483,7 +536,7 @@ __device__ void step_sheet(const BatchDev& b, int s, Group& G) {
   update_active(b, R, G, b.x);
   gsync(G);
   double energy = sheet_energy(b, R, b.x, mt, kb, G);
-  for (int v = R.v0 + G.first; v < R.v1; v += G.stride) {
+  for (int v = R.v0 + G.first(); v < R.v1; v += G.stride()) {
     const double d0 = b.mass[v] * b.invH2 + beta;
     b.diag[v * 3] = d0; b.diag[v * 3 + 1] = d0; b.diag[v * 3 + 2] = d0;
   }
@@ -505,7 +558,7 @@ __device__ void step_sheet(const BatchDev& b, int s, Group& G) {
     bool accepted = false;
     for (int li = 0; li < b.lsIters; li++) {
       trials++;
-      for (int i = 3 * R.v0 + G.first; i < 3 * R.v1; i += G.stride) b.xt[i] = b.x[i] + alpha * b.dx[i];
+      for (int i = 3 * R.v0 + G.first(); i < 3 * R.v1; i += G.stride()) b.xt[i] = b.x[i] + alpha * b.dx[i];
       gsync(G);
       enforce_pins(b, R, G, b.xt);
       gsync(G);
@@ -513,12 +566,12 @@ __device__ void step_sheet(const BatchDev& b, int s, Group& G) {
       const double eNew = sheet_energy(b, R, b.xt, mt, kb, G);
       if (!isfinite(eNew)) { rejected++; alpha *= 0.5; continue; }
       if (eNew <= energy + 1e-4 * alpha * gtdx) {
-        for (int i = 3 * R.v0 + G.first; i < 3 * R.v1; i += G.stride) b.x[i] = b.xt[i];
+        for (int i = 3 * R.v0 + G.first(); i < 3 * R.v1; i += G.stride()) b.x[i] = b.xt[i];
         energy = eNew;
         accepted = true;
         gsync(G);
         // commit: lagged normal force of every active floor contact (contact-assembly.ts:475-485)
-        for (int v = R.v0 + G.first; v < R.v1; v += G.stride)
+        for (int v = R.v0 + G.first(); v < R.v1; v += G.stride())
           if (b.act[v]) {
             const double d = fmax(b.x[v * 3 + 1] - b.floorY, 1e-12);
             if (d < b.dHat) { b.lagLam[v] = barrier_normal_force(d, b.dHat, b.kappa, 1); b.lagOk[v] = 1; }
@@ -532,19 +585,19 @@ __device__ void step_sheet(const BatchDev& b, int s, Group& G) {
     if (!accepted || alpha < 1e-6) break;
   }
   // velocity update, restitution-0 on floor contacts (newton.ts:222-245)
-  for (int i = 3 * R.v0 + G.first; i < 3 * R.v1; i += G.stride) b.v[i] = ((b.x[i] - b.x0[i]) / h) * damp;
+  for (int i = 3 * R.v0 + G.first(); i < 3 * R.v1; i += G.stride()) b.v[i] = ((b.x[i] - b.x0[i]) / h) * damp;
   gsync(G);
   update_active(b, R, G, b.x);
   gsync(G);
-  int nfloor = 0;
-  for (int v = R.v0 + G.first; v < R.v1; v += G.stride)
-    if (b.act[v]) {
-      nfloor++;
-      if (b.v[v * 3 + 1] < 0) b.v[v * 3 + 1] = 0;
-    }
-  enforce_pins(b, R, G, b.x);
   double nf[1];
-  gsums<1>(nf, G, [&](int, int, double (&t)[1]) { t[0] += nfloor; nfloor = 0; });
+  gsums<1>(nf, G, [&](Shares<1, GR::kVirt>& S) {
+    geach(G, S, R.v0, R.v1, [&](int v, double (&s)[1]) {
+      if (!b.act[v]) return;
+      s[0] += 1;
+      if (b.v[v * 3 + 1] < 0) b.v[v * 3 + 1] = 0;
+    });
+  });
+  enforce_pins(b, R, G, b.x);
   if (G.rank == 0 && threadIdx.x == 0) {
     double* o = b.out + (size_t)s * BO_N;
     o[BO_NEWTON] = used;
@@ -559,15 +612,16 @@ __device__ void step_sheet(const BatchDev& b, int s, Group& G) {
   gsync(G);
 }
 
-template <int T>
-__global__ void __launch_bounds__(T, 1) k_batch_step(BatchDev b, const int* order, int count, unsigned int* work,
-                                                     int size, int virt) {
+// 512 threads an SM at the least: 128 registers a thread.
+template <int T, bool CL, int VIRT>
+__global__ void __launch_bounds__(T, 512 / T) k_batch_step(BatchDev b, const int* order, int count, unsigned int* work,
+                                                     int size) {
   __shared__ double sm[32];
   __shared__ double part[2][kParts][32];
   __shared__ double bank[2][3][8];
   __shared__ int sheetSh;
-  const int rank = size > 1 ? (int)cg::this_cluster().block_rank() : 0;
-  Group G{size, rank, rank * T + (int)threadIdx.x, size * T, virt, sm, part, bank, 0};
+  const int rank = CL ? (int)cg::this_cluster().block_rank() : 0;
+  Group<T, CL, VIRT> G{size, rank, sm, part, bank, 0};
   // Shared memory of a peer may be touched once every CTA of the cluster has
   // started, which co-scheduling alone does not promise.
   gsync(G);
@@ -576,7 +630,8 @@ __global__ void __launch_bounds__(T, 1) k_batch_step(BatchDev b, const int* orde
       const unsigned k = atomicAdd(work, 1u);
       const int sheet = k < (unsigned)count ? order[k] : -1;
       sheetSh = sheet;
-      for (int q = 1; q < size; q++) *cg::this_cluster().map_shared_rank(&sheetSh, q) = sheet;
+      if constexpr (CL)
+        for (int q = 1; q < size; q++) *cg::this_cluster().map_shared_rank(&sheetSh, q) = sheet;
     }
     gsync(G);
     const int sheet = sheetSh;
@@ -586,21 +641,29 @@ __global__ void __launch_bounds__(T, 1) k_batch_step(BatchDev b, const int* orde
   }
 }
 
-template <int T>
-int launch_t(const BatchDev& b, const int* order, int count, unsigned int* work, int size, int virt, int ctas,
-             cudaStream_t s) {
-  cudaLaunchConfig_t cfg = {};
+void launch_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* attr, int threads, int size, int ctas) {
   cfg.gridDim = dim3(ctas);
-  cfg.blockDim = dim3(T);
-  cfg.stream = s;
-  cudaLaunchAttribute attr[1];
+  cfg.blockDim = dim3(threads);
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = size;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = size > 1 ? 1 : 0;
-  return (int)cudaLaunchKernelEx(&cfg, k_batch_step<T>, b, order, count, work, size, virt);
+}
+
+template <int T>
+int launch_t(const BatchDev& b, const int* order, int count, unsigned int* work, int size, int virt, int ctas,
+             cudaStream_t s) {
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  launch_config(cfg, attr, T, size, ctas);
+  cfg.stream = s;
+  auto* kernel = size > 1    ? k_batch_step<T, true, 1>
+                 : virt == 4 ? k_batch_step<T, false, 4>
+                 : virt == 2 ? k_batch_step<T, false, 2>
+                             : k_batch_step<T, false, 1>;
+  return (int)cudaLaunchKernelEx(&cfg, kernel, b, order, count, work, size);
 }
 
 }  // namespace
@@ -610,9 +673,9 @@ int batch_max_ctas(int threads) {
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   cudaError_t e = cudaSuccess;
-  if (threads == 128) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_batch_step<128>, 128, 0);
-  else if (threads == 256) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_batch_step<256>, 256, 0);
-  else e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_batch_step<512>, 512, 0);
+  if (threads == 128) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_batch_step<128, false, 1>, 128, 0);
+  else if (threads == 256) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_batch_step<256, false, 1>, 256, 0);
+  else e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_batch_step<512, false, 1>, 512, 0);
   if (e != cudaSuccess || per < 1) per = 1;
   return per * sms;
 }
