@@ -224,13 +224,6 @@ def step_algorithmic_bytes(st, mesh, precision, cfg):
     return float(b)
 
 
-def pcg_kernel_name(precision, prof):
-    if precision != "mixed":
-        return "k_pcg64"
-    info = prof.get("launch_info") or {}
-    return "k_mx_pcg_cluster" if info.get("pcgClusterCtas") else "k_mx_pcg"
-
-
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) of one launch of
 # the PCG kernel on the 64 x 64 floor drape, from one ncu capture of that kernel
 # on that workload (not measured by this run; reported as traffic_from_profile).
@@ -584,7 +577,7 @@ def main():
         peak, peak_kind = measured_peak()
         achieved = prof["bytes"] / prof["launches"] / (prof["ms_per_launch"] / 1000.0) / 1e9 if prof.get("launches") \
             else 0.0
-        kname = pcg_kernel_name("mixed", prof)
+        kname = prof["launch_info"]["pcgKernel"]
         n_h2d = 2 * n * 3 * 8
         line = {
             "metric": "sim steps/s", "value": value, "unit": "steps/s", "n_gpus": world, "steps": args.steps,

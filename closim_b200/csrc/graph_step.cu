@@ -387,7 +387,7 @@ const int* Solver::contact_free_valid() {
 bool Solver::step_graph(double h) {
   if (!graphMode || !mixed() || mxCluster <= 0 || prof || profPhases) return false;
   // the grid-wide PCG is a cooperative launch, which cannot be in a captured step
-  if (grid_pcg(newtonMode == 1 && d.kb > 0 && d.hg > 0)) return false;
+  if (pcg_kernel() != PCG_MX_CLUSTER) return false;
   if (!gstep) gstep = new GraphStep();
   GraphStep& G = *gstep;
   if (G.failed) return false;

@@ -268,9 +268,11 @@ int cs_solver_info(cs_solver* h, int32_t* out, int32_t n) {
   return guarded(h, [&] {
     if (!out || n <= 0) throw std::invalid_argument("null output");
     const auto& S = h->s;
-    const int32_t v[6] = {S.mxGrid > 0 && !S.clRes[0] ? 0 : S.mxCluster, S.mxGrid > 0 ? S.mxGrid : S.mxBlocks, S.pcg.p.G, S.mesh.D,
-                          S.clRes[0] ? (int32_t)S.clSmem[0] : 0, S.clRes[1] ? (int32_t)S.clSmem[1] : 0};
-    for (int i = 0; i < n; i++) out[i] = i < 6 ? v[i] : 0;
+    const cs::PcgKernel k = S.pcg_kernel();
+    const int32_t v[7] = {k == cs::PCG_MX_GRID ? 0 : S.mxCluster, k == cs::PCG_MX_GRID ? S.mxGrid : S.mxBlocks,
+                          S.pcg.p.G, S.mesh.D, S.clRes[0] ? (int32_t)S.clSmem[0] : 0,
+                          S.clRes[1] ? (int32_t)S.clSmem[1] : 0, (int32_t)k};
+    for (int i = 0; i < n; i++) out[i] = i < 7 ? v[i] : 0;
   });
 }
 

@@ -74,6 +74,9 @@ struct AdjStats {
 enum Phase { PH_OTHER = 0, PH_BROADPHASE, PH_ACTIVE_SET, PH_GRADIENT, PH_PRECOND, PH_PCG, PH_TRIAL, PH_ENERGY,
              PH_COMMIT, PH_N };
 
+// Kernels of the linear solve (cs_solver_info's codes).
+enum PcgKernel { PCG_FP64 = 0, PCG_FP64_EXACT, PCG_MX_CLUSTER, PCG_MX_GRID, PCG_MX };
+
 class Solver {
  public:
   int precision = CS_PRECISION_FP64;
@@ -539,23 +542,24 @@ class Solver {
       }
       phase(PH_PCG);
       if (prof) CK(cudaEventRecord(pev0, stream));
-      if (newtonMode == 1 && !exactMixed) {
+      const PcgKernel solve = pcg_kernel();
+      if (solve == PCG_FP64_EXACT) {
         ensure_adj_buffers();
         AdjArgs a{d, adjRhs.p, d.dx, adjR.p, adjZ.p, adjP.p, adjAp.p, adjTri.p, adjHin.p, adjDom.p, d.kb, 1,
                   opts.pcg_max_iters, newtonTol, adjOut.p};
         CK((cudaError_t)newton_exact_solve(a, adj_grid_blocks(d), stream));
         lc += 3;
-      } else if (mixed() && grid_pcg(mb.hrec != nullptr)) {
+      } else if (solve == PCG_MX_GRID) {
         ClPlan plan = grl.plan;
         plan.smemBytes = (int)mxGridSmem[mb.hrec ? 1 : 0];
         CK((cudaError_t)mx_launch_pcg_grid(d, mb, plan, fp.p, fp2.p, d.hasContact ? d.c.dd : nullptr, mxGridPart.p,
                                            opts.pcg_max_iters,
                                            exactMixed ? std::max(newtonTol, kMixedTolFloor) : 1e-3, mxGrid, stream));
-      } else if (mixed() && mxCluster > 0)
+      } else if (solve == PCG_MX_CLUSTER)
         CK((cudaError_t)mx_launch_pcg_cluster(d, mb, cluster_plan_for(mb), fp.p, fp2.p, d.hasContact ? d.c.dd : nullptr,
                                               opts.pcg_max_iters, exactMixed ? std::max(newtonTol, kMixedTolFloor) : 1e-3,
                                               mxCluster, stream));
-      else if (mixed()) CK((cudaError_t)mx_launch_pcg(d, mb, opts.pcg_max_iters, 1e-3, mxBlocks, stream));
+      else if (solve == PCG_MX) CK((cudaError_t)mx_launch_pcg(d, mb, opts.pcg_max_iters, 1e-3, mxBlocks, stream));
       else {
         pcg.p.curv = contact ? contact->dd : nullptr;
         CK((cudaError_t)launch_pcg64(d, pcg.p, opts.pcg_max_iters, 1e-3, stream));
@@ -791,6 +795,13 @@ class Solver {
   // cluster's do not fit in this mode (hinges: with the bending term), or the
   // preconditioner is Jacobi, which the resident cluster kernel does not have.
   bool grid_pcg(bool hinges) const { return mxGrid > 0 && !(clRes[hinges ? 1 : 0] && precond_code() >= 1); }
+  // The kernel the linear solve runs with the current mode and options.
+  PcgKernel pcg_kernel() const {
+    if (!mixed()) return newtonMode == 1 ? PCG_FP64_EXACT : PCG_FP64;
+    if (newtonMode == 1 && mxCluster <= 0) return PCG_FP64_EXACT;
+    if (grid_pcg(newtonMode == 1 && d.kb > 0 && d.hg > 0)) return PCG_MX_GRID;
+    return mxCluster > 0 ? PCG_MX_CLUSTER : PCG_MX;
+  }
   // The plan for a launch: resident when this launch's lists fit.
   ClPlan cluster_plan_for(const MixBufs& m) const {
     ClPlan p = cl.plan;

@@ -447,11 +447,14 @@ class CudaSolver:
         return dict(pcgIters=int(out[0]), solves=int(out[1]), recomputedSteps=int(out[2]), maxRelResidual=out[3],
                     forwardConverged=int(out[4]))
 
+    PCG_KERNELS = ("k_pcg64", "k_adj_pcg", "k_mx_pcg_cluster", "k_mx_pcg_grid", "k_mx_pcg")
+
     def launchInfo(self) -> dict:
-        out = np.zeros(6, np.int32)
+        out = np.zeros(7, np.int32)
         self._check(self._lib.cs_solver_info(self._h, L.ptr(out), len(out)))
-        return dict(pcgClusterCtas=int(out[0]), pcgGridCtas=int(out[1]), fp64PcgCtas=int(out[2]),
-                    schwarzDomains=int(out[3]), residentSmem=int(out[4]), residentSmemExact=int(out[5]))
+        return dict(pcgKernel=self.PCG_KERNELS[out[6]], pcgClusterCtas=int(out[0]), pcgGridCtas=int(out[1]),
+                    fp64PcgCtas=int(out[2]), schwarzDomains=int(out[3]), residentSmem=int(out[4]),
+                    residentSmemExact=int(out[5]))
 
     def profilePhases(self) -> dict:
         out = np.zeros(len(self.PHASES))

@@ -190,12 +190,13 @@ int cs_profile_read(cs_solver* s, double* out5);
  * accumulated per phase since cs_profile: other, broadphase, active set,
  * gradient, preconditioner, PCG, trial check, trial energy, commit. */
 int cs_profile_phases(cs_solver* s, double* out, int32_t n);
-/* Launch shapes chosen at cs_initialize (diagnostic): out[0] CTAs of the
- * one-cluster mixed PCG (0 = the grid-wide kernel is used), out[1] CTAs of the
- * grid-wide mixed PCG, out[2] CTAs of the FP64 PCG, out[3] Schwarz domains,
- * out[4] / out[5] dynamic shared memory per CTA (bytes) of the one-cluster
- * PCG's resident element lists without / with the Gauss-Newton bending term
- * (0 = they do not fit and the kernel gathers from global memory). */
+/* Launch shapes of the linear solve with the current Newton mode, material and
+ * options (diagnostic): out[0] CTAs of the one-cluster mixed PCG (0 = a grid-wide
+ * kernel is used), out[1] CTAs of the grid-wide mixed PCG, out[2] CTAs of the FP64
+ * PCG, out[3] Schwarz domains, out[4] / out[5] dynamic shared memory per CTA
+ * (bytes) of the one-cluster PCG's resident element lists without / with the
+ * Gauss-Newton bending term (0 = they do not fit), out[6] the kernel:
+ * 0 k_pcg64, 1 k_adj_pcg, 2 k_mx_pcg_cluster, 3 k_mx_pcg_grid, 4 k_mx_pcg. */
 int cs_solver_info(cs_solver* s, int32_t* out, int32_t n);
 
 /* ---- SimulationSession.doStep hand-off (src/view/sim-session.ts:132-150) ----

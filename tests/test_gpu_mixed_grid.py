@@ -6,7 +6,8 @@ Every vertex and element does the same FP32 operations in the same order; only
 the FP64 dot products are summed in another order, which moves an FP32 alpha or
 beta by an ulp when their ratio lies within 1e-16 of a rounding boundary, about
 once in 1e8 iterations. So one step at the reference budget agrees to 1e-9 of
-the positions' size, and a converged step to what gradTol leaves."""
+the positions' size, and a converged step to what gradTol leaves. Also which
+kernel a solver says it runs."""
 import numpy as np
 import pytest
 
@@ -47,7 +48,31 @@ def test_grid_pcg_matches_the_kernels_it_replaces(monkeypatch, nx, ny, precond, 
     opts = dict(newtonIters=30, pcgMaxIters=2000, gradTol=1e-9) if mode == "exact" else {}
     x1, st1, info = one_step(monkeypatch, True, cfg, mode, **opts)
     x0, st0, old = one_step(monkeypatch, False, cfg, mode, **opts)
-    assert info["pcgGridCtas"] <= 148 and old["pcgGridCtas"] != info["pcgGridCtas"]
+    assert info["pcgKernel"] == "k_mx_pcg_grid"
+    assert old["pcgKernel"] == ("k_mx_pcg_cluster" if (nx + 1) * (ny + 1) <= 20000 else "k_mx_pcg")
     assert st1.contact["floorPairs"] > 0
     assert st1.newtonItersUsed == st0.newtonItersUsed and st1.pcgIters == st0.pcgIters
     assert np.max(np.abs(x1 - x0)) <= 1e-9 * np.max(np.abs(x0))
+
+
+@pytest.mark.parametrize("precision,nx,ny,precond,mode,kernel", [
+    ("mixed", 63, 63, "schwarz", "exact", "k_mx_pcg_cluster"),
+    ("mixed", 69, 69, "schwarz", "reference", "k_mx_pcg_cluster"),  # the lists fit one cluster without the hinges,
+    ("mixed", 69, 69, "schwarz", "exact", "k_mx_pcg_grid"),         # with them they do not
+    ("mixed", 69, 69, "jacobi", "reference", "k_mx_pcg_grid"),      # the resident cluster kernel has no Jacobi
+    ("mixed", 39, 39, "jacobi", "reference", "k_mx_pcg_cluster"),
+    ("mixed", 150, 140, "schwarz", "reference", "k_mx_pcg_grid"),
+    ("mixed", 150, 140, "schwarz", "exact", "k_adj_pcg"),
+    ("fp64", 20, 20, "schwarz", "reference", "k_pcg64"),
+    ("fp64", 20, 20, "schwarz", "exact", "k_adj_pcg"),
+])
+def test_launch_info_names_the_kernel(precision, nx, ny, precond, mode, kernel):
+    cfg = configs.floor_drape(nx=nx, ny=ny, w=0.0127 * nx, hgt=0.0127 * ny, precond=precond)
+    s = cb.CudaSolver(precision, **cfg["options"])
+    s.initialize(configs.make_scene(cfg))
+    s.setNewtonMode(mode, 3e-4)
+    info = s.launchInfo()
+    s.close()
+    assert info["pcgKernel"] == kernel
+    if precision == "mixed" and kernel != "k_adj_pcg":
+        assert (info["pcgClusterCtas"] > 0) == (kernel == "k_mx_pcg_cluster")
