@@ -55,6 +55,30 @@ def test_grid_pcg_matches_the_kernels_it_replaces(monkeypatch, nx, ny, precond, 
     assert np.max(np.abs(x1 - x0)) <= 1e-9 * np.max(np.abs(x0))
 
 
+@pytest.mark.parametrize("mode", ["reference", "exact"])
+def test_grid_pcg_with_many_contacts_per_vertex(monkeypatch, mode):
+    """A sheet sliding over the pole of a finely divided sphere, where 64 edges
+    meet: vertices with more than four contact records, which a warp sums. That
+    there are some follows from the counts: the records (one per vertex-triangle
+    pair at the least, two per edge-edge pair) outnumber four for every vertex
+    within reach of the sphere. (A converged exact step lifts the sheet off again, so
+    that one stops after two Newton iterations.)"""
+    cell = 0.003
+    cfg = configs.sphere_drape(nx=84, ny=79, w=84 * cell, hgt=79 * cell, radius=0.1, drop=0.1004, segments=64, rings=32)
+    cfg["contact"]["dHatM"] = 1e-3
+    cfg["v"][0::3] = 0.2
+    cfg["v"][1::3] = -0.05
+    opts = dict(newtonIters=2, pcgMaxIters=2000, gradTol=1e-9) if mode == "exact" else {}
+    x1, st1, info = one_step(monkeypatch, True, cfg, mode, **opts)
+    x0, st0, old = one_step(monkeypatch, False, cfg, mode, **opts)
+    assert info["pcgKernel"] == "k_mx_pcg_grid" and old["pcgKernel"] == "k_mx_pcg_cluster"
+    far = np.linalg.norm(cfg["x"].reshape(-1, 3) - np.asarray(cfg["sphere"]["centre"]), axis=1) - 0.1
+    near = int(np.count_nonzero(far < 1e-3 + 3 * cell))
+    assert st1.contact["vtPairs"] + 2 * st1.contact["eePairs"] > 4 * near > 0
+    assert st1.newtonItersUsed == st0.newtonItersUsed and st1.pcgIters == st0.pcgIters
+    assert np.max(np.abs(x1 - x0)) <= 1e-9 * np.max(np.abs(x0))
+
+
 @pytest.mark.parametrize("precision,nx,ny,precond,mode,kernel", [
     ("mixed", 63, 63, "schwarz", "exact", "k_mx_pcg_cluster"),
     ("mixed", 69, 69, "schwarz", "reference", "k_mx_pcg_cluster"),  # the lists fit one cluster without the hinges,
