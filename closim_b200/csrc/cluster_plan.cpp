@@ -78,7 +78,8 @@ void build_cluster_plan(const HostMesh& me, int nrank, int warpsPerCta, ClusterP
   p.incOff.assign(n + 1, 0);
   p.incHin.assign(n, 0);
   p.ownHalo.assign(n, 0);
-  p.inc.reserve(me.memRec.size() + (hinges ? me.hinRec.size() : 0));
+  p.inc.resize(me.memRec.size() + (hinges ? me.hinRec.size() : 0));
+  int nextInc = 0;
   std::vector<int> loc(n, -1), tslot(me.m, -1), hslot(me.hg, -1);
   std::vector<int> tris, hins, halo;
   IdSet triSet(me.m), hinSet(me.hg), haloSet(n);
@@ -97,32 +98,35 @@ void build_cluster_plan(const HostMesh& me, int nrank, int warpsPerCta, ClusterP
     haloSet.drain(halo);
     if (halo.size() > 65535) p.ok = false;
     for (size_t i = 0; i < halo.size(); i++) loc[halo[i]] = (int)i;
-    for (size_t s = 0; s < tris.size(); s++) {
+    p.triLoc.resize(p.triLoc.size() + 4 * tris.size(), 0);
+    uint16_t* tl = p.triLoc.data() + p.triLoc.size() - 4 * tris.size();
+    for (size_t s = 0; s < tris.size(); s++, tl += 4) {
       const int t = tris[s];
       tslot[t] = (int)s;
-      for (int c = 0; c < 3; c++) p.triLoc.push_back((uint16_t)loc[me.idx[3 * (size_t)t + c]]);
-      p.triLoc.push_back(0);
+      for (int c = 0; c < 3; c++) tl[c] = (uint16_t)loc[me.idx[3 * (size_t)t + c]];
     }
-    for (size_t s = 0; s < hins.size(); s++) {
+    p.hinLoc.resize(p.hinLoc.size() + 4 * hins.size());
+    uint16_t* hl = p.hinLoc.data() + p.hinLoc.size() - 4 * hins.size();
+    for (size_t s = 0; s < hins.size(); s++, hl += 4) {
       const int h = hins[s];
       hslot[h] = (int)s;
-      for (int c = 0; c < 4; c++) p.hinLoc.push_back((uint16_t)loc[me.hinge[4 * (size_t)h + c]]);
+      for (int c = 0; c < 4; c++) hl[c] = (uint16_t)loc[me.hinge[4 * (size_t)h + c]];
     }
-    const size_t inc0 = p.inc.size();
+    const int inc0 = nextInc;
     for (int v = v0; v < v1; v++) {
-      p.incOff[v] = (int)p.inc.size();
+      p.incOff[v] = nextInc;
       for (uint32_t q = me.memOff[v]; q < me.memOff[v + 1]; q++) {
         const uint32_t rec = me.memRec[q];
-        p.inc.push_back(((uint32_t)tslot[rec >> 2] << 2) | (rec & 3));
+        p.inc[nextInc++] = ((uint32_t)tslot[rec >> 2] << 2) | (rec & 3);
       }
-      p.incHin[v] = (int)p.inc.size();
+      p.incHin[v] = nextInc;
       for (uint32_t q = me.hinOff[v]; hinges && q < me.hinOff[v + 1]; q++) {
         const uint32_t rec = me.hinRec[q];
-        p.inc.push_back(((uint32_t)hslot[rec >> 2] << 2) | (rec & 3));
+        p.inc[nextInc++] = ((uint32_t)hslot[rec >> 2] << 2) | (rec & 3);
       }
       p.ownHalo[v] = loc[v];
     }
-    const int nInc = (int)(p.inc.size() - inc0), nOwn = v1 - v0;
+    const int nInc = nextInc - inc0, nOwn = v1 - v0;
     p.triId.insert(p.triId.end(), tris.begin(), tris.end());
     p.hinId.insert(p.hinId.end(), hins.begin(), hins.end());
     p.halo.insert(p.halo.end(), halo.begin(), halo.end());
@@ -134,7 +138,7 @@ void build_cluster_plan(const HostMesh& me, int nrank, int warpsPerCta, ClusterP
     p.smemNoHinge = std::max(p.smemNoHinge, (size_t)cl_smem_layout(nh, nt, ng, nInc, nOwn, ns, false).total);
     p.smemHinge = std::max(p.smemHinge, (size_t)cl_smem_layout(nh, nt, ng, nInc, nOwn, ns, true).total);
   }
-  p.incOff[n] = (int)p.inc.size();
+  p.incOff[n] = nextInc;
 }
 
 }  // namespace cs

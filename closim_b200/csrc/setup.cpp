@@ -168,14 +168,19 @@ void build_topology(HostMesh& me) {
 // sub-minimum domains into the smallest adjacent one, members sorted.
 void build_schwarz(HostMesh& me, int target, int minSize) {
   const int n = me.n;
-  std::vector<std::vector<int>> adj(n);
-  {
-    std::vector<std::set<int>> s(n);
-    for (int t = 0; t < me.m; t++) {
-      const int a = me.idx[t * 3], b = me.idx[t * 3 + 1], c = me.idx[t * 3 + 2];
-      s[a].insert(b); s[a].insert(c); s[b].insert(a); s[b].insert(c); s[c].insert(a); s[c].insert(b);
+  // neighbours of each vertex, ascending, from its triangle corners (memRec)
+  std::vector<int> adj, adjOff(n + 1, 0), nb;
+  adj.reserve(2 * me.memRec.size());
+  for (int v = 0; v < n; v++) {
+    nb.clear();
+    for (uint32_t q = me.memOff[v]; q < me.memOff[v + 1]; q++) {
+      const uint32_t t = me.memRec[q] >> 2, c = me.memRec[q] & 3;
+      nb.push_back((int)me.idx[t * 3 + (c + 1) % 3]);
+      nb.push_back((int)me.idx[t * 3 + (c + 2) % 3]);
     }
-    for (int v = 0; v < n; v++) adj[v].assign(s[v].begin(), s[v].end());
+    std::sort(nb.begin(), nb.end());
+    adj.insert(adj.end(), nb.begin(), std::unique(nb.begin(), nb.end()));
+    adjOff[v + 1] = (int)adj.size();
   }
   double lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
   for (int v = 0; v < n; v++)
@@ -211,7 +216,8 @@ void build_schwarz(HostMesh& me, int target, int minSize) {
     while ((int)mem[id].size() < target && !qu.empty()) {
       const int cur = qu.front();
       qu.pop_front();
-      for (int w : adj[cur]) {
+      for (int j = adjOff[cur]; j < adjOff[cur + 1]; j++) {
+        const int w = adj[j];
         if ((int)mem[id].size() >= target) break;
         if (dom[w] >= 0) continue;
         dom[w] = id;
@@ -227,14 +233,14 @@ void build_schwarz(HostMesh& me, int target, int minSize) {
       if (len > 0 && len < minSize && n >= minSize && (small < 0 || len < (int)mem[small].size())) small = d;
     }
     if (small < 0) break;
-    std::set<int> nb;
+    std::set<int> near;
     for (int t = 0; t < me.m; t++) {
       const int ds[3] = {dom[me.idx[t * 3]], dom[me.idx[t * 3 + 1]], dom[me.idx[t * 3 + 2]]};
       if (ds[0] != small && ds[1] != small && ds[2] != small) continue;
-      for (int x : ds) if (x != small) nb.insert(x);
+      for (int x : ds) if (x != small) near.insert(x);
     }
     int best = -1;
-    for (int c : nb)
+    for (int c : near)
       if (!mem[c].empty() && (best < 0 || mem[c].size() < mem[best].size())) best = c;
     if (best < 0) break;
     for (int v : mem[small]) { dom[v] = best; mem[best].push_back(v); }
