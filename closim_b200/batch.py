@@ -97,6 +97,12 @@ class BatchSolver:
         self._check(self._lib.cs_batch_launch_shape(self._h, C.byref(t), C.byref(b)))
         return dict(threads=t.value, blocks=b.value)
 
+    def launchGroups(self) -> list:
+        """Per size class: its sheets, CTAs per sheet, cluster ranks a lone block reproduces."""
+        out = np.zeros(9, np.int32)
+        self._check(self._lib.cs_batch_launch_groups(self._h, L.ptr(out)))
+        return [dict(sheets=int(a), ctas=int(b), ranks=int(c)) for a, b, c in out.reshape(3, 3)]
+
     def setThreads(self, threads: int) -> None:
         self._check(self._lib.cs_batch_set_threads(self._h, int(threads)))
 

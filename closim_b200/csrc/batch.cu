@@ -680,6 +680,23 @@ int batch_max_ctas(int threads) {
   return per * sms;
 }
 
+void batch_device(int& sms, int (&maxGroups)[kBatchClasses]) {
+  int dev = 0;
+  cudaGetDevice(&dev);
+  sms = 1;
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  for (int c = 0; c < kBatchClasses; c++) {
+    maxGroups[c] = sms;
+    if (kBatchSize[c] == 1) continue;
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    launch_config(cfg, attr, 512, kBatchSize[c], sms / kBatchSize[c] * kBatchSize[c]);
+    if (cudaOccupancyMaxActiveClusters(&maxGroups[c], k_batch_step<512, true, 1>, &cfg) != cudaSuccess)
+      maxGroups[c] = 0;
+  }
+  cudaGetLastError();
+}
+
 int batch_launch_step(const BatchDev& b, const int* order, int count, unsigned int* work, int size, int virt,
                       int threads, int ctas, cudaStream_t s) {
   if (threads == 128) return launch_t<128>(b, order, count, work, size, virt, ctas, s);

@@ -5,6 +5,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "batch_plan.hpp"
+
 namespace cs {
 
 // Per-sheet material and Newton constants (one row of 8 doubles).
@@ -52,25 +54,13 @@ struct BatchDev {
   double* out;                 // S x BO_N
 };
 
-// CTAs that step a sheet of n vertices together (a cluster). A function of the sheet
-// alone, because it fixes the shape of the sheet's reductions: its result is the same
-// in every batch. Below 1,500 vertices (three per thread) a cluster's barriers cost
-// what its SMs save. When the sheets want more than kBatchFill times the device's
-// CTAs, a cluster's barriers and its fit into a GPC cost more than the shorter tail
-// saves, and lone blocks stand in for the clusters with the same reductions.
-// Measured (B200, per step): 64 sheets of 16 to 128 vertices a side 222 -> 63 ms in
-// clusters; 512 such sheets 382 / 372 / 348 ms on their first three steps before,
-// 12% more in clusters, 395 / 388 / 362 by lone blocks.
-constexpr int kBatchClasses = 3;
-constexpr int kBatchSize[kBatchClasses] = {4, 2, 1};
-constexpr int kBatchFill = 4;
-inline int batch_class(int n) { return n > 3000 ? 0 : n > 1500 ? 1 : 2; }
-
 // Steps the `count` sheets of one size class once: persistent groups of `size` CTAs
 // take sheets from `order`, reducing as a cluster of size * virt would; work: the
 // class's counter (reset before the launch).
 int batch_launch_step(const BatchDev& b, const int* order, int count, unsigned int* work, int size, int virt,
                       int threads, int ctas, cudaStream_t s);
 int batch_max_ctas(int threads);
+// SMs of the current device and, per class, the clusters of 512-thread blocks it holds at once.
+void batch_device(int& sms, int (&maxGroups)[kBatchClasses]);
 
 }  // namespace cs

@@ -78,6 +78,7 @@ struct Batch {
   // are independent launches; all but the first go to side streams between two
   // events, so small sheets fill the SMs that the clusters leave free.
   int classStart[kBatchClasses + 1] = {0, 0, 0, 0};
+  int groupSize[kBatchClasses] = {1, 1, 1};  // CTAs per sheet (batch_route)
   cudaStream_t side[kBatchClasses] = {};
   cudaEvent_t fork = nullptr, join[kBatchClasses] = {};
   bool ready = false;
@@ -180,6 +181,11 @@ struct Batch {
     });
     for (int c = 0; c <= kBatchClasses; c++)
       classStart[c] = (int)std::count_if(ord.begin(), ord.end(), [&](int a) { return classOf(a) < c; });
+    int sms = 1, maxGroups[kBatchClasses];
+    batch_device(sms, maxGroups);
+    std::vector<int> verts[kBatchClasses];
+    for (int a : ord) verts[classOf(a)].push_back(vs[a + 1] - vs[a]);
+    batch_route(verts, sms, maxGroups, groupSize);
     cudaStream_t st = stream;
     vStart.up(vs.data(), vs.size(), st); tStart.up(ts.data(), ts.size(), st); hStart.up(hs.data(), hs.size(), st);
     order.up(ord.data(), ord.size(), st);
@@ -244,12 +250,9 @@ struct Batch {
     bind(h);
     BK(cudaMemsetAsync(work.p, 0, kBatchClasses * sizeof(unsigned int), stream));
     bool forked = false, used = false;
-    long wanted = 0;
-    for (int c = 0; c < kBatchClasses; c++) wanted += (long)(classStart[c + 1] - classStart[c]) * kBatchSize[c];
-    const bool lone = wanted > (long)kBatchFill * ctas;
     for (int c = 0; c < kBatchClasses; c++) {
       const int count = classStart[c + 1] - classStart[c];
-      const int size = lone ? 1 : kBatchSize[c], virt = lone ? kBatchSize[c] : 1;
+      const int size = groupSize[c], virt = kBatchSize[c] / size;
       if (count == 0) continue;
       cudaStream_t st = stream;
       if (used) {  // another class already runs on the main stream
@@ -484,6 +487,19 @@ int cs_batch_launch_shape(cs_batch* h, int32_t* threads, int32_t* blocks) {
   return bguard(b, [&] {
     if (threads) *threads = b->threads;
     if (blocks) *blocks = b->ctas;
+  });
+}
+
+int cs_batch_launch_groups(cs_batch* h, int32_t* out) {
+  cs::Batch* b = B(h);
+  return bguard(b, [&] {
+    if (!out) throw cs::BErr(CS_E_ARG, "null output");
+    if (!b->ready) throw cs::BErr(CS_E_UNINIT, "batch not initialized");
+    for (int c = 0; c < cs::kBatchClasses; c++) {
+      out[3 * c] = b->classStart[c + 1] - b->classStart[c];
+      out[3 * c + 1] = b->groupSize[c];
+      out[3 * c + 2] = cs::kBatchSize[c] / b->groupSize[c];
+    }
   });
 }
 

@@ -10,9 +10,11 @@
  * sheet (3 doubles per vertex). pin_counts[s] pins of sheet s take the next
  * pin_counts[s] entries of pin_ids (local ids) and pin_pos (3 doubles each).
  *
- * One step is ONE persistent kernel launch: each thread block takes a sheet
- * from a work list ordered largest first and runs that sheet's whole implicit
- * step with block barriers only. cs_batch_step with steps > 1 captures the
+ * One step is one persistent kernel launch per size class of sheets (at most
+ * three, side by side): each thread block, or cluster of two or four blocks, takes
+ * a sheet from a work list ordered largest first and runs that sheet's whole
+ * implicit step with block or cluster barriers only. A sheet's result does not depend on
+ * the rest of the batch or on which of the two steps it. cs_batch_step with steps > 1 captures the
  * sequence once into a CUDA graph and replays it. cs_batch_autotune times the
  * candidate launch shapes (128, 256 or 512 threads per block, i.e. vertices
  * per thread of a sheet; all resident blocks or a half or a third of them,
@@ -56,6 +58,10 @@ int cs_batch_autotune(cs_batch* b, double dt, int32_t* threads);
 int cs_batch_set_threads(cs_batch* b, int32_t threads);
 /* The launch shape in use: threads per block and resident blocks. */
 int cs_batch_launch_shape(cs_batch* b, int32_t* threads, int32_t* blocks);
+/* How the three size classes (over 3,000 vertices, over 1,500, the rest) are
+ * stepped: for each its sheets, the CTAs that step one sheet together, and the
+ * ranks of a cluster whose reductions a lone block reproduces (9 values). */
+int cs_batch_launch_groups(cs_batch* b, int32_t* out);
 void* cs_batch_stream(cs_batch* b);
 
 #ifdef __cplusplus

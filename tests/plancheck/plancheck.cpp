@@ -5,6 +5,7 @@
 #include <cstdint>
 #include <vector>
 
+#include "../../closim_b200/csrc/batch_plan.hpp"
 #include "../../closim_b200/csrc/cluster_plan.hpp"
 #include "../../closim_b200/csrc/setup.hpp"
 
@@ -33,6 +34,17 @@ extern "C" int pc_least(int n, int m, int hg, const uint32_t* idx, const int* hi
           if ((*l[1])[i] <= (*l[1])[i - 1]) return 1;
   }
   return 0;
+}
+
+// The batch's route for `count` sheets of verts[i] vertices: CTAs per sheet of each class.
+extern "C" void pc_batch_route(const int* verts, int count, int sms, int fours, int twos, int* size) {
+  std::vector<int> v[cs::kBatchClasses];
+  for (int i = 0; i < count; i++) v[cs::batch_class(verts[i])].push_back(verts[i]);
+  for (auto& c : v) std::sort(c.rbegin(), c.rend());
+  const int most[3] = {fours, twos, sms};
+  int s[3];
+  cs::batch_route(v, sms, most, s);
+  std::copy(s, s + 3, size);
 }
 
 extern "C" int pc_check(int n, int m, int hg, const uint32_t* idx, const int* hinge, const float* rest, int nrank,

@@ -1,4 +1,5 @@
-"""Per-CTA element lists of the one-cluster PCG's resident phase A (host logic).
+"""Per-CTA element lists of the one-cluster PCG's resident phase A, and the
+batched solver's choice between clusters and lone blocks (host logic).
 
 The builder (closim_b200/csrc/cluster_plan.cpp) is compiled for the host with
 a checker of its invariants (tests/plancheck): the owned vertex ranges cover
@@ -102,3 +103,23 @@ def test_counted_bound_of_the_lists(lib, nx, ny, nrank, fits):
     assert rc == 0
     assert 0 < info[0] <= info[1] and 0 < info[2] <= info[3] and info[0] <= info[2]
     assert (info[0] <= SMEM_LIMIT) == fits, info
+
+
+@pytest.mark.parametrize("sides,sizes", [
+    ([64] * 9, (4, 1, 1)), ([64] * 37, (4, 1, 1)), ([64] * 74, (4, 1, 1)), ([64] * 148, (1, 1, 1)),
+    ([64] * 296, (1, 1, 1)), ([80] * 74, (4, 1, 1)), ([80] * 148, (1, 1, 1)), ([55] * 37, (4, 1, 1)),
+    ([55] * 74, (1, 1, 1)), ([55] * 111, (1, 1, 1)), ([55] * 148, (1, 1, 1)), ([45] * 74, (1, 2, 1)),
+    ([45] * 111, (1, 1, 1)), ([45] * 148, (1, 1, 1)), ([38] * 400, (1, 1, 1)),
+    ([16 + i % 113 for i in range(0, 113, 2)], (4, 1, 1)), ([16 + i * 7 % 113 for i in range(512)], (1, 1, 1)),
+])
+def test_batch_route(lib, sides, sizes):
+    """Clusters or lone blocks as the measured times (batch_plan.hpp) say, on a
+    device of 148 SMs that holds 33 clusters of four and 74 of two; lone blocks
+    where no cluster fits."""
+    verts = np.array([s * s for s in sides], np.int32)
+    out = np.zeros(3, np.int32)
+    p = ctypes.c_void_p
+    lib.pc_batch_route(verts.ctypes.data_as(p), len(verts), 148, 33, 74, out.ctypes.data_as(p))
+    assert tuple(out) == sizes
+    lib.pc_batch_route(verts.ctypes.data_as(p), len(verts), 148, 0, 0, out.ctypes.data_as(p))
+    assert tuple(out) == (1, 1, 1)

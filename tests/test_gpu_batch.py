@@ -134,15 +134,24 @@ def test_batch_matches_the_oracle_exact_mode_when_converged():
         assert err <= 1e-7, err
 
 
-@pytest.mark.parametrize("side,count", [(55, 160), (39, 320), (38, 3)])
-def test_sheet_is_the_same_in_a_cluster_and_by_a_lone_block(side, count):
+@pytest.mark.parametrize("sides", [[55] * 148, [39] * 148, [55] * 148 + [39] * 148 + [38] * 20])
+def test_sheet_is_the_same_in_a_cluster_and_by_a_lone_block(sides):
     """A sheet's reductions have the shape of its size class whether a cluster
     steps it (a small batch) or a lone block does (a batch that fills the
     device): 55 x 55 and 39 x 39 are the smallest sheets of the classes of four
-    and two blocks, 38 x 38 the largest of the class of one."""
-    sheets = configs.batch_sheets(count=count, side_min=side, side_max=side)
-    full, alone = BatchSolver(sheets), BatchSolver([sheets[count // 2]])
+    and two blocks, 38 x 38 the largest of the class of one. The last batch
+    launches the three classes side by side, both ways."""
+    sheets = []
+    for i, s in enumerate(sides):
+        sheets += configs.batch_sheets(seed=i, count=1, side_min=s, side_max=s)
+    picks = [sides.index(s) + sides.count(s) // 2 for s in sorted(set(sides))]
+    full, few = BatchSolver(sheets), BatchSolver([sheets[i] for i in picks])
+    assert all(g["ctas"] == 1 for g in full.launchGroups())
+    assert [g["ctas"] for g in few.launchGroups() if g["sheets"]] == [
+        {55: 4, 39: 2, 38: 1}[s] for s in sorted(set(sides), reverse=True)]
+    assert sum(g["sheets"] for g in full.launchGroups()) == len(sides)
     full.step(0.01, steps=2)
-    alone.step(0.01, steps=2)
-    assert np.array_equal(full.positions(count // 2), alone.positions(0))
-    assert full.stats()[count // 2] == alone.stats()[0]
+    few.step(0.01, steps=2)
+    for k, i in enumerate(picks):
+        assert np.array_equal(full.positions(i), few.positions(k))
+        assert full.stats()[i] == few.stats()[k]
