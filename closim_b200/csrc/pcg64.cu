@@ -12,8 +12,9 @@
 // publishes the stages of its own range, and after a barrier every CTA walks
 // all of them. A stage needs an approximate start; those of |r|^2, r.z and
 // |p|^2 come from recurrences in alpha and beta over sums published one phase
-// earlier, so each costs one barrier. Sheets up to kPcg64ClusterN vertices run
-// in one 16-CTA cluster (hardware barrier), larger ones on the whole grid.
+// earlier, so each costs one barrier. Sheets up to kPcg64SingleN vertices run in
+// one CTA, which adds the terms one by one, sheets up to kPcg64ClusterN in one
+// 16-CTA cluster (hardware barrier), larger ones on the whole grid.
 // Whole steps on a B200 against one-thread chains on a cooperative grid: 41 x 9
 // strip (Jacobi, two steps) 43.7 -> 31.4 ms, 64 x 64 drape (Schwarz) 54.0 ->
 // 14.7 ms, 121 x 95 garment on a sphere (Jacobi) 411 -> 61 ms, the same bits. An
@@ -143,6 +144,21 @@ __device__ __noinline__ void walk(const OrdStage* h0, const OrdStage* h1, const 
   __syncthreads();
 }
 
+// n terms in order by one thread, sixteen loaded together.
+__device__ __noinline__ double serial_sum(const double* t, int n) {
+  double p = 0.0;
+  int j = 0;
+  for (; j + 16 <= n; j += 16) {
+    double a[16];
+#pragma unroll
+    for (int q = 0; q < 16; q++) a[q] = t[j + q];
+#pragma unroll
+    for (int q = 0; q < 16; q++) p = p + a[q];
+  }
+  for (; j < n; j++) p = p + t[j];
+  return p;
+}
+
 template <bool CLUSTER>
 __global__ void __launch_bounds__(kPcg64T, 1) k_pcg64(const __grid_constant__ Args A) {
   extern __shared__ __align__(16) unsigned char dyn[];
@@ -207,6 +223,13 @@ __global__ void __launch_bounds__(kPcg64T, 1) k_pcg64(const __grid_constant__ Ar
   auto walk2 = [&](int k0, int k1, const double* T0, const double* T1) {
     walk(heads(k0), heads(k1), stages(k0), stages(k1), 2, NS, T0, T1, wst, stp, res);
   };
+  // A lone CTA holds all terms: its first two warps add one sum each (ta, tb) in order.
+  const bool single = P.G == 1;
+  auto serial = [&](const double* ta, const double* tb) {
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0 && warp < (tb ? 2 : 1)) res[warp] = serial_sum(warp ? tb : ta, nt);
+    __syncthreads();
+  };
   // Warps q * R .. q * R + R - 1 order the segments of the q-th pending sum.
   auto segment = [&](int q) { return warp - q * R; };
 
@@ -258,7 +281,7 @@ __global__ void __launch_bounds__(kPcg64T, 1) k_pcg64(const __grid_constant__ Ar
   }
   __syncthreads();
   // approximate segment sums of the four initial chains
-  for (int w = warp; w < R * 4; w += W) {
+  for (int w = warp; !single && w < R * 4; w += W) {
     const int q = w / R, r = w - q * R;
     const double* t = q == 0 ? t0 : q == 1 ? t1 : q == 2 ? t2 : t3;
     const Chunk c = seg_chunk(P, r, nt);
@@ -269,18 +292,20 @@ __global__ void __launch_bounds__(kPcg64T, 1) k_pcg64(const __grid_constant__ Ar
     if ((threadIdx.x & 31) == 0) P.sums[(size_t)row * NS + b * R + r] = s;
   }
   barrier();
-  for (int w = warp; w < R * 4; w += W) {
+  for (int w = warp; !single && w < R * 4; w += W) {
     const int q = w / R, r = w - q * R;
     const double* t = q == 0 ? t0 : q == 1 ? t1 : q == 2 ? t2 : t3;
     const int row = q == 0 ? W_PAP : q == 1 ? W_RR : q == 2 ? W_RZ : W_PP;
     order(q, r, t, before(row, r));
   }
   barrier();
-  walk2(D_PAP, D_RR, d.T0, d.T1);
+  if (single) serial(t0, t1);
+  else walk2(D_PAP, D_RR, d.T0, d.T1);
   const double bNorm = sqrt(res[0]);
   double residual = sqrt(res[1]);
   __syncthreads();
-  walk2(D_RZ, D_PP, d.T2, d.T3);
+  if (single) serial(t2, t3);
+  else walk2(D_RZ, D_PP, d.T2, d.T3);
   double rz = res[0];
   double pp = res[1];
   const double absTol = js_max(A.tol * js_max(bNorm, 1e-12), 1e-12);
@@ -401,7 +426,7 @@ __global__ void __launch_bounds__(kPcg64T, 1) k_pcg64(const __grid_constant__ Ar
       }
     }
     __syncthreads();
-    if (warp < 3 * R) {
+    if (!single && warp < 3 * R) {
       // approximate sums: p.Ap, and what the starts of |r|^2 and r.z will need
       const int q = warp / R, r = segment(q);
       const Chunk c = seg_chunk(P, r, nt);
@@ -428,11 +453,15 @@ __global__ void __launch_bounds__(kPcg64T, 1) k_pcg64(const __grid_constant__ Ar
         }
       }
     }
-    barrier();
-    if (warp < R)
-      order(D_PAP, warp, t0, before(W_PAP, warp));
-    barrier();
-    walk1(D_PAP, d.T0);
+    if (single) {
+      serial(t0, nullptr);
+    } else {
+      barrier();
+      if (warp < R)
+        order(D_PAP, warp, t0, before(W_PAP, warp));
+      barrier();
+      walk1(D_PAP, d.T0);
+    }
     const double pAp = res[0];
     if (!(pAp > 1e-30)) { iters = k; done = true; break; }
     const double alpha = rz / pAp;
@@ -467,7 +496,7 @@ __global__ void __launch_bounds__(kPcg64T, 1) k_pcg64(const __grid_constant__ Ar
         o[(size_t)W_ZZ * NS] = u0; o[(size_t)W_ZP * NS] = u1; o[(size_t)W_PP * NS] = u2;
       }
     };
-    if (warp < (jacobi ? 3 * R : R)) {
+    if (!single && warp < (jacobi ? 3 * R : R)) {
       const int q = warp / R, r = segment(q);
       if (q < 2) {
         const int row = q ? W_RZ : W_RR;
@@ -477,7 +506,8 @@ __global__ void __launch_bounds__(kPcg64T, 1) k_pcg64(const __grid_constant__ Ar
       }
     }
     barrier();
-    walk(heads(D_RR), heads(D_RZ), stages(D_RR), stages(D_RZ), jacobi ? 2 : 1, NS, d.T1, d.T2, wst, stp, res);
+    if (single) serial(t1, jacobi ? t2 : nullptr);
+    else walk(heads(D_RR), heads(D_RZ), stages(D_RR), stages(D_RZ), jacobi ? 2 : 1, NS, d.T1, d.T2, wst, stp, res);
     residual = sqrt(res[0]);
     double rzNew = res[1];
     if (residual < absTol) { iters = k + 1; done = true; break; }
@@ -490,7 +520,7 @@ __global__ void __launch_bounds__(kPcg64T, 1) k_pcg64(const __grid_constant__ Ar
         term(t2, d.T2, i, lr[i] * zi);
       }
       __syncthreads();
-      if (warp < 2 * R) {
+      if (!single && warp < 2 * R) {
         const int q = warp / R, r = segment(q);
         if (q == 0) {
           const Chunk c = seg_chunk(P, r, nt);
@@ -502,11 +532,15 @@ __global__ void __launch_bounds__(kPcg64T, 1) k_pcg64(const __grid_constant__ Ar
           direction_sums(r);
         }
       }
-      barrier();
-      if (warp < R)
-        order(D_RZ, warp, t2, before(W_RZ, warp));
-      barrier();
-      walk1(D_RZ, d.T2);
+      if (single) {
+        serial(t2, nullptr);
+      } else {
+        barrier();
+        if (warp < R)
+          order(D_RZ, warp, t2, before(W_RZ, warp));
+        barrier();
+        walk1(D_RZ, d.T2);
+      }
       rzNew = res[0];
     }
     const double beta = rzNew / rz;
@@ -518,11 +552,13 @@ __global__ void __launch_bounds__(kPcg64T, 1) k_pcg64(const __grid_constant__ Ar
     }
     rz = rzNew;
     __syncthreads();
-    if (warp < R) {
-      order(D_PP, warp, t3, before3(W_ZZ, warp, 2 * beta, beta * beta));
+    if (single) {
+      serial(t3, nullptr);
+    } else {
+      if (warp < R) order(D_PP, warp, t3, before3(W_ZZ, warp, 2 * beta, beta * beta));
+      barrier();
+      walk1(D_PP, d.T3);
     }
-    barrier();
-    walk1(D_PP, d.T3);
     pp = res[0];
   }
   if (!done) iters = A.maxIters;
@@ -530,6 +566,10 @@ __global__ void __launch_bounds__(kPcg64T, 1) k_pcg64(const __grid_constant__ Ar
   // ---- descent safeguard + trust region (newton.ts:152-179) ----
   // left-to-right sum of the terms in (t0, d.T0)
   auto sum0 = [&]() {
+    if (single) {
+      serial(t0, nullptr);
+      return res[0];
+    }
     __syncthreads();
     if (warp < R) {
       const Chunk c = seg_chunk(P, warp, nt);
@@ -641,11 +681,21 @@ int pcg64_cluster_max() {
   return r;
 }
 
-// Sheets up to this many vertices run in one cluster: one vertex per thread
-// pair there. Beyond it the FP64 arithmetic of 16 SMs outweighs what the
-// cluster's barrier saves over the grid's.
+// Sheets up to kPcg64SingleN vertices run in one CTA, up to kPcg64ClusterN in one cluster,
+// larger ones on the grid. The ordered sums' stages cost more than adding the terms
+// one by one while there are few: us per iteration on a B200, one thread per sum on a
+// cooperative grid / stages in a cluster / one CTA, Jacobi: 36 vertices 19 / 23.3 / 8.4, 81
+// vertices 23 / 24.4 / 11.7, 169 vertices 31 / 26 / 18.5, 256 vertices 37 / 26 / 24.3,
+// 441 vertices 48 / 28 / 47; Schwarz: 36 vertices 51 / 37 / 18, 256 vertices 111 / 46 / 49.
+constexpr int kPcg64SingleN = 256;
+// One vertex per thread pair of a cluster. Beyond it the FP64 arithmetic of 16 SMs
+// outweighs what the cluster's barrier saves: ms of a two-step drape in a cluster / on
+// the grid, Jacobi: 55 x 55 vertices 60 / 61, 64 x 64 65 / 66, 71 x 71 73 / 67, 77 x 77
+// 88 / 68. (With Schwarz the grid is ahead from 2,000 vertices on: 46 x 46 64 / 62.5, 64 x 64 73 / 64.)
 constexpr int kPcg64ClusterN = 4096;
-// Vertices per CTA of the grid at the least: fewer CTAs mean fewer stages to walk.
+// Vertices per CTA of the grid at the least: fewer CTAs mean fewer stages to walk, but
+// longer ones. The same drape with 64 / 96 / 128 / 192: 71 x 71 72 / 67 / 69 / 76 ms,
+// 91 x 91 89 / 79 / 78 / 83, 111 x 111 102 / 99 / 95 / 97 (Schwarz 63 / 61 / 63 / 64).
 constexpr int kPcg64GridNv = 96;
 
 void build_pcg64_plan(const HostMesh& me, int sms, int clusterMax, bool lists, Pcg64Host& out) {
@@ -653,15 +703,14 @@ void build_pcg64_plan(const HostMesh& me, int sms, int clusterMax, bool lists, P
   p = Pcg64Plan{};
   p.cluster = clusterMax > 0 && me.n <= kPcg64ClusterN * clusterMax / 16 ? 1 : 0;
   if (p.cluster) {
-    p.G = 1;
-    while (p.G < clusterMax && me.n > 8 * p.G) p.G *= 2;
+    p.G = me.n <= kPcg64SingleN ? 1 : clusterMax;
   } else {
     p.G = std::max(1, std::min(sms, (me.n + kPcg64GridNv - 1) / kPcg64GridNv));
   }
   p.nv = (me.n + p.G - 1) / p.G;
   const int terms = 3 * p.nv;
   // fewer segments to walk against fewer terms per lane to map
-  p.R = p.G == 1 ? 4 : p.G <= 16 && terms > 160 ? 2 : 1;
+  p.R = p.G <= 16 && terms > 160 ? 2 : 1;
   p.K = ((terms + p.R * 32 - 1) / (p.R * 32)) | 1;
   p.NS = p.G * p.R;
   out.slotOff.assign(1, 0);

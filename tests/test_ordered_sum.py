@@ -105,7 +105,8 @@ def test_solve_fits_shared_memory_at_any_size(hc, n, parts):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("nx,ny,precond", [
-    (1, 1, "schwarz"), (2, 1, "jacobi"), (7, 9, "mas2"), (10, 12, "jacobi"),   # a cluster of 1 .. 16 CTAs
+    (1, 1, "schwarz"), (2, 1, "jacobi"), (7, 9, "mas2"), (10, 12, "jacobi"),   # one CTA
+    (15, 15, "jacobi"), (15, 15, "mas2"), (42, 5, "jacobi"), (42, 5, "schwarz"),  # the last alone, the first cluster
     (63, 63, "schwarz"), (64, 63, "schwarz"), (64, 63, "jacobi"),              # the last cluster, the first grid
     (255, 70, "mas2"), (300, 299, "jacobi"),                                   # element results in memory
     (500, 399, "jacobi"),                                                      # vectors in memory too
@@ -131,7 +132,7 @@ def test_solve_at_launch_edges(nx, ny, precond):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("n", [0, 1, 127, 128, 129, 3968, 3969, 12288, 196608, 200001])
+@pytest.mark.parametrize("n", [0, 1, 127, 128, 129, 1024, 1025, 3968, 3969, 12288, 196608, 200001])
 def test_block_sum(hc, n):
     for name, t in arrays(n):
         out = np.zeros(1)
