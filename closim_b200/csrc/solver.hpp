@@ -767,6 +767,16 @@ class Solver {
   // cluster's barrier and the captured step (a cooperative launch cannot be in
   // one) are worth more: a 65 x 65 sheet is the first that does not fit.
   static constexpr int kMxGridN = 4096;
+  // Vertices per CTA at the least. A sheet alone is no slower with 64 than with 32
+  // (80 x 80 vertices, three steps, exact mode 197 / 184 ms with 32 / 64, 195 with 96,
+  // 202 with 128; reference budget 37.9 / 37.3 / 37.1 / 38.5; 100 x 100 in exact mode 193
+  // / 193 / 202 / 204), and cooperative launches of several solvers run side by side only
+  // while their CTAs fit: 80 x 80 sheets, six steps each, two of them on two threads 91 / 77
+  // ms, four 172 / 140. (The gathering cluster kernel, which takes 16 SMs and steps in
+  // a captured graph: one sheet 73, two 78, four 106; one of 121 x 121 121, four 154 against
+  // 76 and 208 on the grid.) Where lists of 64 vertices do not fit, CTAs of as few as
+  // 32 are tried.
+  static constexpr int kMxGridNv = 64, kMxGridNvLeast = 32;
   void build_grid_resident(bool forceCluster) {
     mxGrid = 0;
     if (mxCluster <= 0) {
@@ -778,13 +788,18 @@ class Solver {
     if (env && std::string(env) == "0") return;
     int sms = 0;
     CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
-    const int ctas = std::min(std::min(sms, kMxGridMax), (mesh.n + 31) / 32);
     // without a cluster (past 20,000 vertices) exact mode solves in FP64
-    if (cluster_plan_least_smem(mesh, ctas, mxCluster > 0) > (size_t)kMxGridMaxDyn) return;
-    build_cluster_plan(mesh, ctas, kClWarps, grl.host, false, mxCluster > 0);
-    const size_t most = mxCluster > 0 ? grl.host.smemHinge : grl.host.smemNoHinge;
-    if (!grl.host.ok || !mx_grid_ok(ctas, most)) return;
-    mxGrid = ctas;
+    const bool hinges = mxCluster > 0;
+    for (int nv : {kMxGridNv, kMxGridNvLeast}) {
+      const int ctas = std::min(std::min(sms, kMxGridMax), (mesh.n + nv - 1) / nv);
+      if (cluster_plan_least_smem(mesh, ctas, hinges) > (size_t)kMxGridMaxDyn) continue;
+      build_cluster_plan(mesh, ctas, kClWarps, grl.host, false, hinges);
+      if (grl.host.ok && mx_grid_ok(ctas, hinges ? grl.host.smemHinge : grl.host.smemNoHinge)) {
+        mxGrid = ctas;
+        break;
+      }
+    }
+    if (mxGrid == 0) return;
     mxGridSmem[0] = grl.host.smemNoHinge;
     mxGridSmem[1] = grl.host.smemHinge;
     mxGridPart.alloc(8 * (size_t)kMxGridMax);
