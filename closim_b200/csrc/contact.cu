@@ -440,9 +440,9 @@ __global__ void k_contact_prep(CView v, const double* x, int na) {
 // each of the 1024 threads adds a strided subset, then warp and block trees
 // (same bits on every run).
 constexpr int kSumThreads = 1024;
+template <bool SHORT>
 __global__ void __launch_bounds__(kSumThreads) k_contact_sums(CView v, int na) {
-  __shared__ OrdSmem<kSumThreads / 32> os;
-  const double s = block_ordered_sum(blockIdx.x == 0 ? v.tc : v.tf, na, os);
+  const double s = ordered_sum<kSumThreads / 32, SHORT>(blockIdx.x == 0 ? v.tc : v.tf, na);
   if (threadIdx.x != 0) return;
   if (blockIdx.x == 0) v.diag->barrierEnergy = s;
   else v.diag->frictionWork = v.diag->frictionWork + s;
@@ -1323,7 +1323,8 @@ void ContactHost::gradient_terms(Solver& s) {
     lc++;
   }
   if (s.mixed()) k_contact_chains<<<1, 1024, 0, st>>>(v, na);
-  else k_contact_sums<<<2, kSumThreads, 0, st>>>(v, na);
+  else if (na <= kSumThreads) k_contact_sums<true><<<2, kSumThreads, 0, st>>>(v, na);
+  else k_contact_sums<false><<<2, kSumThreads, 0, st>>>(v, na);
   lc++;
   if (na > 0) {
     k_contact_grad_rec<<<cnb(4l * na), kCT, 0, st>>>(v, 4 * na);

@@ -401,6 +401,29 @@ struct OrdSmem {
   double wsum[2][32];
 };
 
+// A sum of at most one term a thread, added by thread 0 from shared memory.
+// Cycles of a block of 1,024 on a B200, this way / by stages: 129 terms 2,100 / 12,100, 512
+// terms 5,200 / 12,100, 1,024 terms 9,700 / 12,400; by stages 2,048 terms take 13,300.
+template <int WARPS>
+__device__ __forceinline__ double block_short_sum(const double* t, int n) {
+  __shared__ double buf[32 * WARPS];
+  if ((int)threadIdx.x < n) buf[threadIdx.x] = t[threadIdx.x];
+  __syncthreads();
+  double p = 0.0;
+  if (threadIdx.x == 0) {
+    int j = 0;
+    for (; j + 16 <= n; j += 16) {
+      double a[16];
+#pragma unroll
+      for (int q = 0; q < 16; q++) a[q] = buf[j + q];
+#pragma unroll
+      for (int q = 0; q < 16; q++) p = p + a[q];
+    }
+    for (; j < n; j++) p = p + buf[j];
+  }
+  return p;
+}
+
 // 0.0 + t[0] + ... + t[n-1], left to right, by a block of 32 * WARPS threads
 // (all of them call it; the sum is valid in thread 0). Warps 1.. turn tiles of
 // terms into stages while warp 0 walks the previous tile's. The arithmetic
@@ -412,28 +435,6 @@ __device__ __forceinline__ double block_ordered_sum(const double* t, int n, OrdS
   constexpr int E = WARPS - 1;
   constexpr int kTile = E * 32 * kOrdK;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  // Short sums: one term a thread, added by thread 0 from shared memory. Cycles of a
-  // block of 1,024 on a B200, this way / by stages: 129 terms 2,100 / 12,100, 512
-  // terms 5,200 / 12,100, 1,024 terms 9,700 / 12,400; by stages 2,048 terms take 13,300.
-  if (n <= 32 * WARPS) {
-    double* const buf = reinterpret_cast<double*>(sm.st);
-    if ((int)threadIdx.x < n) buf[threadIdx.x] = t[threadIdx.x];
-    __syncthreads();
-    double p = 0.0;
-    if (threadIdx.x == 0) {
-      int j = 0;
-      for (; j + 16 <= n; j += 16) {
-        double a[16];
-#pragma unroll
-        for (int q = 0; q < 16; q++) a[q] = buf[j + q];
-#pragma unroll
-        for (int q = 0; q < 16; q++) p = p + a[q];
-      }
-      for (; j < n; j++) p = p + buf[j];
-    }
-    __syncthreads();
-    return p;
-  }
   const int nTiles = (n + kTile - 1) / kTile;
   const int off = ((warp - 1) * 32 + lane) * kOrdK;
   double cur[kOrdK], nxt[kOrdK];
@@ -499,6 +500,15 @@ __device__ __forceinline__ double block_ordered_sum(const double* t, int n, OrdS
     __syncthreads();
   }
   return ord_dbl(S);
+}
+
+// The same by either way. SHORT (n <= 32 * WARPS, chosen at the launch) keeps the
+// stages' code and shared memory out of the kernel. One call per kernel.
+template <int WARPS, bool SHORT>
+__device__ __forceinline__ double ordered_sum(const double* t, int n) {
+  if constexpr (SHORT) return block_short_sum<WARPS>(t, n);
+  __shared__ OrdSmem<WARPS> sm;
+  return block_ordered_sum(t, n, sm);
 }
 
 #endif  // __CUDACC__

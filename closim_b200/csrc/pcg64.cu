@@ -159,7 +159,11 @@ __device__ __noinline__ double serial_sum(const double* t, int n) {
   return p;
 }
 
-template <bool CLUSTER>
+// The CTAs of a launch: one, one thread-block cluster, or a cooperative grid.
+// (GRID_FAR: whose contact-record offsets do not fit in shared memory).
+enum Shape { ONE, CLUSTER, GRID, GRID_FAR };
+
+template <Shape SHAPE>
 __global__ void __launch_bounds__(kPcg64T, 1) k_pcg64(const __grid_constant__ Args A) {
   extern __shared__ __align__(16) unsigned char dyn[];
   __shared__ double res[2];
@@ -169,7 +173,8 @@ __global__ void __launch_bounds__(kPcg64T, 1) k_pcg64(const __grid_constant__ Ar
   const Dev& d = A.d;
   const Pcg64Plan& P = A.P;
   auto barrier = [&]() {
-    if constexpr (CLUSTER) cg::this_cluster().sync();
+    if constexpr (SHAPE == ONE) __syncthreads();
+    else if constexpr (SHAPE == CLUSTER) cg::this_cluster().sync();
     else cg::this_grid().sync();
   };
   constexpr int T = kPcg64T, W = T / 32;
@@ -198,9 +203,9 @@ __global__ void __launch_bounds__(kPcg64T, 1) k_pcg64(const __grid_constant__ Ar
   // this launch's contact-record offsets of the owned vertices, at the end of the
   // shared memory where they fit
   uint32_t* const cOffS = reinterpret_cast<uint32_t*>(dyn + P.smem) - (P.nv + 1);
-  if (d.hasContact && P.offSmem)
+  if (SHAPE != GRID_FAR && d.hasContact)
     for (int i = threadIdx.x; i <= nOwn; i += T) cOffS[i] = d.c.cOff[vb0 + i];
-  auto cOff = [&](int lv) { return P.offSmem ? cOffS[lv] : __ldg(d.c.cOff + vb0 + lv); };
+  auto cOff = [&](int lv) { return SHAPE != GRID_FAR ? cOffS[lv] : __ldg(d.c.cOff + vb0 + lv); };
   // A term in the CTA's copy and (for a walk's fallback) in memory.
   auto term = [&](double* loc, double* glob, int i, double v) {
     loc[i] = v;
@@ -224,7 +229,7 @@ __global__ void __launch_bounds__(kPcg64T, 1) k_pcg64(const __grid_constant__ Ar
     walk(heads(k0), heads(k1), stages(k0), stages(k1), 2, NS, T0, T1, wst, stp, res);
   };
   // A lone CTA holds all terms: its first two warps add one sum each (ta, tb) in order.
-  const bool single = P.G == 1;
+  constexpr bool single = SHAPE == ONE;
   auto serial = [&](const double* ta, const double* tb) {
     __syncthreads();
     if ((threadIdx.x & 31) == 0 && warp < (tb ? 2 : 1)) res[warp] = serial_sum(warp ? tb : ta, nt);
@@ -299,12 +304,12 @@ __global__ void __launch_bounds__(kPcg64T, 1) k_pcg64(const __grid_constant__ Ar
     order(q, r, t, before(row, r));
   }
   barrier();
-  if (single) serial(t0, t1);
+  if constexpr (single) serial(t0, t1);
   else walk2(D_PAP, D_RR, d.T0, d.T1);
   const double bNorm = sqrt(res[0]);
   double residual = sqrt(res[1]);
   __syncthreads();
-  if (single) serial(t2, t3);
+  if constexpr (single) serial(t2, t3);
   else walk2(D_RZ, D_PP, d.T2, d.T3);
   double rz = res[0];
   double pp = res[1];
@@ -453,7 +458,7 @@ __global__ void __launch_bounds__(kPcg64T, 1) k_pcg64(const __grid_constant__ Ar
         }
       }
     }
-    if (single) {
+    if constexpr (single) {
       serial(t0, nullptr);
     } else {
       barrier();
@@ -506,7 +511,7 @@ __global__ void __launch_bounds__(kPcg64T, 1) k_pcg64(const __grid_constant__ Ar
       }
     }
     barrier();
-    if (single) serial(t1, jacobi ? t2 : nullptr);
+    if constexpr (single) serial(t1, jacobi ? t2 : nullptr);
     else walk(heads(D_RR), heads(D_RZ), stages(D_RR), stages(D_RZ), jacobi ? 2 : 1, NS, d.T1, d.T2, wst, stp, res);
     residual = sqrt(res[0]);
     double rzNew = res[1];
@@ -532,7 +537,7 @@ __global__ void __launch_bounds__(kPcg64T, 1) k_pcg64(const __grid_constant__ Ar
           direction_sums(r);
         }
       }
-      if (single) {
+      if constexpr (single) {
         serial(t2, nullptr);
       } else {
         barrier();
@@ -552,7 +557,7 @@ __global__ void __launch_bounds__(kPcg64T, 1) k_pcg64(const __grid_constant__ Ar
     }
     rz = rzNew;
     __syncthreads();
-    if (single) {
+    if constexpr (single) {
       serial(t3, nullptr);
     } else {
       if (warp < R) order(D_PP, warp, t3, before3(W_ZZ, warp, 2 * beta, beta * beta));
@@ -566,7 +571,7 @@ __global__ void __launch_bounds__(kPcg64T, 1) k_pcg64(const __grid_constant__ Ar
   // ---- descent safeguard + trust region (newton.ts:152-179) ----
   // left-to-right sum of the terms in (t0, d.T0)
   auto sum0 = [&]() {
-    if (single) {
+    if constexpr (single) {
       serial(t0, nullptr);
       return res[0];
     }
@@ -665,16 +670,18 @@ int pcg64_cluster_max() {
   std::lock_guard<std::mutex> lock(mu);
   const auto it = known.find(dev);
   if (it != known.end()) return it->second;
-  cudaFuncSetAttribute(k_pcg64<true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-  cudaFuncSetAttribute(k_pcg64<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxDyn);
-  cudaFuncSetAttribute(k_pcg64<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxDyn);
+  cudaFuncSetAttribute(k_pcg64<CLUSTER>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  cudaFuncSetAttribute(k_pcg64<CLUSTER>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxDyn);
+  cudaFuncSetAttribute(k_pcg64<GRID>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxDyn);
+  cudaFuncSetAttribute(k_pcg64<GRID_FAR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxDyn);
+  cudaFuncSetAttribute(k_pcg64<ONE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxDyn);
   int r = 0;
   for (int cs = 16; cs >= 1 && !r; cs /= 2) {
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[1];
     cluster_attr(cfg, attr, cs, kMaxDyn);
     int nc = 0;
-    if (cudaOccupancyMaxActiveClusters(&nc, k_pcg64<true>, &cfg) == cudaSuccess && nc >= 1) r = cs;
+    if (cudaOccupancyMaxActiveClusters(&nc, k_pcg64<CLUSTER>, &cfg) == cudaSuccess && nc >= 1) r = cs;
   }
   cudaGetLastError();
   known[dev] = r;
@@ -754,15 +761,17 @@ void build_pcg64_plan(const HostMesh& me, int sms, int clusterMax, bool lists, P
 
 int launch_pcg64(const Dev& d, const Pcg64Plan& p, int maxIters, double tol, cudaStream_t s) {
   Args a{d, p, maxIters, tol};
+  void* args[] = {&a};
+  if (p.G == 1) return (int)cudaLaunchKernel((void*)k_pcg64<ONE>, dim3(1), dim3(kPcg64T), args, p.smem, s);
   if (p.cluster) {
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[1];
     cluster_attr(cfg, attr, p.G, p.smem);
     cfg.stream = s;
-    return (int)cudaLaunchKernelEx(&cfg, k_pcg64<true>, a);
+    return (int)cudaLaunchKernelEx(&cfg, k_pcg64<CLUSTER>, a);
   }
-  void* args[] = {&a};
-  return (int)cudaLaunchCooperativeKernel((void*)k_pcg64<false>, dim3(p.G), dim3(kPcg64T), args, p.smem, s);
+  auto* grid = p.offSmem ? k_pcg64<GRID> : k_pcg64<GRID_FAR>;
+  return (int)cudaLaunchCooperativeKernel((void*)grid, dim3(p.G), dim3(kPcg64T), args, p.smem, s);
 }
 
 }  // namespace cs

@@ -10,6 +10,8 @@
 
 #include "adjoint_math.cuh"
 #include "contact.cuh"
+#include <algorithm>
+
 #include "ordered_sum.cuh"
 #include "plain.cuh"
 
@@ -23,6 +25,11 @@ __device__ __forceinline__ void load3(const double* x, int v, double o[3]) {
 
 // Block size of the kernels that evaluate one ordered sum (ordered_sum.cuh).
 constexpr int kOrdThreads = 1024;
+#define ORD_LAUNCH(kernel, n, grid, stream, ...)                                  \
+  do {                                                                            \
+    if ((n) <= kOrdThreads) kernel<true><<<grid, kOrdThreads, 0, stream>>>(__VA_ARGS__); \
+    else kernel<false><<<grid, kOrdThreads, 0, stream>>>(__VA_ARGS__);            \
+  } while (0)
 
 // ---- predictor (newton.ts:41-50) -------------------------------------------
 // yHat = x0 + h v + h^2 g is the inertial target and, in the reference, the
@@ -134,9 +141,9 @@ __global__ void __launch_bounds__(kThreads) k_gather_grad(Dev d) {
 
 // Final reduction of the gradient pass: sqrt(sum g^2) in index order
 // (newton.ts:128), max strain (order-free).
+template <bool SHORT>
 __global__ void __launch_bounds__(kOrdThreads) k_grad_final(Dev d, int nbT) {
-  __shared__ OrdSmem<kOrdThreads / 32> os;
-  const double gs = block_ordered_sum(d.T0, d.n * 3, os);
+  const double gs = ordered_sum<kOrdThreads / 32, SHORT>(d.T0, d.n * 3);
   if (threadIdx.x >= 32) return;
   const double ms = warp_max_partials(d.part + 0 * d.partStride, nbT);
   if (threadIdx.x == 0) {
@@ -174,11 +181,11 @@ __global__ void __launch_bounds__(kThreads) k_energy(Dev d, const double* x) {
 
 // totalEnergy (newton.ts:76-88): ((sum inertia) + internal) + merit, each sum a
 // left-to-right chain; block 0 inertia, block 1 internal, block 2 merit.
+template <bool SHORT>
 __global__ void __launch_bounds__(kOrdThreads) k_energy_chains(Dev d, int nMerit) {
-  __shared__ OrdSmem<kOrdThreads / 32> os;
   const double* t = blockIdx.x == 0 ? d.T0 : blockIdx.x == 1 ? d.T1 : d.Tc;
   const int n = blockIdx.x == 0 ? d.n * 3 : blockIdx.x == 1 ? d.m + (d.kb > 0 ? d.hg : 0) : d.hasContact ? nMerit : 0;
-  const double v = block_ordered_sum(t, n, os);
+  const double v = ordered_sum<kOrdThreads / 32, SHORT>(t, n);
   if (threadIdx.x == 0) d.scal[S_E_INERTIA + blockIdx.x] = v;
 }
 __global__ void k_energy_final(Dev d) {
@@ -346,9 +353,9 @@ __global__ void k_hvp_terms(const double* p, int n3, double* T) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n3) T[i] = p[i] * p[i];
 }
+template <bool SHORT>
 __global__ void __launch_bounds__(kOrdThreads) k_hvp_h(const double* T, int n3, double* h) {
-  __shared__ OrdSmem<kOrdThreads / 32> os;
-  const double pp = block_ordered_sum(T, n3, os);
+  const double pp = ordered_sum<kOrdThreads / 32, SHORT>(T, n3);
   if (threadIdx.x == 0) *h = 1e-8 * (1 + sqrt(pp));
 }
 __device__ __forceinline__ void hvp_elem_tri(int t, const uint32_t* idx, const float4* inv, const float* area,
@@ -398,7 +405,7 @@ void launch_membrane_hvp(const uint32_t* idx, const float4* inv, const float* ar
                          int m, const uint32_t* memOff, const uint32_t* memRec, const double* x, const double* p,
                          double* out, double* T, double* h, double* elem, cudaStream_t s) {
   k_hvp_terms<<<nblk(n * 3), kThreads, 0, s>>>(p, n * 3, T);
-  k_hvp_h<<<1, kOrdThreads, 0, s>>>(T, n * 3, h);
+  ORD_LAUNCH(k_hvp_h, n * 3, 1, s, T, n * 3, h);
   k_hvp_elem<<<nblk(m), kThreads, 0, s>>>(idx, inv, area, mat, m, x, p, h, elem);
   k_hvp_gather<<<nblk(n), kThreads, 0, s>>>(memOff, memRec, n, elem, h, out);
 }
@@ -445,9 +452,9 @@ __global__ void __launch_bounds__(kThreads) k_gather_internal(Dev d, double* gra
 }
 // out[0] = the internal energy chain, out[1] = max strain over the triangle
 // partials (nbT of them; 0 when none were computed).
+template <bool SHORT>
 __global__ void __launch_bounds__(kOrdThreads) k_internal_final(Dev d, int nbT, double* out) {
-  __shared__ OrdSmem<kOrdThreads / 32> os;
-  const double e = block_ordered_sum(d.T1, d.m + (d.kb > 0 ? d.hg : 0), os);
+  const double e = ordered_sum<kOrdThreads / 32, SHORT>(d.T1, d.m + (d.kb > 0 ? d.hg : 0));
   if (threadIdx.x >= 32) return;
   const double ms = nbT > 0 ? warp_max_partials(d.part + 0 * d.partStride, nbT) : 0.0;
   if (threadIdx.x == 0) {
@@ -495,7 +502,7 @@ void launch_internal_eval(const Dev& d0, const double* x, double* grad, double* 
     k_gather_internal<<<nblk(d.n), kThreads, 0, s>>>(d, grad);
   }
   k_internal_energy_terms<<<nblk(std::max(d.m, d.hg)), kThreads, 0, s>>>(d, x);
-  k_internal_final<<<1, kOrdThreads, 0, s>>>(d, nbT, out2);
+  ORD_LAUNCH(k_internal_final, d.m + (d.kb > 0 ? d.hg : 0), 1, s, d, nbT, out2);
 }
 
 void launch_membrane_hvp_analytic(const Dev& d, const double* x, const double* p, double* out, cudaStream_t s) {
@@ -556,7 +563,7 @@ void launch_grad_terms(const Dev& d, cudaStream_t s, bool analyticBend) {
 }
 void launch_grad(const Dev& d, cudaStream_t s, bool analyticBend) {
   launch_grad_terms(d, s, analyticBend);
-  k_grad_final<<<1, kOrdThreads, 0, s>>>(d, nblk(d.m));
+  ORD_LAUNCH(k_grad_final, d.n * 3, 1, s, d, nblk(d.m));
 }
 void launch_energy_terms(const Dev& d, const double* x, cudaStream_t s) {
   const int nb = nblk(std::max(std::max(d.n, d.m), d.hg));
@@ -564,7 +571,8 @@ void launch_energy_terms(const Dev& d, const double* x, cudaStream_t s) {
 }
 void launch_energy(const Dev& d, const double* x, cudaStream_t s) {
   launch_energy_terms(d, x, s);
-  k_energy_chains<<<3, kOrdThreads, 0, s>>>(d, d.hasContact ? d.c.nActive : 0);
+  const int nMerit = d.hasContact ? d.c.nActive : 0;
+  ORD_LAUNCH(k_energy_chains, std::max(std::max(d.n * 3, d.m + (d.kb > 0 ? d.hg : 0)), nMerit), 3, s, d, nMerit);
   k_energy_final<<<1, 1, 0, s>>>(d);
 }
 void launch_diag_init(const Dev& d, double beta, cudaStream_t s) {

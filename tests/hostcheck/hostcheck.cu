@@ -7,9 +7,9 @@
 #include "../../closim_b200/csrc/ordered_sum.cuh"
 #include "../../closim_b200/csrc/pcg64.cu"
 
+template <bool SHORT>
 __global__ void __launch_bounds__(1024) k_hc_ordered(const double* t, int n, double* o) {
-  __shared__ cs::OrdSmem<32> os;
-  const double s = cs::block_ordered_sum(t, n, os);
+  const double s = cs::ordered_sum<32, SHORT>(t, n);
   if (threadIdx.x == 0) *o = s;
 }
 
@@ -87,13 +87,14 @@ int64_t hc_pcg64_smem(int n, int* parts) {
   return (int64_t)h.p.smem;
 }
 // The block-wide ordered sum on the GPU; returns a cudaError_t.
-int hc_gpu_ordered_sum(const double* t, int n, double* out) {
+int hc_gpu_ordered_sum(const double* t, int n, int brief, double* out) {
   double *dt = nullptr, *dout = nullptr;
   cudaError_t e = cudaMalloc(&dt, (size_t)(n > 0 ? n : 1) * 8);
   if (e == cudaSuccess) e = cudaMalloc(&dout, 8);
   if (e == cudaSuccess && n > 0) e = cudaMemcpy(dt, t, (size_t)n * 8, cudaMemcpyHostToDevice);
   if (e == cudaSuccess) {
-    k_hc_ordered<<<1, 1024>>>(dt, n, dout);
+    if (brief) k_hc_ordered<true><<<1, 1024>>>(dt, n, dout);
+    else k_hc_ordered<false><<<1, 1024>>>(dt, n, dout);
     e = cudaMemcpy(out, dout, 8, cudaMemcpyDeviceToHost);
   }
   cudaFree(dt);

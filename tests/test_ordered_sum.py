@@ -21,7 +21,7 @@ def hc():
     L = C.CDLL(os.path.join(HERE, "hostcheck", "libhostcheck.so"))
     L.hc_ordered_maps.restype = C.c_double
     L.hc_ordered_maps.argtypes = [PTR, C.c_int, C.c_double, C.POINTER(C.c_int)]
-    L.hc_gpu_ordered_sum.argtypes = [PTR, C.c_int, PTR]
+    L.hc_gpu_ordered_sum.argtypes = [PTR, C.c_int, C.c_int, PTR]
     L.hc_div_rn.argtypes = [PTR, PTR, C.c_int, PTR]
     L.hc_pcg64_smem.restype = C.c_int64
     return L
@@ -136,5 +136,6 @@ def test_solve_at_launch_edges(nx, ny, precond):
 def test_block_sum(hc, n):
     for name, t in arrays(n):
         out = np.zeros(1)
-        assert hc.hc_gpu_ordered_sum(np.ascontiguousarray(t), n, out) == 0
-        assert same_bits(out[0], sequential(t)), name
+        for brief in range(2 if n <= 1024 else 1):  # short sums: by stages, and by one thread
+            assert hc.hc_gpu_ordered_sum(np.ascontiguousarray(t), n, brief, out) == 0
+            assert same_bits(out[0], sequential(t)), (name, brief)
