@@ -439,25 +439,53 @@ __device__ int sheet_pcg(const BatchDev& b, const Range& R, float C00, float C11
     const float alpha = (float)(rz / pAp);
     double s2[2];
     gsums<2>(s2, G, [&](Shares<2, GR::kVirt>& S) {
-      geach<true>(G, S, 3 * R.v0, 3 * R.v1, [&](int i, double (&s)[2]) {
-        const bool pin = b.pinned[i / 3];
-        float xi = b.xs[i] + alpha * b.p[i];
-        float ri = b.r[i] - alpha * b.Ap[i];
-        if (pin) { xi = 0.f; ri = 0.f; }
-        b.xs[i] = xi;
-        b.r[i] = ri;
-        s[0] += (double)ri * ri;
-        const float zi = ri * b.dinv[i];
-        b.z[i] = zi;
-        s[1] += (double)ri * zi;
-      });
+      // four dofs' loads in flight together; item u goes where geach would put it
+      constexpr int U = 4;
+      const int i1 = 3 * R.v1, st = G.stride();
+      for (int i = 3 * R.v0 + G.first(); i < i1; i += U * st) {
+        float x[U], p[U], r[U], a[U], di[U];
+        bool pin[U];
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+          const int k = i + u * st < i1 ? i + u * st : i;
+          x[u] = b.xs[k]; p[u] = b.p[k]; r[u] = b.r[k]; a[u] = b.Ap[k]; di[u] = b.dinv[k];
+          pin[u] = b.pinned[k / 3];
+        }
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+          const int k = i + u * st;
+          if (k < i1) {
+            float xi = x[u] + alpha * p[u];
+            float ri = r[u] - alpha * a[u];
+            if (pin[u]) { xi = 0.f; ri = 0.f; }
+            b.xs[k] = xi;
+            b.r[k] = ri;
+            double(&s)[2] = S.v[u % GR::kVirt];
+            s[0] += (double)ri * ri;
+            const float zi = ri * di[u];
+            b.z[k] = zi;
+            s[1] += (double)ri * zi;
+          }
+        }
+      }
     });
     residual = sqrt(s2[0]);
     const double rzn = s2[1];
     if (residual < absTol) { iters = k + 1; done = true; break; }
     const float beta = (float)(rzn / rz);
     rz = rzn;
-    for (int i = 3 * R.v0 + G.first(); i < 3 * R.v1; i += G.stride()) b.p[i] = b.z[i] + beta * b.p[i];
+    for (int i = 3 * R.v0 + G.first(), st = G.stride(), i1 = 3 * R.v1; i < i1; i += 4 * st) {
+      float z[4], p[4];
+#pragma unroll
+      for (int u = 0; u < 4; u++) {
+        const int k = i + u * st < i1 ? i + u * st : i;
+        z[u] = b.z[k];
+        p[u] = b.p[k];
+      }
+#pragma unroll
+      for (int u = 0; u < 4; u++)
+        if (i + u * st < i1) b.p[i + u * st] = z[u] + beta * p[u];
+    }
     gsync(G);
   }
   if (!done) iters = b.pcgMaxIters;
