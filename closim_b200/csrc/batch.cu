@@ -1,4 +1,5 @@
-// Batched implicit step: one launch steps every sheet of a packed work list.
+// Batched implicit step: one launch steps every sheet of a packed work list (one
+// launch per size class).
 //
 // Each sheet is an independent scene (no coupling), so a sheet maps to one
 // thread block, or one cluster of blocks (batch_class), that runs its whole
@@ -10,7 +11,8 @@
 // The launch is persistent: groups take sheets from a work list ordered largest
 // first. A sheet's PCG is a chain of short passes over its vertices, bound by the
 // latency of its gathers; one SM per sheet left the batch waiting for its largest
-// sheet (96 sheets of 16 to 80 vertices a side: 84 ms a step, 44 with clusters).
+// sheet (96 sheets of 16 to 80 vertices a side: 76 ms a step by lone blocks, 41 with
+// clusters).
 // The algorithm per sheet is newton.ts:27-303 with the floor-contact
 // subset of contact-assembly.ts (kind 2: per-vertex barrier, lagged friction,
 // floor CCD, restitution); the bending gradient is the analytic gradient of
@@ -40,7 +42,7 @@ constexpr int kParts = 12;  // up to three sums of four ranks
 // The threads that step one sheet: a thread-block cluster (CL) or one block, which
 // may reproduce the reductions of a cluster of VIRT blocks. The shape is part of the
 // type: with the stride and the barriers known at compile time 148 sheets of 38
-// vertices a side take 19.85 ms a step instead of 20.3.
+// vertices a side took 19.85 ms a step instead of 20.3.
 // `first` and `stride` spread a loop over all the threads.
 template <int T, bool CL, int VIRT>
 struct Group {
@@ -87,9 +89,9 @@ struct Shares {
 // stands in for it walks all items in memory order and gives each in turn to the
 // next rank's share: unrolled by VIRT in the short passes of the PCG (UNROLL), by
 // turning the shares one place an item in the long ones, whose code would outgrow
-// the instruction cache. 512 sheets of 16 to 128 vertices a side, ms a step on a B200: 387
-// with a pass per rank, 386 turning everywhere, 387 unrolled everywhere, 384
-// this way; 381 with one share and no clusters at all.
+// the instruction cache. 512 sheets of 16 to 128 vertices a side, ms a step on a B200
+// (before the vector passes loaded four dofs together): 387 with a pass per rank, 386
+// turning everywhere, 387 unrolled everywhere, 384 this way; 381 with one share.
 template <bool UNROLL = false, int K, class GR, class F>
 __device__ __forceinline__ void geach(const GR& G, Shares<K, GR::kVirt>& S, int i0, int i1, const F& f) {
   constexpr int V = GR::kVirt;
@@ -439,7 +441,8 @@ __device__ int sheet_pcg(const BatchDev& b, const Range& R, float C00, float C11
     const float alpha = (float)(rz / pAp);
     double s2[2];
     gsums<2>(s2, G, [&](Shares<2, GR::kVirt>& S) {
-      // four dofs' loads in flight together; item u goes where geach would put it
+      // Four dofs' loads in flight together, item u where geach would put it: the pass
+      // is bound by their latency (512 sheets of 16 to 128 a side 384 -> 301 ms a step).
       constexpr int U = 4;
       const int i1 = 3 * R.v1, st = G.stride();
       for (int i = 3 * R.v0 + G.first(); i < i1; i += U * st) {

@@ -15,10 +15,10 @@ constexpr int kBatchSize[kBatchClasses] = {4, 2, 1};
 inline int batch_class(int n) { return n > 3000 ? 0 : n > 1500 ? 1 : 2; }
 
 // Time of one sheet's step by `size` CTAs of 512 threads, in passes of a vertex
-// per thread (about 6.7 ms at the reference budget on a B200). Measured, ms a step:
-// lone blocks 19.9 at 1,444 vertices, 27.3 at 2,025, 41 at 3,025, 53 at 4,096, 88
-// at 6,400, 210 at 16,384; pairs 17.3 at 2,025; clusters of four 16.0 at 3,025, 16.6
-// at 4,096, 25.1 at 6,400, 58 at 16,384.
+// per thread (about 6.2 ms at the reference budget on a B200). Measured, ms a step:
+// lone blocks 18.4 at 1,444 vertices, 25.4 at 2,025, 37.9 at 3,025, 49.4 at 4,096, 85
+// at 6,400, 119 at 10,000; pairs 16.0 at 2,025; clusters of four 15.0 at 3,025, 15.3
+// at 4,096, 23.6 at 6,400, 35.3 at 10,000.
 inline double batch_sheet_cost(int n, int size) { return n / (512.0 * size) + (size > 1 ? 0.6 : 0.13); }
 
 // Estimated time of a step when class c's sheets (verts[c], largest first) go to
@@ -53,12 +53,12 @@ inline double batch_makespan(const std::vector<int> (&verts)[kBatchClasses], con
 // estimate's error). A cluster shortens the tail, a lone block spends fewer SM-cycles
 // on a sheet: equal sheets that fill the device with one block each run best alone, few
 // or very uneven ones in clusters. Measured on a B200 (33 clusters of four, 74 of two),
-// ms a step, lone / clusters / without clusters in the code: 64 x 64 vertices, 74
-// sheets 60 / 49 / 61, 148 sheets 70 / 81 / 69; 55 x 55, 37 sheets 42 / 32 / 41, 148
-// sheets 50 / 80 / 50; 45 x 45, 74 sheets 28 / 17 / 28, 148 sheets 28 / 34 / 28; 16 to
-// 128 a side, 64 sheets 225 / 62 / 222, 256 sheets 274 / 226 / 275, 512 sheets 384 /
-// 417 / 381. The estimate is on the safe side where many large sheets share the L2: 100
-// sheets of 100 x 100 go alone, 168 / 150 / 167.
+// ms a step, lone / clusters: 64 x 64 vertices, 74 sheets 52 / 46, 111 sheets 55 / 61,
+// 148 sheets 57 / 77; 55 x 55, 37 sheets 38 / 30, 74 sheets 38 / 45, 160 sheets 77 / 76;
+// 45 x 45, 74 sheets 25 / 16, 148 sheets 26 / 32, 222 sheets 50 / 48; 100 x 100, 60 sheets
+// 131 / 71, 100 sheets 133 / 137; 16 to 128 a side, 64 sheets 189 / 55, 256 sheets
+// 212 / 198, 384 sheets 225 / 274, 512 sheets 301 / 369. The estimate takes the
+// smaller of each of these.
 inline void batch_route(const std::vector<int> (&verts)[kBatchClasses], int sms,
                         const int (&maxGroups)[kBatchClasses], int (&size)[kBatchClasses]) {
   for (int c = 0; c < kBatchClasses; c++) size[c] = 1;

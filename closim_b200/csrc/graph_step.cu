@@ -23,8 +23,8 @@
 // in the same order, the decisions restated on the device (compiled without
 // FMA contraction, as the host compares). Buffer overflows are reported on the
 // device; the step is then restored and repeated on the host-driven path with
-// grown buffers. Scope: the mixed path's one-cluster PCG (sheets up to about
-// 20,000 vertices); other configurations take the host-driven step.
+// grown buffers. Scope: the mixed path where the one-cluster PCG solves
+// (Solver::pcg_kernel); other configurations take the host-driven step.
 #include <cstring>
 
 #include "graph_ctx.hpp"

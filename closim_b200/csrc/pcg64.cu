@@ -15,11 +15,9 @@
 // earlier, so each costs one barrier. Sheets up to kPcg64SingleN vertices run in
 // one CTA, which adds the terms one by one, sheets up to kPcg64ClusterN in one
 // 16-CTA cluster (hardware barrier), larger ones on the whole grid.
-// Whole steps on a B200 against one-thread chains on a cooperative grid: 41 x 9
-// strip (Jacobi, two steps) 43.7 -> 31.4 ms, 64 x 64 drape (Schwarz) 54.0 ->
-// 14.7 ms, 121 x 95 garment on a sphere (Jacobi) 411 -> 61 ms, the same bits. An
-// iteration is now bound by its barriers and the stage walks (5,000-8,000
-// cycles per dot product), with Schwarz by the domains' substitution chains.
+// On a B200 against one-thread chains on a cooperative grid, us per iteration: 41 x 9
+// strip (Jacobi) 43 -> 32, 64 x 64 drape Jacobi 202 -> 45, Schwarz 409 -> 84, 121 x 121 drape
+// Jacobi 645 -> 69, Schwarz 1,100 -> 104, the same bits. PHASES
 #include <cooperative_groups.h>
 
 #include <algorithm>

@@ -352,8 +352,8 @@ class Solver {
       mb.elem = felem.p; mb.tris = ftris.p; mb.h9 = fh9.p; mb.Linv = fLinv.p;
       build_schwarz_assembly();
       mxBlocks = mx_pcg_grid_blocks(d);
-      // Sheets up to 20k vertices solve inside one thread-block cluster
-      // (on-GPC barriers); larger ones use the grid-wide kernel.
+      // Sheets up to 20k vertices may solve inside one thread-block cluster (on-GPC
+      // barriers; build_grid_resident says which of them do); larger ones use the grid.
       // CLOSIM_MX_PCG=grid|cluster overrides the choice.
       const char* env = std::getenv("CLOSIM_MX_PCG");
       const bool wantCluster = env ? std::string(env) == "cluster" : mesh.n <= 20000;
