@@ -991,7 +991,7 @@ __global__ void __launch_bounds__(kClT, 1) k_mx_pcg_cluster(ClArgs A) {
 
 // ---- the same solve on the whole grid ------------------------------------------------
 // Sheets whose per-CTA lists do not fit one cluster's shared memory (about
-// 4,300 vertices up): one CTA per SM owns a contiguous range of vertices, keeps
+// 4,300 vertices up): each CTA, at most one per SM, owns a contiguous range of vertices, keeps
 // its triangles, hinges and incidence lists in shared memory for the whole solve
 // as the resident cluster kernel does, and exchanges p, Ap, r, z through L2 with
 // two cooperative grid barriers per iteration. Each vertex adds its incidences in
