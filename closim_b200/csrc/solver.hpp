@@ -767,10 +767,10 @@ class Solver {
   // cluster's barrier and the captured step (a cooperative launch cannot be in
   // one) are worth more: a 65 x 65 sheet is the first that does not fit.
   static constexpr int kMxGridN = 4096;
-  // Vertices per CTA at the least. A sheet alone is no slower with 64 than with 32
-  // (80 x 80 vertices, three steps, exact mode 197 / 184 ms with 32 / 64, 195 with 96,
-  // 202 with 128; reference budget 37.9 / 37.3 / 37.1 / 38.5; 100 x 100 in exact mode 193
-  // / 193 / 202 / 204), and cooperative launches of several solvers run side by side only
+  // Vertices per CTA at the least. A sheet alone takes as long with 64 as with 32 (80 x
+  // 80 vertices, three steps, exact mode 197 / 184 ms with 32 / 64, 195 with 96, 202 with
+  // 128; reference budget 37.9 / 37.3 / 37.1 / 38.5; 66 x 66 exact 161.6 / 162.6, Jacobi 36.0
+  // / 34.9; 68 x 65 exact with mas2 177 / 181, the most it loses), and cooperative launches of several solvers run side by side only
   // while their CTAs fit: 80 x 80 sheets, six steps each, two of them on two threads 91 / 77
   // ms, four 172 / 140. (The gathering cluster kernel, which takes 16 SMs and steps in
   // a captured graph: one sheet 73, two 78, four 106; one of 121 x 121 121, four 154 against
