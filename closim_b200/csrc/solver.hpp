@@ -763,19 +763,19 @@ class Solver {
     if (clRes[0] || clRes[1]) cl.upload(stream);
   }
   // Sheets past kMxGridN vertices whose lists do not fit one cluster: the
-  // grid-wide resident PCG (mixed_cluster.cu), one CTA per SM. Below that the
+  // grid-wide resident PCG (mixed_cluster.cu), at most one CTA per SM. Below that the
   // cluster's barrier and the captured step (a cooperative launch cannot be in
   // one) are worth more: a 65 x 65 sheet is the first that does not fit.
   static constexpr int kMxGridN = 4096;
   // Vertices per CTA at the least. A sheet alone takes as long with 64 as with 32 (80 x
   // 80 vertices, three steps, exact mode 197 / 184 ms with 32 / 64, 195 with 96, 202 with
-  // 128; reference budget 37.9 / 37.3 / 37.1 / 38.5; 66 x 66 exact 161.6 / 162.6, Jacobi 36.0
-  // / 34.9; 68 x 65 exact with mas2 177 / 181, the most it loses), and cooperative launches of several solvers run side by side only
-  // while their CTAs fit: 80 x 80 sheets, six steps each, two of them on two threads 91 / 77
-  // ms, four 172 / 140. (The gathering cluster kernel, which takes 16 SMs and steps in
-  // a captured graph: one sheet 73, two 78, four 106; one of 121 x 121 121, four 154 against
-  // 76 and 208 on the grid.) Where lists of 64 vertices do not fit, CTAs of as few as
-  // 32 are tried.
+  // 128; reference budget 37.9 / 37.3 / 37.1 / 38.5; 66 x 66 exact 161.6 / 162.6, Jacobi
+  // 36.0 / 34.9; 68 x 65 exact with mas2 177 / 181, the most it loses), and cooperative
+  // launches of several solvers run side by side only while their CTAs fit: 80 x 80
+  // sheets, six steps each, two of them on two threads 91 / 75 ms, four 172 / 139. (The
+  // gathering cluster kernel, which takes 16 SMs and steps in a captured graph: one
+  // sheet 73, two 78, four 106; one of 121 x 121 121, four 154 against 75 and 209 on the
+  // grid.) Where lists of 64 vertices do not fit, CTAs of as few as 32 are tried.
   static constexpr int kMxGridNv = 64, kMxGridNvLeast = 32;
   void build_grid_resident(bool forceCluster) {
     mxGrid = 0;
